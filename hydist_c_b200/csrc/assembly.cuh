@@ -23,15 +23,23 @@ struct PreT {
 };
 using Pre = PreT<double>;
 
-// _uzSolver_calculate_preindex (UVZSolver_multithread.cpp:210-278).
+// The momentum part of the preindex step: f1 u_{-} + f2 u + f3 u_{+} +
+// f4 (z - z_{+}) = f5 along the line, before the continuity rows enter it.
 template <class R>
-__device__ __forceinline__ PreT<R> pre_x(const StateT<R>& S, const CoefT<R>& c, int i, int j) {
+struct MomF {
+  R f1, f2, f3, f5;
+};
+
+// _uzSolver_calculate_preindex (UVZSolver_multithread.cpp:210-278): the
+// momentum coefficients of a cell ...
+template <class R>
+__device__ __forceinline__ MomF<R> mom_x(const StateT<R>& S, const CoefT<R>& c, int i, int j) {
   const int w = S.W;
   const int g = i * w + j;
   const R* u = S.u;
   const R* v = S.v;
   const R* Hm = S.Hmoi;
-  PreT<R> P;
+  MomF<R> P;
   R p = 0, q = 0;
   const R vtb = (v[g - 1] + v[g] + v[g + w - 1] + v[g + w]) * R(0.25);
   const R uu = u[g], VI = S.visco[g], Hu = S.Htdu[g];
@@ -59,21 +67,33 @@ __device__ __forceinline__ PreT<R> pre_x(const StateT<R>& S, const CoefT<R>& c, 
   }
   P.f5 = -2 * uu + dT * p - dT * c.CORIOLIS_FORCE * vtb - dT * VI * q -
          dT * (c.Windx - S.Tsxw[g]) * rH;
-  P.c2 = c.dTchia2dX * Hu;
-  P.a2 = -c.dTchia2dX * S.Htdu[g - w];
-  P.d2 = R(S.z[g]) - c.dTchia2dY * (S.Htdv[g] * v[g] - S.Htdv[g - 1] * v[g - 1]);
   return P;
+}
+
+// ... and its continuity row a2 u_{-} + z + c2 u = d2, a2 = -k Htdu(i-1, j),
+// c2 = k Htdu(i, j), d2 = z - flux_x (k = dT / 2dX).
+template <class R>
+__device__ __forceinline__ R flux_x(const StateT<R>& S, const CoefT<R>& c, int g) {
+  return c.dTchia2dY * (S.Htdv[g] * S.v[g] - S.Htdv[g - 1] * S.v[g - 1]);
+}
+
+template <class R>
+__device__ __forceinline__ PreT<R> pre_x(const StateT<R>& S, const CoefT<R>& c, int i, int j) {
+  const int g = i * S.W + j;
+  const MomF<R> m = mom_x(S, c, i, j);
+  return PreT<R>{m.f1, m.f2, m.f3, m.f5, -c.dTchia2dX * S.Htdu[g - S.W], c.dTchia2dX * S.Htdu[g],
+                 R(S.z[g]) - flux_x(S, c, g)};
 }
 
 // _vzSolver_calculate_preindex (UVZSolver_multithread.cpp:142-208).
 template <class R>
-__device__ __forceinline__ PreT<R> pre_y(const StateT<R>& S, const CoefT<R>& c, int i, int j) {
+__device__ __forceinline__ MomF<R> mom_y(const StateT<R>& S, const CoefT<R>& c, int i, int j) {
   const int w = S.W;
   const int g = i * w + j;
   const R* u = S.u;
   const R* v = S.v;
   const R* Hm = S.Hmoi;
-  PreT<R> P;
+  MomF<R> P;
   R p = 0, q = 0;
   const R utb = (u[g - w] + u[g] + u[g - w + 1] + u[g + 1]) * R(0.25);
   const R vv = v[g], VI = S.visco[g], Hv = S.Htdv[g];
@@ -105,10 +125,20 @@ __device__ __forceinline__ PreT<R> pre_y(const StateT<R>& S, const CoefT<R>& c, 
   }
   P.f5 = -2 * vv + dT * q + dT * c.CORIOLIS_FORCE * utb - dT * VI * p -
          dT * (c.Windy - S.Tsyw[g]) * rH;
-  P.c2 = c.dTchia2dY * Hv;
-  P.a2 = -c.dTchia2dY * S.Htdv[g - 1];
-  P.d2 = R(S.z[g]) - c.dTchia2dX * (S.Htdu[g] * u[g] - S.Htdu[g - w] * u[g - w]);
   return P;
+}
+
+template <class R>
+__device__ __forceinline__ R flux_y(const StateT<R>& S, const CoefT<R>& c, int g) {
+  return c.dTchia2dX * (S.Htdu[g] * S.u[g] - S.Htdu[g - S.W] * S.u[g - S.W]);
+}
+
+template <class R>
+__device__ __forceinline__ PreT<R> pre_y(const StateT<R>& S, const CoefT<R>& c, int i, int j) {
+  const int g = i * S.W + j;
+  const MomF<R> m = mom_y(S, c, i, j);
+  return PreT<R>{m.f1, m.f2, m.f3, m.f5, -c.dTchia2dY * S.Htdv[g - 1], c.dTchia2dY * S.Htdv[g],
+                 R(S.z[g]) - flux_y(S, c, g)};
 }
 
 template <class R>

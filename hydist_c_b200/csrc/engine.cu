@@ -527,7 +527,7 @@ int new_handle(const HydistParams* p, const HydistOptions* o, int device, int M,
 // The arrays only this library uses: smoothing buffers, boundary weights,
 // line-solver scratch, flags, counters, the device clock.
 // The FP64 / FP32 arrays only this library uses: smoothing buffers and the
-// line-solver scratch (3 values per unknown, 4 lines per slot, one slot per
+// line-solver scratch (4 values per unknown, 4 lines per slot, one slot per
 // CTA of the persistent sweep grid).
 template <class R>
 int bulk_private(HydistHandle* h, StateT<R>& B) {
@@ -540,12 +540,12 @@ int bulk_private(HydistHandle* h, StateT<R>& B) {
   int nsm = 0;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
   B.lslots = 2 * nsm;
-  const size_t U = (size_t)2 * std::max(S.M, S.N);
+  const size_t U = (size_t)std::max(S.M, S.N);
   // at least 4 (max(M,N)+3) doubles: preprocess_data borrows it as FP64;
-  // the refined FP32 form keeps 7 values per unknown (its refinement stores
+  // the refined FP32 form keeps 8 values per unknown (its refinement stores
   // the rows)
-  const size_t arrays = S.refine ? 7 : 3;
-  TRY(dalloc(h, &B.lscratch, std::max((size_t)B.lslots * arrays * U * 4, 8 * U + 64)));
+  const size_t arrays = S.refine ? 8 : 4;
+  TRY(dalloc(h, &B.lscratch, std::max((size_t)B.lslots * arrays * U * 4, 16 * U + 128)));
   return HYDIST_OK;
 }
 

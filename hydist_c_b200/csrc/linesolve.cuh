@@ -38,7 +38,7 @@ constexpr int XPB = 8;  // lines per CTA of the 128-chunk column sweeps
 // One wet segment of a line, with its system layout.
 struct SegD {
   int first, last;
-  int off, rend;  // absolute rows [off, rend] of the segment's system
+  int off, rend;  // cells off..rend hold the segment's unknowns
   unsigned char br1, br2, ran, qfirst, last_kind, xq_first, xq_last, pad;
 };
 
@@ -114,7 +114,6 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
   R* sc_y = scr + UL;
   R* sc_v = scr + 2 * UL;
   const int ncells = G0.cells_per_line();
-  const int upc = Gen::UPC;
 
   // one group of L lines: gg-th of its scenario, with that scenario's G
   auto solve_group = [&](const Gen& G, int gg) {
@@ -129,7 +128,7 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
     // ---- chunk bounds (balanced split of the line's cells)
     const int c0 = (int)(((long long)k * ncells) / P);
     const int c1 = (int)(((long long)(k + 1) * ncells) / P);
-    const int q0 = c0 * upc, nu = (c1 - c0) * upc;  // chunk unknowns [q0, q0+nu)
+    const int q0 = c0, nu = c1 - c0;  // chunk unknowns [q0, q0+nu)
 
     // ---- pass A: forward elimination of the interior, separator row
     {
@@ -140,46 +139,43 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
       // first interior row in terms of both separators, accumulated forward:
       // x_0 = sum_k P_k (y'_k + v'_k x_L) + P_L x_R, P_0 = 1, P_{k+1} = -c'_k P_k
       R Pk = 1, fy = 0, fv = 0;
-      int s = 0;
       for (int c = c0; c < c1; ++c) {
         W.cell(G, LS, c);
-#pragma unroll
-        for (int e = 0; e < Gen::UPC; ++e, ++s) {
-          R A, B, C, D;
-          W.row(G, LS, e, A, B, C, D);
-          if (s == nu - 1) {
-            sh.sep[0][cidx] = A;
-            sh.sep[1][cidx] = B;
-            sh.sep[2][cidx] = C;
-            sh.sep[3][cidx] = D;
+        R A, B, C, D;
+        W.row(G, LS, A, B, C, D);
+        const size_t o = (size_t)c * L + l;
+        if constexpr (Gen::AUX != 0) scr[Gen::AUX * UL + o] = W.aux;
+        if (c == c1 - 1) {
+          sh.sep[0][cidx] = A;
+          sh.sep[1][cidx] = B;
+          sh.sep[2][cidx] = C;
+          sh.sep[3][cidx] = D;
+        } else {
+          R m;
+          if (c == c0) {
+            m = rcp(B);
+            cp = C * m;
+            yp = D * m;
+            vp = -A * m;
           } else {
-            R m;
-            if (s == 0) {
-              m = rcp(B);
-              cp = C * m;
-              yp = D * m;
-              vp = -A * m;
-            } else {
-              m = rcp(B - A * cp);
-              yp = (D - A * yp) * m;
-              vp = -A * vp * m;
-              cp = C * m;
-            }
-            const size_t o = (size_t)(q0 + s) * L + l;
-            if constexpr (Gen::REFINE && !Gen::ROWS_AGAIN) {
-              // the interior rows, for the residual
-              scr[3 * UL + o] = A;
-              scr[4 * UL + o] = B;
-              scr[5 * UL + o] = C;
-              scr[6 * UL + o] = D;
-            }
-            sc_c[o] = cp;
-            sc_y[o] = yp;
-            sc_v[o] = vp;
-            fy += Pk * yp;
-            fv += Pk * vp;
-            Pk *= -cp;
+            m = rcp(B - A * cp);
+            yp = (D - A * yp) * m;
+            vp = -A * vp * m;
+            cp = C * m;
           }
+          if constexpr (Gen::REFINE && !Gen::ROWS_AGAIN) {
+            // the interior rows, for the residual
+            scr[3 * UL + o] = A;
+            scr[4 * UL + o] = B;
+            scr[5 * UL + o] = C;
+            scr[6 * UL + o] = D;
+          }
+          sc_c[o] = cp;
+          sc_y[o] = yp;
+          sc_v[o] = vp;
+          fy += Pk * yp;
+          fv += Pk * vp;
+          Pk *= -cp;
         }
       }
       // first and last interior rows in terms of the neighbouring separators
@@ -254,15 +250,18 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
       const R xl = (k > 0) ? sh.xsep[cidx - L] : R(0);
       typename Gen::Emitter E;
       E.init(G, LS, line);
-      E.emit(G, LS, sh.xlast[l], q0 + nu - 1, xr);
-      R xn = xr;
+      // an unknown is emitted once the one before it is known
+      R xn = xr, ax = 0;
 #pragma unroll 4
       for (int t = nu - 2; t >= 0; --t) {
         const size_t o = (size_t)(q0 + t) * L + l;
         const R x = sc_y[o] + sc_v[o] * xl - sc_c[o] * xn;
-        E.emit(G, LS, sh.xlast[l], q0 + t, x);
+        if constexpr (Gen::AUX != 0) ax = scr[Gen::AUX * UL + o + L];
+        E.emit(G, LS, sh.xlast[l], q0 + t + 1, xn, x, ax);
         xn = x;
       }
+      if constexpr (Gen::AUX != 0) ax = scr[Gen::AUX * UL + (size_t)q0 * L + l];
+      E.emit(G, LS, sh.xlast[l], q0, xn, xl, ax);
     } else {
       // one refinement pass. The back substitution stores x over y' and, as
       // soon as x_{t-1..t+1} are known, takes row t's residual
@@ -339,8 +338,7 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
         // the unknown left of the separator: the chunk's last interior one,
         // or the previous chunk's separator; right of it: the next chunk's
         // first unknown, its separator where that chunk holds nothing else
-        const int nu_next = (k + 1 < P)
-            ? ((int)(((long long)(k + 2) * ncells) / P) - c1) * upc : 0;
+        const int nu_next = (k + 1 < P) ? (int)(((long long)(k + 2) * ncells) / P) - c1 : 0;
         const R xm = nu >= 2 ? x_before_sep : (q > 0 ? xl : R(0));
         const R xp = q + 1 < U ? (nu_next >= 2 ? sc_y[o + L] : sh.xsep[cidx + L]) : R(0);
         const R as = sh.sep[0][cidx], bs = sh.sep[1][cidx], cs = sh.sep[2][cidx],
@@ -370,14 +368,21 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
         const R dl = (k > 0) ? sh.xsep[cidx - L] : R(0);
         typename Gen::Emitter E;
         E.init_fwd(G, LS, line);
-        R dp = dl;
+        R dp = dl, ax = 0;
+        double xm = (double)xl + (double)dl;  // the refined unknown before
         for (int t = 0; t <= nu - 2; ++t) {
           const size_t o = (size_t)(q0 + t) * L + l;
           const R d = sD[o] - sA[o] * dp - sC[o] * dr;
-          E.template emit<true>(G, LS, sh.xlast[l], q0 + t, (double)sc_y[o] + (double)d);
+          const double x = (double)sc_y[o] + (double)d;
+          if constexpr (Gen::AUX != 0) ax = scr[Gen::AUX * UL + o];
+          E.template emit<true>(G, LS, sh.xlast[l], q0 + t, x, xm, ax);
           dp = d;
+          xm = x;
         }
-        if (nu >= 1) E.template emit<true>(G, LS, sh.xlast[l], q0 + nu - 1, (double)xr + (double)dr);
+        if (nu >= 1) {
+          if constexpr (Gen::AUX != 0) ax = scr[Gen::AUX * UL + (size_t)(q0 + nu - 1) * L + l];
+          E.template emit<true>(G, LS, sh.xlast[l], q0 + nu - 1, (double)xr + (double)dr, xm, ax);
+        }
       }
     }
     __syncthreads();

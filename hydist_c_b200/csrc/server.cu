@@ -141,8 +141,8 @@ int64_t hydist_scenario_bytes(int32_t M, int32_t N) {
   int nsm = 148;
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const uint64_t U = 2 * (uint64_t)(M > N ? M : N);
-  t += r((uint64_t)2 * nsm * 3 * U * 4 * 8 + 64);  // line-solver scratch
+  const uint64_t U = (uint64_t)(M > N ? M : N);
+  t += r((uint64_t)2 * nsm * 4 * U * 4 * 8 + 64);  // line-solver scratch
   t += 24 * r(4096);                              // series, tables, flags, clock, ...
   return (int64_t)t;
 }

@@ -1,11 +1,14 @@
 // sweep.cu -- the hydraulic ADI line sweeps on the partitioned line solver.
 //
 // HydroGen<0> is the x sweep (UZ half-step: lines are columns j, cells run
-// along i, unknowns z_i and u_i interleaved); HydroGen<1> is the y sweep (VZ
-// half-step: lines are rows i, cells along j, unknowns z_j and v_j). Both
-// generate the reference's tridiagonal rows on the fly (assembly.cuh) and
-// write the extraction of UZSolver_extract_solution / VZSolver_extract_
-// solution (UVZSolver_multithread.cpp:472-603) directly from the solution.
+// along i, unknowns u_i); HydroGen<1> is the y sweep (VZ half-step: lines are
+// rows i, cells along j, unknowns v_j). Both generate the rows of the
+// velocities alone (the reference's interleaved z, u system with its
+// continuity rows eliminated, make_row) on the fly (assembly.cuh) and write
+// the extraction of UZSolver_extract_solution / VZSolver_extract_solution
+// (UVZSolver_multithread.cpp:472-603) directly from the solution, each cell's
+// level by its continuity row. FP64 on 2048x1024, against the interleaved
+// system: XXX
 #include "assembly.cuh"
 #include "common.cuh"
 
@@ -33,8 +36,10 @@ struct HydroGen {
   static constexpr bool REFINE = REF;
   // the rows are generated from the stencils: the refinement keeps them
   static constexpr bool ROWS_AGAIN = false;
-  static constexpr int SCRATCH_ARRAYS = REFINE ? 7 : 3;
-  static constexpr int UPC = 2;
+  // c', y', v', with refinement the rows A, B, C, D, and the emitter's value
+  static constexpr int AUX = REFINE ? 7 : 3;
+  static constexpr int SCRATCH_ARRAYS = AUX + 1;
+  static constexpr bool HYDRO = true;
   static constexpr int DIRECTION = DIR;
   // x sweeps (columns, 4 adjacent per warp) run faster with two CTAs per SM
   // despite the register cap, and so do the FP32 y sweeps; the FP64 and the
@@ -55,17 +60,10 @@ struct HydroGen {
   }
   __device__ int lines() const { return nl; }
   __device__ int cells_per_line() const { return DIR == 0 ? S.N - 1 : S.M - 1; }
-  __device__ int unknowns_per_line() const { return 2 * cells_per_line(); }
+  __device__ int unknowns_per_line() const { return cells_per_line(); }
   __device__ int end_pos() const { return DIR == 0 ? S.N : S.M; }
   // field index of position p on line position lp
   __device__ int at(int lp, int p) const { return DIR == 0 ? p * S.W + lp : lp * S.W + p; }
-  // the preindex values of a cell, from its stencil (computed where the
-  // walker reaches the cell: a separate per-cell pass writing them to HBM
-  // ahead of the sweep costs more in traffic and a launch than it saves)
-  __device__ PreT<R> pre(int lp, int p) const {
-    return DIR == 0 ? pre_x(S, c, p, lp) : pre_y(S, c, lp, p);
-  }
-  __device__ R* vel() const { return DIR == 0 ? S.tu : S.tv; }
   // the VZ extraction reaches columns j <= N only (UVZSolver_multithread.cpp:851)
   __device__ bool extract_ok(int p) const { return DIR == 0 ? true : p <= S.N; }
 
@@ -104,8 +102,8 @@ struct HydroGen {
     const LineSys L = line_sys(first, last, br1, br2, q1, q2, end_pos());
     d.first = first;
     d.last = last;
-    d.off = L.off;
-    d.rend = L.off + L.sn;
+    d.off = first;
+    d.rend = last - 1;
     d.br1 = br1;
     d.br2 = br2;
     d.ran = L.ran;
@@ -115,90 +113,108 @@ struct HydroGen {
     d.xq_last = q2;
   }
 
-  // Generates the rows of the line system cell by cell (two unknowns per cell).
+  // One cell's continuity values: depth at its velocity point, level, and the
+  // cross-line flux w (continuity: z_new = z - w + k (Ha_{-} a_{-} - Ha a)).
+  struct Cont {
+    R H, w;
+    double z;
+  };
+  __device__ R depth(int g) const { return DIR == 0 ? S.Htdu[g] : S.Htdv[g]; }
+  __device__ Cont cont(int g) const {
+    return Cont{depth(g), DIR == 0 ? flux_x(S, c, g) : flux_y(S, c, g), S.z[g]};
+  }
+  // the prescribed velocities beyond the line's first and last cells
+  __device__ R q_first(int lp) const { return DIR == 0 ? S.ubt[lp] : S.vbd[lp]; }
+  __device__ R q_last(int lp) const { return DIR == 0 ? S.ubp[lp] : S.vbt[lp]; }
+
+  // The row of the velocity a_pos of cell pos, first <= pos < last of segment
+  // d: the momentum row with the levels of the cells pos and pos + 1 replaced
+  // by their continuity rows,
+  //   (f1 + e Ha_{-}) a_{-} + (f2 - 2 e Ha) a + (f3 + e Ha_{+}) a_{+}
+  //     = f5 + f4 (d2_{+} - d2),   e = f4 k, d2 = z - w,
+  // which is what eliminating the z unknowns of the reference's interleaved
+  // system (_calculate_abcd + _calculate_matrix_coeff, UVZSolver_
+  // multithread.cpp:280-470) leaves: its f1/a2 and f3/c2 terms cancel. Half
+  // the unknowns, and one division per cell instead of four. Ends: a solid or
+  // discharge end prescribes the velocity beyond it; at an open end (level
+  // given) the reference keeps the substituted f1/a2 (f3/c2) term.
+  __device__ void make_row(const SegD& d, int lp, int pos, MomF<R> m, R Hm, const Cont& c0,
+                           const Cont& c1, R& A, R& B, R& C, R& D) const {
+    const R kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY, e = f4 * kk;
+    if (d.last - 1 <= d.first) m.f1 = m.f3 = 0;  // a two-cell segment
+    A = m.f1 + e * Hm;
+    B = m.f2 - 2 * e * c0.H;
+    C = m.f3 + e * c1.H;
+    D = m.f5 + f4 * (R(c1.z - c0.z) - (c1.w - c0.w));
+    if (pos == d.first) {
+      if (d.qfirst) {
+        D -= A * q_first(lp);
+      } else if (!d.ran) {
+        // level given at the first cell
+        const double zl = S.tz[at(lp, pos)];
+        const R ra = -m.f1 / (kk * Hm);
+        B = m.f2 - (ra * kk + e) * c0.H;
+        D = m.f5 + f4 * (R(c1.z - zl) - c1.w) - ra * (R(c0.z - zl) - c0.w);
+      }
+      A = 0;
+    }
+    if (pos == d.last - 1) {
+      if (d.last_kind == 1) {
+        D -= C * q_last(lp);
+      } else if (d.last_kind == 2) {
+        const double zr = S.tz[at(lp, d.last)];
+        const R rc = m.f3 / (kk * c1.H);
+        B += (f4 + rc) * kk * c0.H;
+        // (between two given levels one velocity alone: the reference's last
+        // row overwrites the first level's term)
+        if (pos == d.first && !d.ran) D = m.f5 + f4 * R(zr);
+        else D += (f4 + rc) * (R(zr - c1.z) + c1.w);
+      }
+      C = 0;
+    }
+  }
+
+  // Generates the rows of the line system cell by cell.
   struct Walker {
     int lp, si, pos, prev;
     bool in;
-    PreT<R> Pc, Pn;
-    MomT<R> Mi;
-    __device__ void init(const HydroGen& G, const LineSeg& LS, int line, int c0) {
+    R Hm, aux;  // depth before c0; what the emitter needs to form the level
+    Cont c0, c1;
+    MomF<R> m;
+    __device__ void init(const HydroGen& G, const LineSeg& LS, int line, int first_cell) {
       lp = line + G.lp0;
       si = 0;
       prev = -10;
       in = false;
     }
-    __device__ void cell(const HydroGen& G, const LineSeg& LS, int c) {
-      pos = c + 2;
-      while (si < LS.nseg && LS.s[si].last < pos) ++si;
+    __device__ void cell(const HydroGen& G, const LineSeg& LS, int cc) {
+      pos = cc + 2;
+      while (si < LS.nseg && LS.s[si].last <= pos) ++si;
       in = si < LS.nseg && LS.s[si].first <= pos;
       if (!in) {
         prev = -10;
         return;
       }
-      const SegD& d = LS.s[si];
-      if (prev == pos - 1 && pos > d.first) Pc = Pn;
-      else Pc = G.pre(lp, pos);
-      if (pos + 1 <= d.last) Pn = G.pre(lp, pos + 1);
-      else Pn = Pc;
-      if (pos <= d.last - 1 || pos == d.first) Mi = abcd(Pc, Pn, pos, d.first, d.last, G.f4, d.br1, d.br2);
-      else Mi = MomT<R>{0, 0, 0, 0};
+      if (prev == pos - 1) {
+        Hm = c0.H;
+        c0 = c1;
+      } else {
+        Hm = G.depth(G.at(lp, pos - 1));
+        c0 = G.cont(G.at(lp, pos));
+      }
+      c1 = G.cont(G.at(lp, pos + 1));
+      m = DIR == 0 ? mom_x(G.S, G.c, pos, lp) : mom_y(G.S, G.c, lp, pos);
       prev = pos;
+      aux = sizeof(R) == 8 ? R(c0.z - c0.w) : c0.w;
     }
-    __device__ void row(const HydroGen& G, const LineSeg& LS, int e, R& A, R& B, R& C,
-                        R& D) const {
+    __device__ void row(const HydroGen& G, const LineSeg& LS, R& A, R& B, R& C, R& D) const {
       if (!in) {
         A = 0; B = 1; C = 0; D = 0;
         return;
       }
-      G.rows_in(LS.s[si], lp, pos, Pc, Pn, Mi, e, A, B, C, D);
+      G.make_row(LS.s[si], lp, pos, m, Hm, c0, c1, A, B, C, D);
     }
   };
-
-  // Row 2*pos + e of the line system at line position lp, for a cell pos of
-  // segment d with its preindex values Pc, those of the next cell Pn (Pc at
-  // the segment's last cell) and its momentum coefficients Mi.
-  __device__ void rows_in(const SegD& d, int lp, int pos, const PreT<R>& Pc, const PreT<R>& Pn,
-                          const MomT<R>& Mi, int e, R& A, R& B, R& C, R& D) const {
-    const int r = 2 * pos + e;
-    if (r < d.off || r > d.rend) {
-      A = 0; B = 1; C = 0; D = 0;
-      return;
-    }
-    const bool even = (r & 1) == 0;
-    if ((bool)d.ran == even) {
-      const PreT<R>& P = d.ran ? Pc : Pn;
-      A = P.a2; B = 1; C = P.c2; D = P.d2;
-    } else {
-      A = Mi.a1; B = Mi.b1; C = Mi.c1; D = Mi.d1;
-    }
-    if (r == d.off) {
-      if (d.ran) {
-        if (d.qfirst) {
-          const R ub = DIR == 0 ? S.ubt[lp] : S.vbd[lp];
-          D = Pc.d2 - Pc.a2 * ub;
-        } else {
-          D = Pc.d2;
-        }
-      } else {
-        const R TZ_l = R(S.tz[at(lp, d.first)]);
-        D = Mi.d1 - Mi.a1 * TZ_l;
-      }
-      A = 0;  // the system starts here
-    }
-    if (r == d.rend) {
-      const PreT<R>& PL = (pos == d.last) ? Pc : Pn;
-      if (d.last_kind == 1) {
-        const R ub = DIR == 0 ? S.ubp[lp] : S.vbt[lp];
-        A = PL.a2; B = 1; D = PL.d2 - PL.c2 * ub;
-      } else if (d.last_kind == 2) {
-        const R TZ_r = R(S.tz[at(lp, d.last)]);
-        A = Mi.a1; B = Mi.b1; D = Mi.d1 - Mi.c1 * TZ_r;
-      } else {
-        A = PL.a2; B = 1; D = PL.d2;
-      }
-      C = 0;  // and ends here
-    }
-  }
 
   // (the refinement reads the stored rows: no cursor over them)
   struct RowCursor {
@@ -206,8 +222,9 @@ struct HydroGen {
     __device__ void row(const HydroGen&, const LineSeg&, int, R&, R&, R&, R&) {}
   };
 
-  // Writes each solved unknown to t_z / t_u (t_v) as the extraction does.
-  // FWD: the unknowns come in increasing order (init_fwd), else decreasing.
+  // Writes each solved velocity and its cell's level to t_u (t_v) / t_z as
+  // the extraction does. FWD: the unknowns come in increasing order
+  // (init_fwd), else decreasing.
   struct Emitter {
     int lp, si;
     __device__ void init(const HydroGen& G, const LineSeg& LS, int line) {
@@ -218,42 +235,37 @@ struct HydroGen {
       lp = line + G.lp0;
       si = -1;
     }
+    // unknown q with value x, the one before it xm, its cell's aux
     template <bool FWD = false>
-    __device__ void emit(const HydroGen& G, const LineSeg& LS, double* xlast, int q, double x) {
-      const int r = q + 4, pos = r >> 1;
+    __device__ void emit(const HydroGen& G, const LineSeg& LS, double* xlast, int q, double x,
+                         double xm, R aux) {
+      const int pos = q + 2;
       if constexpr (FWD) {
         while (si + 1 < LS.nseg && LS.s[si + 1].first <= pos) ++si;
       } else {
         while (si >= 0 && LS.s[si].first > pos) --si;
       }
       if (si < 0) return;
-      G.store_in(LS.s[si], xlast + si, lp, q, x);
+      G.store_in(LS.s[si], xlast + si, lp, pos, x, xm, aux);
     }
   };
 
-  // The extraction of unknown q (row q + 4) of segment d on line position
-  // lp; the segment's last row also goes to *xl for the end fix-up.
-  __device__ void store_in(const SegD& d, double* xl, int lp, int q, double x) const {
-    const int r = q + 4, pos = r >> 1;
-    if (pos > d.last || r < d.off || r > d.rend) return;
-    if (r == d.rend) *xl = x;
-    R* v = vel_ptr();
-    if (d.ran) {
-      const int i = r >> 1;
-      if (i < d.last && extract_ok(i)) {
-        if (r & 1) v[at(lp, i)] = x;
-        else S.tz[at(lp, i)] = x;
-      }
-    } else {
-      if (r == 2 * d.first) {
-        if (extract_ok(d.first)) v[at(lp, d.first)] = x;
-      } else {
-        const int i = (r + 1) >> 1;
-        if (i > d.first && i < d.last && extract_ok(i)) {
-          if (r & 1) S.tz[at(lp, i)] = x;
-          else v[at(lp, i)] = x;
-        }
-      }
+  // The extraction of the velocity x of cell pos of segment d on line position
+  // lp, and of the cell's level by continuity (the first cell's where it is
+  // not given); the segment's last velocity also goes to *xl for the end
+  // fix-up. aux: d2 = z - w in FP64, w in FP32 (the level itself stays FP64).
+  __device__ void store_in(const SegD& d, double* xl, int lp, int pos, double x, double xm,
+                           R aux) const {
+    if (pos >= d.last) return;
+    if (pos == d.last - 1) *xl = x;
+    if (!extract_ok(pos)) return;
+    const int g = at(lp, pos);
+    vel_ptr()[g] = x;
+    if (pos > d.first || d.ran) {
+      if (pos == d.first) xm = d.qfirst ? (double)q_first(lp) : 0.0;
+      const double kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
+      const double base = sizeof(R) == 8 ? (double)aux : S.z[g] - (double)aux;
+      S.tz[g] = base + kk * ((double)depth(DIR == 0 ? g - S.W : g - 1) * xm - (double)depth(g) * x);
     }
   }
 
@@ -263,27 +275,40 @@ struct HydroGen {
     const int lp = line + lp0, first = d.first, last = d.last;
     R* vel = vel_ptr();
     double* tz = S.tz;
+    const double kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
     if (first < last && extract_ok(first)) {
       if (d.br1) {
         vel[at(lp, first - 1)] = 0;
       } else if (d.xq_first && first == 2) {
-        vel[at(lp, first - 1)] = DIR == 0 ? S.ubt[lp] : S.vbd[lp];
+        vel[at(lp, first - 1)] = q_first(lp);
       } else {
-        const PreT<R> Pf = pre(lp, first);
-        vel[at(lp, first - 1)] = (Pf.d2 - tz[at(lp, first)] - Pf.c2 * vel[at(lp, first)]) / Pf.a2;
+        const Cont cf = cont(at(lp, first));
+        vel[at(lp, first - 1)] = ((cf.z - cf.w) - tz[at(lp, first)] - kk * cf.H * vel[at(lp, first)]) /
+                                 (-kk * depth(at(lp, first - 1)));
       }
     }
     if (!extract_ok(last)) return;
-    const double xl = (d.rend >= d.off) ? xlast[s] : 0.0;
+    const Cont cl = cont(at(lp, last));
+    const double d2 = cl.z - cl.w;
+    // the value of the reference system's last row: the last cell's level, the
+    // last velocity where that level is given, 0 where no row was solved
+    double xl = 0.0;
+    if (last > first) {
+      xl = d.last_kind == 2 ? xlast[s]
+                            : d2 + kk * depth(at(lp, last - 1)) * xlast[s] -
+                                  (d.last_kind == 1 ? kk * cl.H * q_last(lp) : 0.0);
+    } else if (d.ran && d.last_kind != 2) {
+      xl = d2 - (d.last_kind == 1 ? kk * cl.H * q_last(lp) : 0.0);
+    }
     if (d.br2) {
       vel[at(lp, last)] = 0;
       tz[at(lp, last)] = xl;
     } else if (d.xq_last && last == end_pos()) {
-      vel[at(lp, last)] = DIR == 0 ? S.ubp[lp] : S.vbt[lp];
+      vel[at(lp, last)] = q_last(lp);
       tz[at(lp, last)] = xl;
     } else {
-      const PreT<R> Pl = pre(lp, last);
-      vel[at(lp, last)] = (Pl.d2 - Pl.a2 * vel[at(lp, last - 1)] - tz[at(lp, last)]) / Pl.c2;
+      vel[at(lp, last)] =
+          (d2 + kk * depth(at(lp, last - 1)) * vel[at(lp, last - 1)] - tz[at(lp, last)]) / (kk * cl.H);
     }
   }
   __device__ R* vel_ptr() const { return DIR == 0 ? S.tu : S.tv; }
@@ -362,7 +387,7 @@ static int resident_slots() {
 template <class Gen>
 static int launch_lines(const Gen& G, int P, int lines, int lslots, cudaStream_t st,
                         const Batch<typename Gen::Real>& b = {}) {
-  if constexpr (Gen::DIRECTION == 1 && Gen::UPC == 2 && !Gen::REFINE &&
+  if constexpr (Gen::DIRECTION == 1 && Gen::HYDRO && !Gen::REFINE &&
                 sizeof(typename Gen::Real) == 4) {
     if (P == 128) {
       // the FP32 hydraulic row sweep: groups of 8 rows, one 1024-thread CTA
@@ -376,7 +401,7 @@ static int launch_lines(const Gen& G, int P, int lines, int lslots, cudaStream_t
       return 1;
     }
   }
-  if constexpr (Gen::DIRECTION == 1 && Gen::UPC == 2 && Gen::REFINE) {
+  if constexpr (Gen::DIRECTION == 1 && Gen::HYDRO && Gen::REFINE) {
     if (P == 128 && b.n == 0) {
       // the refined hydraulic row sweep: groups of 8 rows of 64 chunks (one
       // 512-thread CTA per SM): 0.210 -> 0.204 ms on 2048x1024 (the FP64 and
@@ -387,7 +412,7 @@ static int launch_lines(const Gen& G, int P, int lines, int lslots, cudaStream_t
     }
   }
   if constexpr (Gen::DIRECTION == 1) {
-    if (P == 64 || (P == 128 && Gen::UPC == 1 && sizeof(typename Gen::Real) == 4)) {
+    if (P == 64 || (P == 128 && !Gen::HYDRO && sizeof(typename Gen::Real) == 4)) {
       // row sweeps of 64 chunks (rows of 256 to 511 cells), and the FP32
       // concentration row sweeps of 128: groups of 8 adjacent rows (their
       // stencil rows shared through L1 by twice as many lines). The
@@ -401,7 +426,7 @@ static int launch_lines(const Gen& G, int P, int lines, int lslots, cudaStream_t
       const int grid = (int)std::min<long long>(total, lslots / 2);
       if (P == 64) {
         launch_gen<Gen, 64, XPB>(G, st, grid, 0, (int)total, b, b.n > 0 ? g8 : 0);
-      } else if constexpr (Gen::UPC == 1 && sizeof(typename Gen::Real) == 4) {
+      } else if constexpr (!Gen::HYDRO && sizeof(typename Gen::Real) == 4) {
         launch_gen<Gen, 128, XPB>(G, st, grid, 0, (int)total, b, b.n > 0 ? g8 : 0);
       }
       return 1;
@@ -463,7 +488,7 @@ static int launch_lines(const Gen& G, int P, int lines, int lslots, cudaStream_t
 }
 
 // Scratch slots for a sweep of lines of `unknowns` unknowns in P chunks:
-// the scratch holds StateT::lslots slots of lines of 2*max(M, N) unknowns,
+// the scratch holds StateT::lslots slots of lines of max(M, N) unknowns,
 // so a sweep of shorter lines has proportionally more. Only the solvers of
 // fewer than 128 chunks (smaller CTAs, more of them resident per SM) use
 // them: their grid may then exceed the CTAs resident at once, the extra
@@ -472,7 +497,7 @@ static int launch_lines(const Gen& G, int P, int lines, int lslots, cudaStream_t
 template <class R>
 static int sweep_slots(const StateT<R>& S, int unknowns, int P) {
   if (P >= 128) return S.lslots;
-  const int umax = 2 * std::max(S.M, S.N);
+  const int umax = std::max(S.M, S.N);
   return S.lslots * std::max(1, umax / std::max(unknowns, 1));
 }
 
@@ -486,7 +511,7 @@ static int launch_dir(const StateT<R>& S, const CoefT<R>& c, cudaStream_t st, in
   G.nl = DIR == 0 ? S.x_hi - S.x_lo + 1 : S.N - S.y_lo + 1;
   if (G.nl <= 0) return 0;
   const int ncells = DIR == 0 ? S.N - 1 : S.M - 1;
-  return launch_lines(G, P, G.nl, sweep_slots(S, 2 * ncells, P), st, b);
+  return launch_lines(G, P, G.nl, sweep_slots(S, ncells, P), st, b);
 }
 
 // ---------------------------------------------------------------------
@@ -500,8 +525,9 @@ struct FSGen {
   static constexpr bool REFINE = REF;
   // the rows are in StateT::pre (k_fs_rows): the refinement reads them again
   static constexpr bool ROWS_AGAIN = true;
+  static constexpr int AUX = 0;  // the emitter needs nothing but the solution
   static constexpr int SCRATCH_ARRAYS = REFINE ? 4 : 3;
-  static constexpr int UPC = 1;
+  static constexpr bool HYDRO = false;
   static constexpr int DIRECTION = DIR;
   // two CTAs per SM in both directions and precisions
   static constexpr int MIN_BLOCKS = 2;
@@ -568,8 +594,7 @@ struct FSGen {
       while (si < LS.nseg && LS.s[si].last < pos) ++si;
       in = si < LS.nseg && LS.s[si].off <= pos && pos <= LS.s[si].rend;
     }
-    __device__ void row(const FSGen& G, const LineSeg& LS, int e, R& A, R& B, R& C,
-                        R& D) const {
+    __device__ void row(const FSGen& G, const LineSeg& LS, R& A, R& B, R& C, R& D) const {
       if (!in) {
         A = 0; B = 1; C = 0; D = 0;
         return;
@@ -640,7 +665,8 @@ struct FSGen {
       si = -1;
     }
     template <bool FWD = false>
-    __device__ void emit(const FSGen& G, const LineSeg& LS, double* xlast, int q, double x) {
+    __device__ void emit(const FSGen& G, const LineSeg& LS, double* xlast, int q, double x, double,
+                         R) {
       const int pos = q + 2;
       if constexpr (FWD) {
         while (si + 1 < LS.nseg && LS.s[si + 1].first <= pos) ++si;
