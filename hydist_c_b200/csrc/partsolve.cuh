@@ -128,12 +128,11 @@ __device__ __forceinline__ void part_back(T* rA, T* rC, T* rD, int q0, int nu, i
   }
 }
 
-// Reduced-system work space of a CTA of NT threads.
+// Reduced-system work space of a CTA of NT threads: what each warp's first
+// and last chunks give the others (tridiag.cu, tile_reduce).
 template <class T, int NT>
 struct PartCtaShared {
-  T tri[3][NT];  // yF vF wF of each chunk (read by the previous chunk)
-  T red[4][NT];
-  T xsep[NT];
+  T blk[NT / 32][8];
 };
 
 // Warp-wide solve (all 32 lanes call it; the rows are in the warp's slice of
@@ -157,33 +156,19 @@ __device__ void part_solve_warp(T* rA, T* rB, T* rC, T* rD, const PartGeom& g, i
     rc = sep[2] * (nx ? wF : T(0));
     rd = sep[3] - sep[0] * tri[3] - sep[2] * (nx ? yF : T(0));
   }
+  // (rows normalised to a unit diagonal: one reciprocal per level)
+  const T inv = T(1) / rb;
+  T a = ra * inv, c = rc * inv, d = rd * inv;
   for (int st = 1; st < P; st <<= 1) {
-    T am = __shfl_up_sync(full, ra, st), bm = __shfl_up_sync(full, rb, st);
-    T cm = __shfl_up_sync(full, rc, st), dm = __shfl_up_sync(full, rd, st);
-    T an = __shfl_down_sync(full, ra, st), bn = __shfl_down_sync(full, rb, st);
-    T cn = __shfl_down_sync(full, rc, st), dn = __shfl_down_sync(full, rd, st);
-    if (!(k < P && k - st >= 0)) {
-      am = 0;
-      bm = 1;
-      cm = 0;
-      dm = 0;
-    }
-    if (!(k + st < P)) {
-      an = 0;
-      bn = 1;
-      cn = 0;
-      dn = 0;
-    }
-    const T k1 = ra / bm, k2 = rc / bn;
-    const T na = -am * k1, nc = -cn * k2;
-    const T nb = rb - cm * k1 - an * k2;
-    const T nd = rd - dm * k1 - dn * k2;
-    ra = na;
-    rb = nb;
-    rc = nc;
-    rd = nd;
+    const T am = __shfl_up_sync(full, a, st), cm = __shfl_up_sync(full, c, st), dm = __shfl_up_sync(full, d, st);
+    const T an = __shfl_down_sync(full, a, st), cn = __shfl_down_sync(full, c, st), dn = __shfl_down_sync(full, d, st);
+    const T au = k >= st ? a : T(0), cd = k + st < P ? c : T(0);
+    const T r = T(1) / (T(1) - au * cm - cd * an);
+    d = (d - au * dm - cd * dn) * r;
+    a = -au * am * r;
+    c = -cd * cn * r;
   }
-  const T xs = rd / rb;
+  const T xs = d;
   const T xl = __shfl_up_sync(full, xs, 1);
   if (k < P) part_back(rA, rC, rD, q0, nu, S, k > 0 ? xl : T(0), xs);
   __syncwarp();

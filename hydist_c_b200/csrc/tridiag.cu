@@ -8,20 +8,24 @@
 // Packed batch: system s occupies rows [off[s], off[s]+len[s]); dl of its
 // first row and du of its last row are ignored.
 //
-// Three solvers, chosen per length band:
+// Four solvers, chosen per length band:
 //   Thomas      one thread per system, in place in global memory (any length);
 //   warp        one warp per system staged in shared memory, partition
 //               method with a shuffle PCR of the 32 chunk separators
 //               (systems up to GT_WARP_MAX rows);
-//   CTA         one CTA of 256 or 512 threads per system, its rows staged
+//   CTA         one CTA of 128, 256 or 512 threads per system, its rows staged
 //               in shared memory by TMA bulk copies (the next system's while
-//               one is solved, where two fit), partition method with a
-//               shared-memory PCR (systems up to the shared memory of one
-//               CTA, about 6000 FP64 / 12000 FP32 rows).
-// A classification kernel files each system under its length band on the
-// device; the bands' solvers then run over their lists. The autotuner times
-// the feasible solvers per band on synthetic diagonally dominant batches and
-// keeps the fastest (per device and dtype).
+//               one is solved, where two fit), partition method over chunks,
+//               warps and the CTA (systems up to the shared memory of one
+//               CTA, about 6000 FP64 / 12000 FP32 rows);
+//   tiles       longer systems cut into tiles of one CTA each: a pass that
+//               reduces every tile to its last row, a small solve of those
+//               rows per system, a pass that solves the tiles.
+// A classification kernel files each system under its length class on the
+// device (the public bands, the longer ones split so that a class's shared
+// memory fits its systems more closely); the classes' solvers then run over
+// their lists. The autotuner times the feasible solvers per band on synthetic
+// diagonally dominant batches and keeps the fastest (per device and dtype).
 #include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 
@@ -56,6 +60,31 @@ __host__ __device__ inline int gt_band_hi(int b) {
     default: return INT_MAX;
   }
 }
+
+// Length classes of the lists: the bands, those above 512 rows split where
+// the systems' rows in shared memory set how many CTAs an SM holds (three of
+// 2048 FP64 rows, six of 1024).
+constexpr int GT_NC = 10;
+__host__ __device__ inline int gt_class_hi(int k) {
+  switch (k) {
+    case 0: return 32;
+    case 1: return 128;
+    case 2: return 512;
+    case 3: return 1024;
+    case 4: return 1536;
+    case 5: return 2048;
+    case 6: return 3072;
+    case 7: return 4096;
+    case 8: return 6144;
+    default: return INT_MAX;
+  }
+}
+// the band of class k
+inline int gt_class_band(int k) { return k < 3 ? k : (k < 6 ? 3 : (k < 8 ? 4 : k - 3)); }
+// what the classification counts: systems per class, the packed extent, a
+// negative offset seen, tiles of the open class; then a flag that stays set
+// until read (a CTA gave its systems up)
+enum { GT_EXTENT = GT_NC, GT_BADOFF, GT_TILES, GT_STALLED, GT_COUNTS };
 
 // ---------------------------------------------------------------- Thomas
 // The reference's algorithm (no pivoting): forward sweep with the modified
@@ -329,6 +358,229 @@ __device__ __forceinline__ int bulk_chunk(int n, int NT) {
 // for without end)
 constexpr long GT_WAIT_TRIES = 1L << 22;
 
+// The rows of one chunk, eliminated forward (in place where KEEP): its
+// separator row, its first interior row in terms of both neighbouring
+// separators (yF, vF, wF) and its last one (yL, vL, wL).
+template <class T>
+struct ChunkEnds {
+  T as = 0, bs = 1, cs = 0, ds = 0;
+  T yF = 0, vF = 0, wF = 1, yL = 0, vL = 0, wL = 0;
+};
+
+// row(q, A, B, C, D) gives row q of the tile's rows
+template <bool KEEP, class T, class Row>
+__device__ __forceinline__ ChunkEnds<T> chunk_forward(T* rA, T* rC, T* rD, int q0, int nu, Row row) {
+  ChunkEnds<T> e;
+  T cp = 0, yp = 0, vp = 0;
+  for (int s = 0; s < nu - 1; ++s) {
+    T A, B, C, D;
+    row(q0 + s, A, B, C, D);
+    if (s == 0) {
+      const T m = T(1) / B;
+      cp = C * m;
+      yp = D * m;
+      vp = -A * m;
+    } else {
+      const T m = T(1) / (B - A * cp);
+      yp = (D - A * yp) * m;
+      vp = -A * vp * m;
+      cp = C * m;
+    }
+    if constexpr (KEEP) {
+      rC[q0 + s] = cp;
+      rD[q0 + s] = yp;
+      rA[q0 + s] = vp;
+    }
+    e.yF += e.wF * yp;
+    e.vF += e.wF * vp;
+    e.wF *= -cp;
+  }
+  if (nu > 0) row(q0 + nu - 1, e.as, e.bs, e.cs, e.ds);
+  e.yL = yp;
+  e.vL = vp;
+  e.wL = -cp;
+  return e;
+}
+
+// One level of parallel cyclic reduction on normalised rows (unit diagonal:
+// one reciprocal a level): a, c, d of this lane against the lanes st below
+// and above, where up / dn. A coupling with no partner stays: it is to the
+// unknown beyond the lanes' end.
+template <class T>
+__device__ __forceinline__ void pcr_level(T& a, T& c, T& d, int st, bool up, bool dn) {
+  constexpr unsigned full = 0xffffffffu;
+  T am = __shfl_up_sync(full, a, st), cm = __shfl_up_sync(full, c, st), dm = __shfl_up_sync(full, d, st);
+  T an = __shfl_down_sync(full, a, st), cn = __shfl_down_sync(full, c, st), dn_ = __shfl_down_sync(full, d, st);
+  const T au = up ? a : T(0), cd = dn ? c : T(0);
+  const T r = T(1) / (T(1) - au * cm - cd * an);
+  d = (d - au * dm - cd * dn_) * r;
+  a = (up ? -a * am : a) * r;
+  c = (dn ? -c * cn : c) * r;
+}
+
+// A tile's separators, one per thread of NT: each warp reduces the chunks of
+// its lanes by shuffles, lanes 0..30 to x = d - a XL - c XR (XL, XR the
+// previous and this warp's last separators: a coupling out of the warp stays
+// in its row), then every warp solves the warps' last separators, one lane
+// each, by shuffles again: one barrier, against two per level of a reduction
+// over the CTA in shared memory (16 of them for 256 chunks).
+// blk: NT / 32 rows of 8 values. FULL: the whole tile is solved here; x and xl
+// come back as this chunk's and the previous chunk's separators. Otherwise
+// the tile's last separator is the tile's own unknown and tile[0..6] gets the
+// first unknown's e0 + e1 XL + e2 X and the row A XL + B X + cs x_next = D
+// (written by thread 0).
+template <class T, int NT, bool FULL>
+__device__ __forceinline__ void tile_reduce(const ChunkEnds<T>& e, T (*blk)[8], T& x, T& xl, T* tile) {
+  constexpr unsigned full = 0xffffffffu;
+  constexpr int W = NT / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T nyF = __shfl_down_sync(full, e.yF, 1), nvF = __shfl_down_sync(full, e.vF, 1),
+          nwF = __shfl_down_sync(full, e.wF, 1);
+  const T ra = e.as * e.vL, rb = e.bs + e.as * e.wL, rd = e.ds - e.as * e.yL;
+  T a, c, d;
+  {
+    const T inv = T(1) / (rb + e.cs * nvF);
+    a = ra * inv;
+    c = e.cs * nwF * inv;
+    d = (rd - e.cs * nyF) * inv;
+    // (lane 31 holds the warp's separator, whose row is completed below)
+    if (lane == 31) a = c = d = 0;
+  }
+#pragma unroll
+  for (int st = 1; st < 32; st <<= 1) pcr_level(a, c, d, st, lane >= st, lane + st < 31);
+  {
+    const T a30 = __shfl_up_sync(full, a, 1), c30 = __shfl_up_sync(full, c, 1), d30 = __shfl_up_sync(full, d, 1);
+    if (lane == 0) {
+      blk[warp][0] = e.yF + e.wF * d;
+      blk[warp][1] = e.vF - e.wF * a;
+      blk[warp][2] = -e.wF * c;
+    }
+    if (lane == 31) {
+      blk[warp][3] = -ra * a30;
+      blk[warp][4] = rb - ra * c30;
+      blk[warp][5] = e.cs;
+      blk[warp][6] = rd - ra * d30;
+    }
+  }
+  __syncthreads();
+  // the warps' separators: lane l takes warp l's (not the tile's last one
+  // where that is the tile's unknown)
+  constexpr int V = FULL ? W : W - 1;
+  T A = 0, B = 1, C = 0, D = 0;
+  if (lane < V) {
+    A = blk[lane][3];
+    B = blk[lane][4];
+    C = blk[lane][5];
+    D = blk[lane][6];
+    if (lane + 1 < W) {
+      B += C * blk[lane + 1][1];
+      D -= C * blk[lane + 1][0];
+      C *= blk[lane + 1][2];
+    } else {
+      C = 0;
+    }
+  }
+  {
+    const T inv = T(1) / B;
+    A *= inv;
+    C *= inv;
+    D *= inv;
+  }
+#pragma unroll
+  for (int st = 1; st < V; st <<= 1) pcr_level(A, C, D, st, lane >= st, lane + st < V);
+  if constexpr (FULL) {
+    T XL = __shfl_sync(full, D, warp > 0 ? warp - 1 : 0);
+    if (warp == 0) XL = 0;
+    const T XR = __shfl_sync(full, D, warp);
+    x = lane == 31 ? XR : d - a * XL - c * XR;
+    xl = __shfl_up_sync(full, x, 1);
+    if (lane == 0) xl = XL;
+  } else if (warp == 0) {
+    const T Av = __shfl_sync(full, A, V - 1), Cv = __shfl_sync(full, C, V - 1), Dv = __shfl_sync(full, D, V - 1);
+    if (lane == 0) {
+      tile[0] = blk[0][0] + blk[0][2] * D;
+      tile[1] = blk[0][1] - blk[0][2] * A;
+      tile[2] = -blk[0][2] * C;
+      tile[3] = -blk[V][3] * Av;
+      tile[4] = blk[V][4] - blk[V][3] * Cv;
+      tile[5] = blk[V][5];
+      tile[6] = blk[V][6] - blk[V][3] * Dv;
+    }
+  }
+}
+
+// rows [o, o + n) of the four arrays into a buffer's regions: the bulk copies
+// of the aligned part (thread 0) ...
+template <class T>
+__device__ __forceinline__ void stage_issue(const T* const src[4], T* buf, int region, int o, int n,
+                                            uint64_t* bar) {
+  constexpr int E = 16 / sizeof(T);
+  const int a0 = (o + E - 1) / E * E, a1 = (o + n) / E * E;
+  T* base = buf + bulk_pad<T>(o);
+  if (a1 > a0) {
+    const unsigned bytes = (unsigned)((a1 - a0) * sizeof(T));
+    mbar_arrive_expect(bar, 4 * bytes);
+    for (int a = 0; a < 4; ++a) bulk_g2s(base + (size_t)a * region + (a0 - o), src[a] + a0, bytes, bar);
+  } else {
+    mbar_arrive_expect(bar, 0);
+  }
+}
+
+// ... the bounded wait for them (false: a copy never completed; the copy in
+// flight has then been given one more bounded wait) ...
+__device__ __forceinline__ bool stage_wait(uint64_t* bar, unsigned parity, int* stalled) {
+  bool ok = false;
+  for (long t = 0; t < GT_WAIT_TRIES && !ok; ++t) ok = mbar_try_wait(bar, parity);
+  if (__syncthreads_and(ok)) return true;
+  if (threadIdx.x == 0) {
+    atomicExch(stalled, 1);
+    bool done = false;
+    for (long t = 0; t < GT_WAIT_TRIES && !done; ++t) done = mbar_try_wait(bar, parity);
+  }
+  __syncthreads();
+  return false;
+}
+
+// ... and the rows outside the aligned part by plain loads
+template <class T, int NT>
+__device__ __forceinline__ void stage_ends(const T* const src[4], T* buf, int region, int o, int n) {
+  constexpr int E = 16 / sizeof(T);
+  const int a0 = (o + E - 1) / E * E, a1 = (o + n) / E * E;
+  const int head = min(a0 - o, n), tail0 = max(a1 - o, head);
+  T* base = buf + bulk_pad<T>(o);
+  for (int q = threadIdx.x; q < head + (n - tail0); q += NT) {
+    const int r = q < head ? q : tail0 + (q - head);
+    for (int a = 0; a < 4; ++a) base[(size_t)a * region + r] = src[a][o + r];
+  }
+}
+
+// The partition solve of n staged rows, the solution over rD (threads of the
+// CTA: NT); row() reads a row, the chunks walked in odd lengths.
+template <class T, int NT, class Row>
+__device__ __forceinline__ void cta_solve(T* rA, T* rC, T* rD, int n, T (*blk)[8], Row row) {
+  const int tid = threadIdx.x, S = bulk_chunk(n, NT), P = max(1, n / S);
+  const int q0 = tid * S;
+  const int nu = tid < P ? (tid == P - 1 ? n - q0 : S) : 0;
+  const ChunkEnds<T> e = chunk_forward<true>(rA, rC, rD, q0, nu, row);
+  T x, xl;
+  tile_reduce<T, NT, true>(e, blk, x, xl, nullptr);
+  if (nu > 0) {
+    rD[q0 + nu - 1] = x;
+    T xn = x;
+#pragma unroll 4
+    for (int q = q0 + nu - 2; q >= q0; --q) {
+      const T xq = rD[q] + rA[q] * xl - rC[q] * xn;
+      rD[q] = xq;
+      xn = xq;
+    }
+  }
+}
+
+// Systems of one class, a CTA of NT threads each (about 9 to 17 rows a
+// thread). Bound by the chunks' dependent chains and the rows resident in
+// shared memory. 16384 systems of 16..4096 rows (12 M) on a B200: FP64 434 ->
+// 193 us a batch (2.5 of the 6.6 TB/s at 40 B a row), FP32 280 -> 116 us,
+// against a reduction over the CTA in shared memory on 512 threads.
 template <class T, int NT, int NBUF>
 __global__ void __launch_bounds__(NT) k_gtsv_bulk(const T* __restrict__ dl, const T* __restrict__ d,
                                                   const T* __restrict__ du, const T* __restrict__ b,
@@ -341,23 +593,13 @@ __global__ void __launch_bounds__(NT) k_gtsv_bulk(const T* __restrict__ dl, cons
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);  // NBUF barriers
   auto& sh = *reinterpret_cast<PartCtaShared<T, NT>*>(smem_raw + 128);
   T* bufs = reinterpret_cast<T*>(smem_raw + 128 + (sizeof(PartCtaShared<T, NT>) + 127) / 128 * 128);
-  constexpr int E = 16 / sizeof(T);
   const int tid = threadIdx.x;
   const int cnt = *count;
-  const T* src[4] = {dl, d, du, b};
+  const T* const src[4] = {dl, d, du, b};
   // thread 0: the bulk copies of system list[i] into buffer k
   auto issue = [&](int i, int k) {
     const int sys = list[i];
-    const int o = off[sys], n = len[sys];
-    const int a0 = (o + E - 1) / E * E, a1 = (o + n) / E * E;
-    T* base = bufs + (size_t)k * 4 * region + bulk_pad<T>(o);
-    if (a1 > a0) {
-      const unsigned bytes = (unsigned)((a1 - a0) * sizeof(T));
-      mbar_arrive_expect(&bar[k], 4 * bytes);
-      for (int a = 0; a < 4; ++a) bulk_g2s(base + (size_t)a * region + (a0 - o), src[a] + a0, bytes, &bar[k]);
-    } else {
-      mbar_arrive_expect(&bar[k], 0);
-    }
+    stage_issue(src, bufs + (size_t)k * 4 * region, region, off[sys], len[sys], &bar[k]);
   };
   if (tid == 0) {
     for (int k = 0; k < NBUF; ++k) mbar_init(&bar[k], 1);
@@ -371,136 +613,28 @@ __global__ void __launch_bounds__(NT) k_gtsv_bulk(const T* __restrict__ dl, cons
     const int k = NBUF == 2 ? (it & 1) : 0;
     const int sys = list[i];
     const int o = off[sys], n = len[sys];
-    // wait for the rows (bounded)
-    bool ok = false;
-    for (long t = 0; t < GT_WAIT_TRIES && !ok; ++t) ok = mbar_try_wait(&bar[k], (phase >> k) & 1u);
-    if (!__syncthreads_and(ok)) {
-      // a copy that never completed: record it, give the copy in flight
-      // (the only one: the next system's is issued after this test) one
-      // more bounded wait, and leave the CTA's remaining systems unsolved;
-      // the call reports HYDIST_ERR_TIMEOUT for this batch
-      if (tid == 0) {
-        atomicExch(stalled, 1);
-        bool done = false;
-        for (long t = 0; t < GT_WAIT_TRIES && !done; ++t) done = mbar_try_wait(&bar[k], (phase >> k) & 1u);
-      }
-      __syncthreads();
-      return;
-    }
+    // (the next system's copy is issued after this test; on a stall the CTA's
+    // remaining systems stay unsolved and the call reports HYDIST_ERR_TIMEOUT)
+    if (!stage_wait(&bar[k], (phase >> k) & 1u, stalled)) return;
     phase ^= 1u << k;
     const int inext = i + gridDim.x;
     if (NBUF == 2 && tid == 0 && inext < cnt) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       issue(inext, k ^ 1);
     }
-    T* rA = bufs + (size_t)k * 4 * region + bulk_pad<T>(o);
+    T* buf = bufs + (size_t)k * 4 * region;
+    stage_ends<T, NT>(src, buf, region, o, n);
+    T* rA = buf + bulk_pad<T>(o);
     T* rB = rA + region;
     T* rC = rB + region;
     T* rD = rC + region;
-    // the rows outside the aligned bulk part
-    const int a0 = (o + E - 1) / E * E, a1 = (o + n) / E * E;
-    const int head = min(a0 - o, n), tail0 = max(a1 - o, head);
-    for (int q = tid; q < head + (n - tail0); q += NT) {
-      const int r = q < head ? q : tail0 + (q - head);
-      rA[r] = dl[o + r];
-      rB[r] = d[o + r];
-      rC[r] = du[o + r];
-      rD[r] = b[o + r];
-    }
     __syncthreads();
-    // ---- partition solve in place: forward per chunk, separators by PCR
-    const int S = bulk_chunk(n, NT), P = max(1, n / S);
-    const int q0 = tid * S;
-    const int nu = tid < P ? (tid == P - 1 ? n - q0 : S) : 0;
-    T sep[4] = {0, 1, 0, 0};
-    T cp = 0, yp = 0, vp = 0, Pk = 1, fy = 0, fv = 0;
-    for (int s = 0; s < nu; ++s) {
-      const int q = q0 + s;
-      const T A = q > 0 ? rA[q] : T(0), B = rB[q], C = q + 1 < n ? rC[q] : T(0), Dv = rD[q];
-      if (s == nu - 1) {
-        sep[0] = A;
-        sep[1] = B;
-        sep[2] = C;
-        sep[3] = Dv;
-      } else {
-        if (s == 0) {
-          const T m = T(1) / B;
-          cp = C * m;
-          yp = Dv * m;
-          vp = -A * m;
-        } else {
-          const T m = T(1) / (B - A * cp);
-          yp = (Dv - A * yp) * m;
-          vp = -A * vp * m;
-          cp = C * m;
-        }
-        rC[q] = cp;
-        rD[q] = yp;
-        rA[q] = vp;
-        fy += Pk * yp;
-        fv += Pk * vp;
-        Pk *= -cp;
-      }
-    }
-    sh.tri[0][tid] = fy;
-    sh.tri[1][tid] = fv;
-    sh.tri[2][tid] = Pk;
-    __syncthreads();
-    T ra = 0, rb = 1, rc = 0, rd = 0;
-    if (tid < P) {
-      T yF = 0, vF = 0, wF = 0;
-      if (tid + 1 < P) {
-        yF = sh.tri[0][tid + 1];
-        vF = sh.tri[1][tid + 1];
-        wF = sh.tri[2][tid + 1];
-      }
-      ra = sep[0] * vp;
-      rb = sep[1] - sep[0] * cp + sep[2] * vF;
-      rc = sep[2] * wF;
-      rd = sep[3] - sep[0] * yp - sep[2] * yF;
-    }
-    for (int st = 1; st < P; st <<= 1) {
-      sh.red[0][tid] = ra;
-      sh.red[1][tid] = rb;
-      sh.red[2][tid] = rc;
-      sh.red[3][tid] = rd;
-      __syncthreads();
-      T am = 0, bm = 1, cm = 0, dm = 0, an = 0, bn = 1, cn = 0, dn = 0;
-      if (tid < P && tid - st >= 0) {
-        am = sh.red[0][tid - st];
-        bm = sh.red[1][tid - st];
-        cm = sh.red[2][tid - st];
-        dm = sh.red[3][tid - st];
-      }
-      if (tid + st < P) {
-        an = sh.red[0][tid + st];
-        bn = sh.red[1][tid + st];
-        cn = sh.red[2][tid + st];
-        dn = sh.red[3][tid + st];
-      }
-      __syncthreads();
-      const T k1 = ra / bm, k2 = rc / bn;
-      const T na = -am * k1, nc = -cn * k2;
-      const T nb = rb - cm * k1 - an * k2;
-      const T nd = rd - dm * k1 - dn * k2;
-      ra = na;
-      rb = nb;
-      rc = nc;
-      rd = nd;
-    }
-    sh.xsep[tid] = rd / rb;
-    __syncthreads();
-    if (tid < P) {
-      const T xl = tid > 0 ? sh.xsep[tid - 1] : T(0), xr = sh.xsep[tid];
-      rD[q0 + nu - 1] = xr;
-      T xn = xr;
-      for (int t = nu - 2; t >= 0; --t) {
-        const int q = q0 + t;
-        const T xq = rD[q] + rA[q] * xl - rC[q] * xn;
-        rD[q] = xq;
-        xn = xq;
-      }
-    }
+    cta_solve<T, NT>(rA, rC, rD, n, sh.blk, [&](int q, T& A, T& B, T& C, T& D) {
+      A = q > 0 ? rA[q] : T(0);
+      B = rB[q];
+      C = q + 1 < n ? rC[q] : T(0);
+      D = rD[q];
+    });
     __syncthreads();
     for (int q = tid; q < n; q += NT) x[o + q] = rD[q];
     __syncthreads();  // the buffer is free
@@ -511,18 +645,182 @@ __global__ void __launch_bounds__(NT) k_gtsv_bulk(const T* __restrict__ dl, cons
   }
 }
 
+// ------------------------------------------------------ systems in tiles
+// Systems longer than a CTA's shared memory, cut into tiles of GT_TILE rows
+// (one CTA of GT_TILE_NT threads, 9 rows a thread; the last tile takes the
+// rest, at least two rows). PASS 0 reduces each tile but the last to its last
+// row (tile_reduce) and the last one to its first unknown's e0 + e1 XL; k_gt_
+// tile_solve solves those rows per system; PASS 2 solves each tile with the
+// unknown before it and its last one known. The rows are read twice (72 B
+// per FP64 unknown against 40), by as many CTAs as there are tiles, where one
+// thread per system (Thomas) walked them alone: 512 systems of 4096..16384
+// rows (4.6 M) 22.7 ms -> 0.13 ms, 1.4 TB/s at 40 B a row.
+constexpr int GT_TILE_NT = 256;
+constexpr int GT_TILE = GT_TILE_NT * 9;
+
+__host__ __device__ inline int gt_tiles(int n) {
+  const int t = (n + GT_TILE - 1) / GT_TILE;
+  // a last tile of one row joins the one before it
+  return t > 1 && n - (t - 1) * GT_TILE < 2 ? t - 1 : t;
+}
+
+// items: (system, tile) of every tile, a system's tiles in a row from
+// base[i] on (i its place in the list)
+__global__ void k_gt_tile_items(const int* __restrict__ len, const int* __restrict__ list,
+                                const int* __restrict__ count, int2* __restrict__ items,
+                                int* __restrict__ base, int* __restrict__ next) {
+  const int cnt = *count;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
+    const int s = list[i], nt = gt_tiles(len[s]);
+    const int b = atomicAdd(next, nt);
+    base[i] = b;
+    for (int t = 0; t < nt; ++t) items[b + t] = make_int2(s, t);
+  }
+}
+
+template <class T, int PASS>
+__global__ void __launch_bounds__(GT_TILE_NT) k_gt_tiles_pass(
+    const T* __restrict__ dl, const T* __restrict__ d, const T* __restrict__ du,
+    const T* __restrict__ b, T* __restrict__ x, const int* __restrict__ off,
+    const int* __restrict__ len, const int2* __restrict__ items, T* __restrict__ vals, int region,
+    int* __restrict__ stalled) {
+  constexpr int NT = GT_TILE_NT;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
+  auto& sh = *reinterpret_cast<PartCtaShared<T, NT>*>(smem_raw + 128);
+  T* buf = reinterpret_cast<T*>(smem_raw + 128 + (sizeof(PartCtaShared<T, NT>) + 127) / 128 * 128);
+  const int tid = threadIdx.x;
+  const T* const src[4] = {dl, d, du, b};
+  const int2 item = items[blockIdx.x];
+  const int nsys = len[item.x], r0 = item.y * GT_TILE;
+  const bool last = item.y + 1 == gt_tiles(nsys);
+  const int o = off[item.x] + r0, n = last ? nsys - r0 : GT_TILE;
+  T* v = vals + (size_t)blockIdx.x * 8;
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    stage_issue(src, buf, region, o, n, bar);
+  }
+  __syncthreads();
+  if (!stage_wait(bar, 0, stalled)) return;
+  stage_ends<T, NT>(src, buf, region, o, n);
+  T* rA = buf + bulk_pad<T>(o);
+  T* rB = rA + region;
+  T* rC = rB + region;
+  T* rD = rC + region;
+  __syncthreads();
+  const bool first = item.y == 0;
+  if constexpr (PASS == 0) {
+    auto row = [&](int q, T& A, T& B, T& C, T& D) {
+      A = q > 0 || !first ? rA[q] : T(0);
+      B = rB[q];
+      C = q + 1 < n || !last ? rC[q] : T(0);
+      D = rD[q];
+    };
+    if (!last) {
+      const ChunkEnds<T> e = chunk_forward<false>(rA, rC, rD, tid * 9, 9, row);
+      T x0, x1;
+      tile_reduce<T, NT, false>(e, sh.blk, x0, x1, v);
+    } else {
+      // nothing follows: the first unknown for XL = 0 and for XL = 1 alone
+      // (each a solve of the tile; the rows are kept)
+      const int S = bulk_chunk(n, NT), P = max(1, n / S), q0 = tid * S;
+      const int nu = tid < P ? (tid == P - 1 ? n - q0 : S) : 0;
+      T got[2];
+      for (int g = 0; g < 2; ++g) {
+        const ChunkEnds<T> e = chunk_forward<false>(rA, rC, rD, q0, nu, [&](int q, T& A, T& B, T& C, T& D) {
+          row(q, A, B, C, D);
+          if (g == 1) D = q == 0 ? -A : T(0);
+          if (q == 0) A = 0;
+        });
+        T xs, xl;
+        tile_reduce<T, NT, true>(e, sh.blk, xs, xl, nullptr);
+        got[g] = e.yF + e.vF * xl + e.wF * xs;
+        __syncthreads();
+      }
+      if (tid == 0) {
+        v[0] = got[0];
+        v[1] = got[1];
+        v[2] = 0;
+        v[3] = 0;
+        v[4] = 1;
+        v[5] = 0;
+        v[6] = 0;
+      }
+    }
+  } else {
+    // the last unknowns of the previous tile and of this one
+    const T XL = first ? T(0) : v[-8 + 7], X = v[7];
+    cta_solve<T, NT>(rA, rC, rD, n, sh.blk, [&](int q, T& A, T& B, T& C, T& D) {
+      A = rA[q];
+      B = rB[q];
+      C = q + 1 < n ? rC[q] : T(0);
+      D = rD[q];
+      if (q == 0) {
+        if (!first) D -= A * XL;
+        A = 0;
+      }
+      if (q == n - 1 && !last) {
+        A = C = 0;
+        B = 1;
+        D = X;
+      }
+    });
+    __syncthreads();
+    for (int q = tid; q < n; q += NT) x[o + q] = rD[q];
+  }
+}
+
+// The tiles' last rows of each long system, solved serially by one thread:
+// vals[7] of each tile is its last unknown (the last tile's row is empty).
+template <class T>
+__global__ void k_gt_tile_solve(const int* __restrict__ len, const int* __restrict__ list,
+                                const int* __restrict__ count, const int* __restrict__ base,
+                                T* __restrict__ vals) {
+  const int cnt = *count;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
+    const int nt = gt_tiles(len[list[i]]);
+    T* v = vals + (size_t)base[i] * 8;
+    T cp = 0, yp = 0;
+    for (int t = 0; t < nt; ++t) {
+      T* w = v + (size_t)t * 8;
+      T A = w[3], B = w[4], C = w[5], D = w[6];
+      if (t + 1 < nt) {
+        B += C * w[8 + 1];
+        D -= C * w[8];
+        C *= w[8 + 2];
+      }
+      const T m = T(1) / (B - A * cp);
+      yp = (D - A * yp) * m;
+      cp = C * m;
+      w[3] = cp;  // (the row is consumed)
+      w[7] = yp;
+    }
+    T xn = yp;
+    for (int t = nt - 2; t >= 0; --t) {
+      T* w = v + (size_t)t * 8;
+      xn = w[7] - w[3] * xn;
+      w[7] = xn;
+    }
+  }
+}
+
 template <class T>
 __global__ void __launch_bounds__(GT_WARPS * 32) k_gtsv_warp(
     const T* __restrict__ dl, const T* __restrict__ d, const T* __restrict__ du,
     const T* __restrict__ b, T* __restrict__ x, const int* __restrict__ off,
-    const int* __restrict__ len, const int* __restrict__ list, const int* __restrict__ count,
-    int slice) {
+    const int* __restrict__ len, const int* __restrict__ lists, size_t ld,
+    const int* __restrict__ counts, int k0, int k1, int slice) {
+  // the systems of classes k0..k1 (lists of ld entries each), longest first
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   T* base = reinterpret_cast<T*>(smem_raw) + (size_t)warp * 4 * slice;
-  const int cnt = *count;
+  int cnt = 0;
+  for (int k = k0; k <= k1; ++k) cnt += counts[k];
   for (int i = blockIdx.x * GT_WARPS + warp; i < cnt; i += gridDim.x * GT_WARPS) {
-    const int s = list[i];
+    int k = k1, at = i;
+    while (k > k0 && at >= counts[k]) at -= counts[k--];
+    const int s = lists[(size_t)k * ld + at];
     const int o = off[s], n = len[s];
     const PartGeom g = part_geom(n, 32);
     T* rA = base;
@@ -537,25 +835,60 @@ __global__ void __launch_bounds__(GT_WARPS * 32) k_gtsv_warp(
   }
 }
 
-// Files system s under its length band (empty systems under none). Also
-// counts[GT_NB] = the packed extent max(off + len), counts[GT_NB + 1] = 1 if
-// a system has a negative offset (the batch is then refused).
+// Files the systems under their length classes (empty systems under none) and
+// counts (see GT_EXTENT...). The last block to finish writes the counts to
+// mapped host memory and sets them back to zero for the next call, so that a
+// batch is classified by one launch without a memset and a copy around it.
 __global__ void k_gt_classify(const int* __restrict__ off, const int* __restrict__ len, int nsys,
-                              int* __restrict__ lists, int* __restrict__ counts) {
+                              int* __restrict__ lists, size_t ld, int* __restrict__ work,
+                              int* __restrict__ counts, volatile int* __restrict__ host) {
+  __shared__ bool last_block;
+  __shared__ int sh_n[GT_NC], sh_at[GT_NC], sh_ext, sh_bad, sh_tiles;
+  for (int k = threadIdx.x; k < GT_NC; k += blockDim.x) sh_n[k] = 0;
+  if (threadIdx.x == 0) sh_ext = sh_bad = sh_tiles = 0;
+  __syncthreads();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
-  const int n = len[s];
-  if (n <= 0) return;
-  const int o = off[s];
-  if (o < 0 || o > INT_MAX - n) {
-    counts[GT_NB + 1] = 1;
-    return;
+  int k = -1, idx = 0;
+  if (s < nsys) {
+    const int n = len[s];
+    if (n > 0) {
+      const int o = off[s];
+      if (o < 0 || o > INT_MAX - n) {
+        sh_bad = 1;
+      } else {
+        atomicMax(&sh_ext, o + n);
+        k = 0;
+        while (k < GT_NC - 1 && n > gt_class_hi(k)) ++k;
+        idx = atomicAdd(&sh_n[k], 1);
+        if (k == GT_NC - 1) atomicAdd(&sh_tiles, gt_tiles(n));
+      }
+    }
   }
-  atomicMax(&counts[GT_NB], o + n);
-  int b = 0;
-  while (b < GT_NB - 1 && n > gt_band_hi(b)) ++b;
-  const int idx = atomicAdd(&counts[b], 1);
-  lists[(size_t)b * nsys + idx] = s;
+  __syncthreads();
+  // one global atomic per block and class
+  if (threadIdx.x < GT_NC && sh_n[threadIdx.x] > 0)
+    sh_at[threadIdx.x] = atomicAdd(&work[threadIdx.x], sh_n[threadIdx.x]);
+  if (threadIdx.x == 0) {
+    if (sh_ext) atomicMax(&work[GT_EXTENT], sh_ext);
+    if (sh_bad) atomicExch(&work[GT_BADOFF], 1);
+    if (sh_tiles) atomicAdd(&work[GT_TILES], sh_tiles);
+  }
+  __syncthreads();
+  if (k >= 0) lists[(size_t)k * ld + sh_at[k] + idx] = s;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last_block = atomicAdd(&work[GT_COUNTS], 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last_block) return;
+  __threadfence();
+  if (threadIdx.x < GT_STALLED) {
+    const int v = atomicExch(&work[threadIdx.x], 0);
+    counts[threadIdx.x] = v;
+    host[threadIdx.x] = v;
+    __threadfence_system();
+  }
+  if (threadIdx.x == 0) work[GT_COUNTS] = 0;
 }
 
 // diagonally dominant synthetic systems for the autotuner (a counter hash)
@@ -595,9 +928,13 @@ struct DevScratch {
   size_t flags_bytes = 0;
   float* f32 = nullptr;  // refinement: FP32 copies of the systems and x (rows x 5 x 4 B)
   size_t f32_bytes = 0;
-  int* lists = nullptr;  // GT_NB x nsys
+  int* lists = nullptr;  // GT_NC x nsys
   size_t lists_cap = 0;  // systems
-  int* counts = nullptr;  // GT_NB
+  int* counts = nullptr;  // the classification's counts and its working copy
+  int* host = nullptr;    // the counts and the stall flag in mapped host memory
+  int* host_dev = nullptr;
+  void* tiles = nullptr;  // tiles of long systems: vals, items, bases
+  size_t tiles_bytes = 0;
 };
 
 struct DevInfo {
@@ -607,9 +944,12 @@ struct DevInfo {
   DevScratch scr;
   // the bands of a batch run side by side: one stream per band, forked from
   // the caller's stream and joined back (created on first use, kept)
-  cudaStream_t band_st[GT_NB] = {};
-  cudaEvent_t fork = nullptr, join[GT_NB] = {};
+  cudaStream_t band_st[hyd::GT_NC] = {};
+  cudaEvent_t fork = nullptr, join[hyd::GT_NC] = {};
   bool streams = false;
+  // the end of the last batch: the next one, on whatever stream, waits for it
+  // before it uses the scratch again
+  cudaEvent_t done = nullptr;
 };
 
 std::mutex g_mu;
@@ -651,6 +991,10 @@ int cta_max_rows(const DevInfo& D) {
   return lo;
 }
 
+// the tile solver of the open band (not a public algo: what the shared-memory
+// solvers become for systems that fit no CTA)
+constexpr int GTSV_TILES = 100;
+
 struct Caps {
   int cta128, cta256, cta512;  // longest systems of the three CTA tiles
 };
@@ -670,11 +1014,14 @@ bool feasible(int algo, int band, const Caps& c) {
   return false;
 }
 
-// solver of a band when nothing was tuned: warp for short systems, the
-// 512-thread tile for long ones that fit, the 256-thread tile beyond,
-// Thomas for what fits no shared memory
+// solver of a band when nothing was tuned: warp for short systems, then the
+// CTA solver on as many threads as leave each 9 to 17 rows (128 up to 2048
+// rows, 256 up to 4096, 512 beyond), Thomas for what fits no shared memory
 int default_algo(int band, const Caps& c) {
   if (feasible(HYDIST_GTSV_WARP, band, c)) return HYDIST_GTSV_WARP;
+  const int hi = hyd::gt_band_hi(band);
+  if (hi <= 2048 && feasible(HYDIST_GTSV_PARTITION_128, band, c)) return HYDIST_GTSV_PARTITION_128;
+  if (hi <= 4096 && feasible(HYDIST_GTSV_PARTITION, band, c)) return HYDIST_GTSV_PARTITION;
   if (feasible(HYDIST_GTSV_PARTITION_512, band, c)) return HYDIST_GTSV_PARTITION_512;
   if (feasible(HYDIST_GTSV_PARTITION, band, c)) return HYDIST_GTSV_PARTITION;
   return HYDIST_GTSV_THOMAS;
@@ -735,12 +1082,63 @@ int launch_cta(int nmax, const T* dl, const T* d, const T* du, const T* b, T* x,
   return launch_bulk<T, NT, 1>(nmax, dl, d, du, b, x, off, len, list, count, stalled, nsys_band, D, st);
 }
 
+// the systems of more rows than a CTA's shared memory holds, in tiles
 template <class T>
-int launch_band(int algo, int band, const T* dl, const T* d, const T* du, const T* b, T* x, T* w,
-                unsigned char* flags, const int* off, const int* len, const int* list,
-                const int* count, int* stalled, int nsys_band, const DevInfo& D, cudaStream_t st) {
+int launch_tiles(const T* dl, const T* d, const T* du, const T* b, T* x, const int* off,
+                 const int* len, const int* list, const int* count, int nsys, int tiles,
+                 int* stalled, DevInfo& D, cudaStream_t st) {
+  using hyd::GT_TILE;
+  // a last tile of one row is solved with the one before it
+  const int region = hyd::bulk_region<T>(GT_TILE + 1);
+  const size_t smem = cta_smem<T, hyd::GT_TILE_NT>(GT_TILE + 1);
+  if (resident_ctas(hyd::k_gt_tiles_pass<T, 0>, hyd::GT_TILE_NT, smem, D.optin) < 1 ||
+      resident_ctas(hyd::k_gt_tiles_pass<T, 2>, hyd::GT_TILE_NT, smem, D.optin) < 1)
+    return HYDIST_ERR_CUDA;
+  DevScratch& s = D.scr;
+  const size_t need = (size_t)tiles * (8 * sizeof(double) + sizeof(int2)) + (size_t)(nsys + 1) * sizeof(int);
+  if (s.tiles_bytes < need) {
+    if (s.tiles) cudaFree(s.tiles);
+    s.tiles = nullptr;
+    s.tiles_bytes = 0;
+    if (cudaMalloc(&s.tiles, need + 256) != cudaSuccess) return HYDIST_ERR_OOM;
+    s.tiles_bytes = need;
+  }
+  T* vals = (T*)s.tiles;
+  int2* items = (int2*)((char*)s.tiles + (size_t)tiles * 8 * sizeof(double));
+  int* next = (int*)(items + tiles);
+  int* base = next + 1;
+  if (cudaMemsetAsync(next, 0, sizeof(int), st) != cudaSuccess) return HYDIST_ERR_CUDA;
+  const int g = std::min((nsys + 127) / 128, 8 * D.nsm);
+  hyd::k_gt_tile_items<<<g, 128, 0, st>>>(len, list, count, items, base, next);
+  hyd::k_gt_tiles_pass<T, 0><<<tiles, hyd::GT_TILE_NT, smem, st>>>(dl, d, du, b, x, off, len, items, vals,
+                                                                  region, stalled);
+  hyd::k_gt_tile_solve<T><<<g, 128, 0, st>>>(len, list, count, base, vals);
+  hyd::k_gt_tiles_pass<T, 2><<<tiles, hyd::GT_TILE_NT, smem, st>>>(dl, d, du, b, x, off, len, items, vals,
+                                                                  region, stalled);
+  return HYDIST_OK;
+}
+
+// the warp solver over classes k0..k1
+template <class T>
+int launch_warp(int k0, int k1, const T* dl, const T* d, const T* du, const T* b, T* x,
+                const int* off, const int* len, int nsys, const DevInfo& D, cudaStream_t st) {
+  const int nmax = std::min(hyd::gt_class_hi(k1), hyd::GT_WARP_MAX);
+  const int slice = hyd::part_stride_bound(nmax, 32);
+  const size_t smem = warp_smem<T>(nmax);
+  const int per_sm = resident_ctas(hyd::k_gtsv_warp<T>, hyd::GT_WARPS * 32, smem, D.optin);
+  if (per_sm < 1) return HYDIST_ERR_CUDA;
+  const int grid = std::min((nsys + hyd::GT_WARPS - 1) / hyd::GT_WARPS, per_sm * D.nsm);
+  hyd::k_gtsv_warp<T><<<grid, hyd::GT_WARPS * 32, smem, st>>>(dl, d, du, b, x, off, len, D.scr.lists,
+                                                              D.scr.lists_cap, D.scr.counts, k0, k1, slice);
+  return HYDIST_OK;
+}
+
+template <class T>
+int launch_class(int algo, int cls, const T* dl, const T* d, const T* du, const T* b, T* x, T* w,
+                 unsigned char* flags, const int* off, const int* len, const int* list,
+                 const int* count, int* stalled, int nsys_band, DevInfo& D, cudaStream_t st) {
   if (nsys_band <= 0) return HYDIST_OK;
-  const int hi = hyd::gt_band_hi(band);
+  const int hi = hyd::gt_class_hi(cls);
   int rc = HYDIST_OK;
   if (algo == HYDIST_GTSV_PIVOT) {
     const int bs = 128;
@@ -753,14 +1151,10 @@ int launch_band(int algo, int band, const T* dl, const T* d, const T* du, const 
   } else if (algo == HYDIST_GTSV_PARTITION_512) {
     rc = launch_cta<T, 512>(hi, dl, d, du, b, x, off, len, list, count, stalled, nsys_band, D, st);
   } else if (algo == HYDIST_GTSV_WARP) {
-    const int nmax = std::min(hi, hyd::GT_WARP_MAX);
-    const int slice = hyd::part_stride_bound(nmax, 32);
-    const size_t smem = warp_smem<T>(nmax);
-    const int per_sm = resident_ctas(hyd::k_gtsv_warp<T>, hyd::GT_WARPS * 32, smem, D.optin);
-    if (per_sm < 1) return HYDIST_ERR_CUDA;
-    const int grid = std::min((nsys_band + hyd::GT_WARPS - 1) / hyd::GT_WARPS, per_sm * D.nsm);
-    hyd::k_gtsv_warp<T><<<grid, hyd::GT_WARPS * 32, smem, st>>>(dl, d, du, b, x, off, len, list,
-                                                                  count, slice);
+    rc = launch_warp<T>(cls, cls, dl, d, du, b, x, off, len, nsys_band, D, st);
+  } else if (algo == GTSV_TILES) {
+    rc = launch_tiles<T>(dl, d, du, b, x, off, len, list, count, nsys_band, D.scr.host[hyd::GT_TILES],
+                         stalled, D, st);
   } else {
     const int bs = 128;
     const int grid = std::min((nsys_band + bs - 1) / bs, 8 * D.nsm);
@@ -789,23 +1183,35 @@ int ensure_scratch(DevScratch& s, size_t w_bytes, size_t nsys, size_t flag_bytes
     if (s.lists) cudaFree(s.lists);
     s.lists = nullptr;
     s.lists_cap = 0;
-    if (cudaMalloc(&s.lists, (size_t)GT_NB * nsys * sizeof(int)) != cudaSuccess) return HYDIST_ERR_OOM;
+    if (cudaMalloc(&s.lists, (size_t)hyd::GT_NC * nsys * sizeof(int)) != cudaSuccess) return HYDIST_ERR_OOM;
     s.lists_cap = nsys;
   }
-  // band sizes, packed extent, offset check, and a flag that stays set
-  // until read: a CTA solver gave a system up (its staging never completed)
   if (!s.counts) {
-    if (cudaMalloc(&s.counts, (GT_NB + 3) * sizeof(int)) != cudaSuccess) return HYDIST_ERR_OOM;
-    if (cudaMemset(s.counts, 0, (GT_NB + 3) * sizeof(int)) != cudaSuccess) return HYDIST_ERR_CUDA;
+    const size_t bytes = 2 * (hyd::GT_COUNTS + 1) * sizeof(int);
+    if (cudaMalloc(&s.counts, bytes) != cudaSuccess) return HYDIST_ERR_OOM;
+    if (cudaMemset(s.counts, 0, bytes) != cudaSuccess) return HYDIST_ERR_CUDA;
+    if (cudaHostAlloc((void**)&s.host, (hyd::GT_COUNTS + 1) * sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&s.host_dev, s.host, 0) != cudaSuccess)
+      return HYDIST_ERR_CUDA;
+    s.host[hyd::GT_STALLED] = 0;
   }
   return HYDIST_OK;
+}
+
+// files a batch's systems on stream st and waits for the counts (s.host)
+int classify(DevScratch& s, const int* off, const int* len, int nsys, cudaStream_t st) {
+  hyd::k_gt_classify<<<(nsys + 255) / 256, 256, 0, st>>>(off, len, nsys, s.lists, s.lists_cap,
+                                                         s.counts + hyd::GT_COUNTS + 1, s.counts,
+                                                         s.host_dev);
+  if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return HYDIST_ERR_CUDA;
+  return s.host[hyd::GT_BADOFF] ? HYDIST_ERR_ARG : HYDIST_OK;
 }
 
 // the per-band streams and events of a device (false if they cannot be made:
 // the bands then run one after another on the caller's stream)
 bool band_streams(DevInfo& D) {
   if (D.streams) return true;
-  for (int k = 0; k < GT_NB; ++k) {
+  for (int k = 0; k < hyd::GT_NC; ++k) {
     if (!D.band_st[k] && cudaStreamCreateWithFlags(&D.band_st[k], cudaStreamNonBlocking) != cudaSuccess)
       return false;
     if (!D.join[k] && cudaEventCreateWithFlags(&D.join[k], cudaEventDisableTiming) != cudaSuccess)
@@ -816,78 +1222,91 @@ bool band_streams(DevInfo& D) {
   return true;
 }
 
+bool staged_algo(int a) {
+  return a == HYDIST_GTSV_PARTITION || a == HYDIST_GTSV_PARTITION_512 || a == HYDIST_GTSV_PARTITION_128 ||
+         a == GTSV_TILES;
+}
+
 // one batched solve with a given solver per band (table[b])
 template <class T>
 int solve_batch(const T* dl, const T* d, const T* du, const T* b, T* x, const int* off,
                 const int* len, int nsys, const int table[GT_NB], DevInfo& D, cudaStream_t st) {
+  using hyd::GT_NC;
   int rc = ensure_scratch(D.scr, 0, (size_t)nsys);
   if (rc != HYDIST_OK) return rc;
-  if (cudaMemsetAsync(D.scr.counts, 0, (GT_NB + 2) * sizeof(int), st) != cudaSuccess)
+  if (!D.done && cudaEventCreateWithFlags(&D.done, cudaEventDisableTiming) != cudaSuccess)
     return HYDIST_ERR_CUDA;
-  hyd::k_gt_classify<<<(nsys + 255) / 256, 256, 0, st>>>(off, len, nsys, D.scr.lists, D.scr.counts);
-  // band sizes, packed extent and the offset check in one synchronisation
-  int counts[GT_NB + 3];
-  if (cudaMemcpyAsync(counts, D.scr.counts, sizeof(counts), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return HYDIST_ERR_CUDA;
-  if (counts[GT_NB + 1]) return HYDIST_ERR_ARG;
+  // an earlier batch may still run on another stream
+  if (cudaStreamWaitEvent(st, D.done, 0) != cudaSuccess) return HYDIST_ERR_CUDA;
+  rc = classify(D.scr, off, len, nsys, st);
+  if (rc != HYDIST_OK) return rc;
+  const int* counts = D.scr.host;
   // the CTA solvers stage rows with bulk copies, which need 16-byte aligned
   // arrays; misaligned ones go to Thomas
-  int tab[GT_NB];
+  int tab[GT_NC];
   const bool aligned =
       (((uintptr_t)dl | (uintptr_t)d | (uintptr_t)du | (uintptr_t)b) & 15) == 0;
-  for (int bnd = 0; bnd < GT_NB; ++bnd)
-    tab[bnd] = (!aligned && (table[bnd] == HYDIST_GTSV_PARTITION ||
-                             table[bnd] == HYDIST_GTSV_PARTITION_512 ||
-                             table[bnd] == HYDIST_GTSV_PARTITION_128))
-                   ? HYDIST_GTSV_THOMAS
-                   : table[bnd];
-  table = tab;
-  bool thomas = false, pivot = false;
-  for (int bnd = 0; bnd < GT_NB; ++bnd) {
-    thomas |= counts[bnd] > 0 && table[bnd] == HYDIST_GTSV_THOMAS;
-    pivot |= counts[bnd] > 0 && table[bnd] == HYDIST_GTSV_PIVOT;
+  bool thomas = false, pivot = false, staged = false;
+  int nonempty = 0, top_warp = -1, short_sys = 0;
+  for (int k = 0; k < GT_NC; ++k) {
+    const int a = table[hyd::gt_class_band(k)];
+    tab[k] = !aligned && staged_algo(a) ? HYDIST_GTSV_THOMAS : a;
+    if (counts[k] == 0) continue;
+    ++nonempty;
+    thomas |= tab[k] == HYDIST_GTSV_THOMAS;
+    pivot |= tab[k] == HYDIST_GTSV_PIVOT;
+    staged |= staged_algo(tab[k]);
+    if (tab[k] == HYDIST_GTSV_WARP) {
+      top_warp = k;
+      short_sys += counts[k];
+    }
   }
   if (thomas || pivot) {
-    rc = ensure_scratch(D.scr, (size_t)counts[GT_NB] * sizeof(T), (size_t)nsys,
-                        pivot ? (size_t)counts[GT_NB] : 0);
+    rc = ensure_scratch(D.scr, (size_t)counts[hyd::GT_EXTENT] * sizeof(T), (size_t)nsys,
+                        pivot ? (size_t)counts[hyd::GT_EXTENT] : 0);
     if (rc != HYDIST_OK) return rc;
   }
-  bool staged = false;  // a bulk-staged CTA solver ran
-  // the bands' solves are independent (disjoint systems, per-band lists,
-  // per-system scratch): each non-empty band on its own stream, so that the
-  // short bands' launches and the long bands' tails overlap
-  int nonempty = 0;
-  for (int bnd = 0; bnd < GT_NB; ++bnd) nonempty += counts[bnd] > 0;
+  // the warp solver's classes as one launch where one wave of warps takes
+  // them all: each launch costs a small batch more than the shared memory
+  // that its shorter systems leave unused (64 systems of 16..256 rows, with the
+  // classification in one launch: 39 -> 25 us a call)
+  bool merge = top_warp > 0 && short_sys <= 4 * D.nsm;
+  for (int k = 0; k < top_warp; ++k) merge = merge && (counts[k] == 0 || tab[k] == HYDIST_GTSV_WARP);
+  if (merge)
+    for (int k = 0; k < top_warp; ++k) nonempty -= counts[k] > 0 && tab[k] == HYDIST_GTSV_WARP;
+  // the classes' solves are independent (disjoint systems, per-class lists,
+  // per-system scratch): each on its own stream, so that the short classes'
+  // launches and the long classes' tails overlap; the longest first
   const bool side = nonempty > 1 && band_streams(D);
   if (side && cudaEventRecord(D.fork, st) != cudaSuccess) return HYDIST_ERR_CUDA;
-  for (int bnd = 0; bnd < GT_NB; ++bnd) {
-    if (counts[bnd] == 0) continue;
+  for (int k = GT_NC - 1; k >= 0; --k) {
+    if (counts[k] == 0) continue;
+    const bool warps = merge && tab[k] == HYDIST_GTSV_WARP;
+    if (warps && k != top_warp) continue;
     cudaStream_t bs = st;
     if (side) {
-      bs = D.band_st[bnd];
+      bs = D.band_st[k];
       if (cudaStreamWaitEvent(bs, D.fork, 0) != cudaSuccess) return HYDIST_ERR_CUDA;
     }
-    rc = launch_band<T>(table[bnd], bnd, dl, d, du, b, x, (T*)D.scr.w, D.scr.flags, off, len,
-                        D.scr.lists + (size_t)bnd * nsys, D.scr.counts + bnd,
-                        D.scr.counts + GT_NB + 2, counts[bnd], D, bs);
-    if (side && (cudaEventRecord(D.join[bnd], bs) != cudaSuccess ||
-                 cudaStreamWaitEvent(st, D.join[bnd], 0) != cudaSuccess))
+    if (warps)
+      rc = launch_warp<T>(0, top_warp, dl, d, du, b, x, off, len, short_sys, D, bs);
+    else
+      rc = launch_class<T>(tab[k], k, dl, d, du, b, x, (T*)D.scr.w, D.scr.flags, off, len,
+                           D.scr.lists + (size_t)k * D.scr.lists_cap, D.scr.counts + k,
+                           D.scr.host_dev + hyd::GT_STALLED, counts[k], D, bs);
+    if (side && (cudaEventRecord(D.join[k], bs) != cudaSuccess ||
+                 cudaStreamWaitEvent(st, D.join[k], 0) != cudaSuccess))
       return HYDIST_ERR_CUDA;
     if (rc != HYDIST_OK) return rc;
-    staged |= table[bnd] == HYDIST_GTSV_PARTITION || table[bnd] == HYDIST_GTSV_PARTITION_512 ||
-              table[bnd] == HYDIST_GTSV_PARTITION_128;
   }
+  if (cudaEventRecord(D.done, st) != cudaSuccess) return HYDIST_ERR_CUDA;
   if (staged) {
     // a CTA whose staging copy never completed left systems unsolved: read
     // its flag now, so that this batch, not a later one, reports it
-    int flag = 0;
-    if (cudaMemcpyAsync(&flag, D.scr.counts + GT_NB + 2, sizeof(int), cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      return HYDIST_ERR_CUDA;
-    if (flag) {
-      cudaMemsetAsync(D.scr.counts + GT_NB + 2, 0, sizeof(int), st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) return HYDIST_ERR_CUDA;
+    volatile int* flag = D.scr.host + hyd::GT_STALLED;
+    if (*flag) {
+      *flag = 0;
       return HYDIST_ERR_TIMEOUT;
     }
   }
@@ -1032,6 +1451,8 @@ extern "C" int hydist_gtsv_batched(const void* dl, const void* d, const void* du
     if (a == HYDIST_GTSV_WARP && !feasible(a, bnd, caps)) a = HYDIST_GTSV_PARTITION_512;
     if (a == HYDIST_GTSV_PARTITION_512 && !feasible(a, bnd, caps)) a = HYDIST_GTSV_PARTITION;
     if (a == HYDIST_GTSV_PARTITION && !feasible(a, bnd, caps)) a = HYDIST_GTSV_THOMAS;
+    // what fits no CTA: in tiles, unless Thomas (or pivoting) was asked for
+    if (bnd == GT_NB - 1 && a == HYDIST_GTSV_THOMAS && algo != HYDIST_GTSV_THOMAS) a = GTSV_TILES;
     table[bnd] = a;
   }
   int rc;
@@ -1075,20 +1496,12 @@ extern "C" int hydist_gtsv_batched_refine(const double* dl, const double* d, con
     if (!D) return HYDIST_ERR_ARG;
     int rc = ensure_scratch(D->scr, 0, (size_t)nsys);
     if (rc != HYDIST_OK) return rc;
-    if (cudaMemsetAsync(D->scr.counts, 0, (GT_NB + 2) * sizeof(int), st) != cudaSuccess)
-      return HYDIST_ERR_CUDA;
-    hyd::k_gt_classify<<<(nsys + 255) / 256, 256, 0, st>>>(offsets, lengths, nsys, D->scr.lists,
-                                                           D->scr.counts);
-    int counts[GT_NB + 2];
-    if (cudaMemcpyAsync(counts, D->scr.counts, sizeof(counts), cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      return HYDIST_ERR_CUDA;
-    if (counts[GT_NB + 1]) {
+    if (D->done && cudaStreamWaitEvent(st, D->done, 0) != cudaSuccess) return HYDIST_ERR_CUDA;
+    rc = classify(D->scr, offsets, lengths, nsys, st);
+    if (rc == HYDIST_ERR_ARG)
       hyd::set_last_error("hydist_gtsv_batched_refine: a system has a negative offset");
-      return HYDIST_ERR_ARG;
-    }
-    rows = (size_t)counts[GT_NB];
+    if (rc != HYDIST_OK) return rc;
+    rows = (size_t)D->scr.host[hyd::GT_EXTENT];
     // each FP32 array starts 16-byte aligned (the CTA solvers stage rows
     // with bulk copies)
     const size_t need = (rows + 3) / 4 * 4 * 5 * sizeof(float);
@@ -1118,7 +1531,12 @@ extern "C" int hydist_gtsv_batched_refine(const double* dl, const double* d, con
   rc = hydist_gtsv_batched(fl, fd, fu, fb, fx, offsets, lengths, nsys, 1, algo, stream);
   if (rc != HYDIST_OK) return rc;
   hyd::k_gt_correct<<<nsys, 128, 0, st>>>(x, fx, offsets, lengths, nsys);
-  if (cudaGetLastError() != cudaSuccess) {
+  cudaError_t err = cudaGetLastError();
+  if (err == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    err = cudaEventRecord(dev_info(dev)->done, st);
+  }
+  if (err != cudaSuccess) {
     hyd::set_last_error("hydist_gtsv_batched_refine: a kernel launch failed");
     return HYDIST_ERR_CUDA;
   }

@@ -365,8 +365,8 @@ int hydist_kernel_launches(HydistHandle* h, int64_t* count);
  * dtype: 0 = FP64, 1 = FP32. algo (enum HydistGtsvAlgo):
  *   AUTO       per length band, the solver hydist_gtsv_autotune chose on
  *              this device (before any tuning: WARP up to 512 rows, then
- *              PARTITION_512 or PARTITION where the system fits a CTA's
- *              shared memory, THOMAS beyond);
+ *              PARTITION_128 up to 2048, PARTITION up to 4096 and
+ *              PARTITION_512 up to 6144), tiles beyond;
  *   THOMAS     one thread per system, in place in global memory;
  *   PARTITION  one 256-thread CTA per system staged in shared memory:
  *              chunked Thomas with the chunk separators' reduced system
@@ -377,7 +377,11 @@ int hydist_kernel_launches(HydistHandle* h, int64_t* count);
  *   PARTITION_512  PARTITION with 512-thread tiles (more warps per system,
  *              less shared memory left for long systems).
  * A solver that cannot take a band's lengths passes it on (WARP ->
- * PARTITION_512 -> PARTITION -> THOMAS; PARTITION_128 -> PARTITION).
+ * PARTITION_512 -> PARTITION -> THOMAS; PARTITION_128 -> PARTITION). The open
+ * band, whose only solver of the table is THOMAS, is solved in tiles of one
+ * CTA each (the partition method over the tiles) unless THOMAS or PIVOT is
+ * asked for. Arrays that are not 16-byte aligned go to THOMAS where a CTA
+ * solver was chosen.
  * PARTITION_128, PARTITION and PARTITION_512 are the same CTA partition
  * solver on 128, 256 or 512 threads per system: fewer threads give each
  * thread a longer chunk and the separators a shorter reduction. Systems of length 0 are skipped.
