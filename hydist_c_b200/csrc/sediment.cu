@@ -171,12 +171,9 @@ __device__ __forceinline__ void fs_rows_cells(StateT<R> S_arg, CoefT<R> c_arg, B
   const int j = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int i = blockIdx.y + 2;
   if (i > S.N || j > S.M) return;
-  const int W = S.W, g = i * W + j, gp = DIR == 0 ? g - W : g - 1;
-  const R* vel = DIR == 0 ? S.tu : S.tv;
-  const R hk_c = DIR == 0 ? S.Htdu[g] * S.Kx[g] : S.Htdv[g] * S.Ky[g];
-  const R hk_p = DIR == 0 ? S.Htdu[gp] * S.Kx[gp] : S.Htdv[gp] * S.Ky[gp];
+  const int W = S.W, g = i * W + j;
   R A, B, C, D;
-  fs_cell(S, c, DIR == 0, i, j, vel[g], hk_c, vel[gp], hk_p, S.clock[0], S.src_start, A, B, C, D);
+  fs_row<DIR>(S, c, i, j, A, B, C, D);
   const size_t n = (size_t)W * S.H;
   R* q = S.pre + g;
   q[0] = A;
@@ -242,7 +239,8 @@ void launch_sediment(const StateT<R>& S, const CoefT<R>& c, bool xdir, bool bed,
   // Find_VTH + hesoK ran in the half-step's commit (k_commit_a/k_commit_b)
   if (tr) tr->kbegin(st, xdir ? KS_FS_X : KS_FS_Y);
   const unsigned z = grid_z(b);
-  {
+  const bool rows = !fs_rows_in_sweep(S, xdir ? 0 : 1);
+  if (rows) {
     const dim3 gr(cdiv(S.M - 1, 128), S.N - 1, z);
     if (b.n > 0) {
       if (xdir) k_fs_rows_b<R, 0><<<gr, 128, 0, st>>>(S, c, b);
@@ -252,7 +250,7 @@ void launch_sediment(const StateT<R>& S, const CoefT<R>& c, bool xdir, bool bed,
       else k_fs_rows<R, 1, 0><<<gr, 128, 0, st>>>(S, c, b);
     }
   }
-  const int nfs = 1 + launch_fs_sweep(S, c, xdir ? 0 : 1, st, b);
+  const int nfs = (rows ? 1 : 0) + launch_fs_sweep(S, c, xdir ? 0 : 1, st, b);
   if (tr) tr->kend(st, xdir ? KS_FS_X : KS_FS_Y);
   const dim3 gfs(cdiv(S.M, 128), cdiv(S.N, FS_ROWS), z);
   if (b.n > 0) k_update_fs<R, 1><<<gfs, 128, 0, st>>>(S, c, b);

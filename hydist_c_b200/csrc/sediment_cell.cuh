@@ -157,4 +157,16 @@ __device__ __forceinline__ void fs_cell(const StateT<R>& S, const CoefT<R>& c, b
   D = fs * c.HaiChiadT - q + p + Sx * rH;
 }
 
+// The row of cell (i, j), without its segment's end conditions. DIR 0: the
+// i-sweep (the cell before is (i-1, j)), 1: the j-sweep.
+template <int DIR, class R>
+__device__ __forceinline__ void fs_row(const StateT<R>& S, const CoefT<R>& c, int i, int j, R& A,
+                                       R& B, R& C, R& D) {
+  const int W = S.W, g = i * W + j, gp = DIR == 0 ? g - W : g - 1;
+  const R* vel = DIR == 0 ? S.tu : S.tv;
+  const R hk_c = DIR == 0 ? S.Htdu[g] * S.Kx[g] : S.Htdv[g] * S.Ky[g];
+  const R hk_p = DIR == 0 ? S.Htdu[gp] * S.Kx[gp] : S.Htdv[gp] * S.Ky[gp];
+  fs_cell(S, c, DIR == 0, i, j, vel[g], hk_c, vel[gp], hk_p, S.clock[0], S.src_start, A, B, C, D);
+}
+
 }  // namespace hyd

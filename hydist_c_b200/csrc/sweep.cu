@@ -9,11 +9,13 @@
 // (UVZSolver_multithread.cpp:472-603) directly from the solution, each cell's
 // level by its continuity row. FP64 on 2048x1024, against the interleaved
 // system: XXX
+#include <algorithm>
+
 #include "assembly.cuh"
 #include "common.cuh"
-
 #include "hydro.cuh"
 #include "linesolve.cuh"
+#include "rowsolve.cuh"
 #include "sediment_cell.cuh"
 
 namespace hyd {
@@ -75,24 +77,22 @@ struct HydroGen {
       return;
     }
     if (!ok) return;
+    // (count and ends in one round of latency)
     const int n = DIR == 0 ? S.mocj[lp] : S.moci[lp];
+    const int first = (DIR == 0 ? S.dauj : S.daui)[lp * SEG + s];
+    const int last = (DIR == 0 ? S.cuoij : S.cuoii)[lp * SEG + s];
     if (s >= n) return;
     const int w = S.W;
     SegD& d = LS.s[s];
-    int first, last;
     bool br1, br2;
     bool q1, q2;
     if (DIR == 0) {
-      first = S.dauj[lp * SEG + s];
-      last = S.cuoij[lp * SEG + s];
       // locate_segment_u (support_funcs.cpp:845-851)
       br1 = (first > 2) || ((first == 2) && ((S.h[1 * w + lp] + S.h[1 * w + lp - 1]) * 0.5 == c.NANGDAY));
       br2 = (last < S.N) || ((last == S.N) && ((S.h[S.N * w + lp] + S.h[S.N * w + lp - 1]) * 0.5 == c.NANGDAY));
       q1 = S.bienQ[2] != 0;
       q2 = S.bienQ[3] != 0;
     } else {
-      first = S.daui[lp * SEG + s];
-      last = S.cuoii[lp * SEG + s];
       // locate_segment_v (support_funcs.cpp:823-826)
       br1 = (first > 2) || ((first == 2) && ((S.h[lp * w + first - 1] + S.h[(lp - 1) * w + first - 1]) * 0.5 == c.NANGDAY));
       br2 = (last < S.M) || ((last == S.M) && ((S.h[lp * w + last] + S.h[(lp - 1) * w + last]) * 0.5 == c.NANGDAY));
@@ -171,6 +171,71 @@ struct HydroGen {
         else D += (f4 + rc) * (R(zr - c1.z) + c1.w);
       }
       C = 0;
+    }
+  }
+
+  // a cell's operands and row for the staged row solver (rowsolve.cuh); load
+  // is in bounds for every cell of the mesh, wet or not
+  struct Ops {
+    R Hm;
+    Cont c0, c1;
+    MomF<R> m;
+  };
+  __device__ int line_pos(int line) const { return line + lp0; }
+  __device__ Ops load(int lp, int pos) const {
+    Ops o;
+    const int g = at(lp, pos), s = DIR == 0 ? S.W : 1;
+    o.Hm = depth(g - s);
+    o.c0 = cont(g);
+    o.c1 = cont(g + s);
+    o.m = DIR == 0 ? mom_x(S, c, pos, lp) : mom_y(S, c, lp, pos);
+    return o;
+  }
+  __device__ void row(const SegD& d, int lp, int pos, const Ops& o, R& A, R& B, R& C, R& D) const {
+    make_row(d, lp, pos, o.m, o.Hm, o.c0, o.c1, A, B, C, D);
+  }
+  // the part of a cell's new level that does not depend on the solution is
+  // kept where the level goes, if the emission will write it there (nothing
+  // reads t_z in between: the given levels are at cells that are not written)
+  __device__ bool level_out(const SegD& d, int pos) const {
+    return (pos > d.first || d.ran) && extract_ok(pos);
+  }
+  __device__ void keep(const SegD& d, int lp, int pos, const Ops& o) const {
+    if (level_out(d, pos)) S.tz[at(lp, pos)] = o.c0.z - (double)o.c0.w;
+  }
+  __device__ void prefetch(int lp) const {
+    const int w = S.W;
+    const size_t r = (size_t)lp * w;
+    prefetch_l2(S.u + r, w);
+    prefetch_l2(S.v + r + 2 * w, w);
+    prefetch_l2(S.Hmoi + r + w, w);
+    prefetch_l2(S.Htdu + r, w);
+    prefetch_l2(S.Htdv + r, w);
+    prefetch_l2(S.visco + r, w);
+    prefetch_l2(S.Ky1 + r, w);
+    prefetch_l2(S.Tsyw + r, w);
+    prefetch_l2(S.z + r, w);
+  }
+  // Writes what the sweep gives at cell pos, first <= pos <= last, of segment
+  // d: velocity and level, and beyond the first and at the last cell what
+  // fixup does. value(p): the solved velocity of cell p.
+  template <class V>
+  __device__ void emit_cell(const SegD& d, int lp, int pos, V value) const {
+    const int g = at(lp, pos), s = DIR == 0 ? S.W : 1;
+    if (!extract_ok(pos)) return;
+    R* v = vel_ptr();
+    if (pos < d.last) {
+      const R x = value(pos);
+      v[g] = x;
+      if (level_out(d, pos)) {
+        const double xm = pos > d.first ? value(pos - 1) : (d.qfirst ? (double)q_first(lp) : 0.0);
+        const double kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
+        S.tz[g] = S.tz[g] + kk * ((double)depth(g - s) * xm - (double)depth(g) * value(pos));
+      }
+      if (pos == d.first) end_first(d, lp, x);
+    } else {
+      const bool two = d.last > d.first;
+      end_last(d, lp, two ? value(pos - 1) : 0.0, two ? (R)value(pos - 1) : v[g - s]);
     }
   }
 
@@ -269,33 +334,37 @@ struct HydroGen {
     }
   }
 
-  // Segment ends (_uzSolver_extract_solution :558-601 / _vzSolver_ :488-536).
-  __device__ void fixup(const LineSeg& LS, const double* xlast, int line, int s) const {
-    const SegD& d = LS.s[s];
-    const int lp = line + lp0, first = d.first, last = d.last;
+  // Segment ends (_uzSolver_extract_solution :558-601 / _vzSolver_ :488-536):
+  // the velocity beyond the first cell, x the first cell's ...
+  __device__ void end_first(const SegD& d, int lp, R x) const {
+    R* vel = vel_ptr();
+    const int first = d.first;
+    if (d.br1) {
+      vel[at(lp, first - 1)] = 0;
+    } else if (d.xq_first && first == 2) {
+      vel[at(lp, first - 1)] = q_first(lp);
+    } else {
+      const double kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
+      const Cont cf = cont(at(lp, first));
+      vel[at(lp, first - 1)] = ((cf.z - cf.w) - S.tz[at(lp, first)] - kk * cf.H * x) /
+                               (-kk * depth(at(lp, first - 1)));
+    }
+  }
+  // ... and the last cell's velocity and level; x the solved velocity before
+  // it (0 where none was solved), v1 that velocity as t_u (t_v) holds it
+  __device__ void end_last(const SegD& d, int lp, double x, R v1) const {
     R* vel = vel_ptr();
     double* tz = S.tz;
+    const int first = d.first, last = d.last;
     const double kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
-    if (first < last && extract_ok(first)) {
-      if (d.br1) {
-        vel[at(lp, first - 1)] = 0;
-      } else if (d.xq_first && first == 2) {
-        vel[at(lp, first - 1)] = q_first(lp);
-      } else {
-        const Cont cf = cont(at(lp, first));
-        vel[at(lp, first - 1)] = ((cf.z - cf.w) - tz[at(lp, first)] - kk * cf.H * vel[at(lp, first)]) /
-                                 (-kk * depth(at(lp, first - 1)));
-      }
-    }
-    if (!extract_ok(last)) return;
     const Cont cl = cont(at(lp, last));
     const double d2 = cl.z - cl.w;
     // the value of the reference system's last row: the last cell's level, the
     // last velocity where that level is given, 0 where no row was solved
     double xl = 0.0;
     if (last > first) {
-      xl = d.last_kind == 2 ? xlast[s]
-                            : d2 + kk * depth(at(lp, last - 1)) * xlast[s] -
+      xl = d.last_kind == 2 ? x
+                            : d2 + kk * depth(at(lp, last - 1)) * x -
                                   (d.last_kind == 1 ? kk * cl.H * q_last(lp) : 0.0);
     } else if (d.ran && d.last_kind != 2) {
       xl = d2 - (d.last_kind == 1 ? kk * cl.H * q_last(lp) : 0.0);
@@ -307,9 +376,15 @@ struct HydroGen {
       vel[at(lp, last)] = q_last(lp);
       tz[at(lp, last)] = xl;
     } else {
-      vel[at(lp, last)] =
-          (d2 + kk * depth(at(lp, last - 1)) * vel[at(lp, last - 1)] - tz[at(lp, last)]) / (kk * cl.H);
+      vel[at(lp, last)] = (d2 + kk * depth(at(lp, last - 1)) * v1 - tz[at(lp, last)]) / (kk * cl.H);
     }
+  }
+  // both ends of segment s (after the emission)
+  __device__ void fixup(const LineSeg& LS, const double* xlast, int line, int s) const {
+    const SegD& d = LS.s[s];
+    const int lp = line + lp0;
+    if (d.first < d.last && extract_ok(d.first)) end_first(d, lp, vel_ptr()[at(lp, d.first)]);
+    if (extract_ok(d.last)) end_last(d, lp, d.last > d.first ? xlast[s] : 0.0, vel_ptr()[at(lp, d.last - 1)]);
   }
   __device__ R* vel_ptr() const { return DIR == 0 ? S.tu : S.tv; }
 };
@@ -357,95 +432,103 @@ static void launch_any(const Gen& G, int P, cudaStream_t st, int grid, int line0
   else launch_gen<Gen, 1>(G, st, grid, line0, ngroups, b, gpm);
 }
 
-// CTAs of the 128-chunk solver resident on the device at once (queried once
-// per device)
-template <class Gen>
-static int resident_slots() {
-  static int slots[64] = {};
+// Threads per row of the staged row solver: 5 to 9 cells each (odd chunks),
+// a warp for the shortest rows.
+static int row_threads(int ncells) {
+  return ncells <= 160 ? 32 : ncells <= 352 ? 64 : ncells <= 1152 ? 128 : ncells <= 2304 ? 256 : 512;
+}
+
+// Device limits the launches need, queried once per device.
+struct DevLimits {
+  int nsm = 0, optin = 0;
+};
+static DevLimits dev_limits() {
+  static DevLimits lim[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 64) return 0;
-  if (!slots[dev]) {
-    const size_t smem = prepare<Gen, 128, LPB>(dev);
-    int per_sm = 0, nsm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_line_solve<Gen, 128, LPB>, LPB * 128,
-                                                  smem);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    slots[dev] = per_sm * nsm;
+  if (dev < 0 || dev >= 64) return {};
+  if (!lim[dev].optin) {
+    DevLimits l;
+    cudaDeviceGetAttribute(&l.nsm, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&l.optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    lim[dev] = l;
   }
-  return slots[dev];
+  return lim[dev];
+}
+
+// The staged row solver takes rows that one CTA's shared memory holds (beside
+// its tables): about 9300 cells in FP64, 18000 in FP32, 8000 refined. Longer
+// ones keep the chunked solver with its scratch in global memory.
+template <class Gen>
+static bool row_fits(int ncells) {
+  return row_smem<Gen>(ncells) + 8192 <= (size_t)dev_limits().optin;
+}
+
+template <class Gen, int NT, int BATCH>
+static void launch_row_nt(const Gen& G, int ncells, int lines, cudaStream_t st,
+                          const Batch<typename Gen::Real>& b) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const DevLimits lim = dev_limits();
+  static bool attr[64] = {};
+  if (dev < 64 && !attr[dev]) {
+    cudaFuncSetAttribute(k_row_solve<Gen, NT, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         lim.optin - 8192);
+    attr[dev] = true;
+  }
+  k_row_solve<Gen, NT, BATCH>
+      <<<dim3(lines, std::max(b.n, 1)), NT, row_smem<Gen>(ncells), st>>>(G, b);
+}
+
+template <class Gen, int NT>
+static void launch_row_b(const Gen& G, int ncells, int lines, cudaStream_t st,
+                         const Batch<typename Gen::Real>& b) {
+  if (b.n > 0) launch_row_nt<Gen, NT, 1>(G, ncells, lines, st, b);
+  else launch_row_nt<Gen, NT, 0>(G, ncells, lines, st, b);
+}
+
+template <class Gen>
+static void launch_rows(const Gen& G, int ncells, int lines, cudaStream_t st,
+                        const Batch<typename Gen::Real>& b) {
+  switch (row_threads(ncells)) {
+    case 32: return launch_row_b<Gen, 32>(G, ncells, lines, st, b);
+    case 64: return launch_row_b<Gen, 64>(G, ncells, lines, st, b);
+    case 128: return launch_row_b<Gen, 128>(G, ncells, lines, st, b);
+    case 256: return launch_row_b<Gen, 256>(G, ncells, lines, st, b);
+    default: return launch_row_b<Gen, 512>(G, ncells, lines, st, b);
+  }
 }
 
 // Launches a sweep over `lines` lines and returns the number of launches.
-// In a row sweep whose last round of 4-line groups would leave more than
-// half of the resident CTAs idle (2047 rows on 148 one-CTA SMs: 68 of 512
-// groups), that remainder runs as a second launch of 2-line groups with 256
-// chunks per line, half the chain per thread, on every SM.
-//
 // With a batch, one launch walks the line groups of every member (the
 // persistent grid takes them in member order).
 template <class Gen>
-static int launch_lines(const Gen& G, int P, int lines, int lslots, cudaStream_t st,
+static int launch_lines(const Gen& G, int P, int ncells, int lines, int lslots, cudaStream_t st,
                         const Batch<typename Gen::Real>& b = {}) {
-  if constexpr (Gen::DIRECTION == 1 && Gen::HYDRO && !Gen::REFINE &&
-                sizeof(typename Gen::Real) == 4) {
-    if (P == 128) {
-      // the FP32 hydraulic row sweep: groups of 8 rows, one 1024-thread CTA
-      // per SM (its 64 registers as at two 512-thread CTAs): 0.130 -> 0.121
-      // ms on 2048x1024 (the FP64 one, capped from 102 registers, 0.247
-      // against 0.172: it keeps 4-row groups)
-      const int g8 = cdiv(lines, XPB);
-      const long long total = (long long)g8 * std::max(b.n, 1);
-      launch_gen<Gen, 128, XPB>(G, st, (int)std::min<long long>(total, lslots / 2), 0, (int)total,
-                                b, b.n > 0 ? g8 : 0);
-      return 1;
-    }
-  }
-  if constexpr (Gen::DIRECTION == 1 && Gen::HYDRO && Gen::REFINE) {
-    if (P == 128 && b.n == 0) {
-      // the refined hydraulic row sweep: groups of 8 rows of 64 chunks (one
-      // 512-thread CTA per SM): 0.210 -> 0.204 ms on 2048x1024 (the FP64 and
-      // FP32 ones slower that way: 0.231 / 0.153 against 0.173 / 0.131 ms)
-      const int g8 = cdiv(lines, XPB);
-      launch_gen<Gen, 64, XPB>(G, st, std::min(g8, lslots / 2), 0, g8);
-      return 1;
-    }
-  }
   if constexpr (Gen::DIRECTION == 1) {
-    if (P == 64 || (P == 128 && !Gen::HYDRO && sizeof(typename Gen::Real) == 4)) {
-      // row sweeps of 64 chunks (rows of 256 to 511 cells), and the FP32
-      // concentration row sweeps of 128: groups of 8 adjacent rows (their
-      // stencil rows shared through L1 by twice as many lines). The
-      // 64-member ensemble of 1024x512 in FP32 with refinement: 13.64 ->
-      // 12.63 ms per step (FP64 unchanged); the concentration y sweep of
-      // 2048x1024 0.122 -> 0.108 ms refined, 0.087 -> 0.079 ms in FP32 (the
-      // FP64 one 3 us slower, so it keeps 4-row groups). A group's scratch
-      // slot is two 4-line slots.
-      const int g8 = cdiv(lines, XPB);
-      const long long total = (long long)g8 * std::max(b.n, 1);
-      const int grid = (int)std::min<long long>(total, lslots / 2);
+    if (row_fits<Gen>(ncells)) {
+      launch_rows(G, ncells, lines, st, b);
+      return 1;
+    }
+    const int groups = cdiv(lines, LPB);
+    const long long total = (long long)groups * std::max(b.n, 1);
+    launch_gen<Gen, 128>(G, st, (int)std::min<long long>(total, lslots), 0, (int)total, b,
+                         b.n > 0 ? groups : 0);
+    return 1;
+  } else {
+    if constexpr (Gen::REFINE) {
       if (P == 64) {
-        launch_gen<Gen, 64, XPB>(G, st, grid, 0, (int)total, b, b.n > 0 ? g8 : 0);
-      } else if constexpr (!Gen::HYDRO && sizeof(typename Gen::Real) == 4) {
-        launch_gen<Gen, 128, XPB>(G, st, grid, 0, (int)total, b, b.n > 0 ? g8 : 0);
+        // the refined column sweeps of 64 chunks (columns of 256 to 511
+        // cells) in groups of 8 columns: a 512x256 step 0.185 -> 0.178 ms,
+        // 8 of them batched 0.576 -> 0.537 ms (the FP64 ones 3% slower that
+        // way alone, unchanged batched: they keep groups of 4)
+        const int g8 = cdiv(lines, XPB);
+        const long long total = (long long)g8 * std::max(b.n, 1);
+        launch_gen<Gen, 64, XPB>(G, st, (int)std::min<long long>(total, lslots / 2), 0, (int)total, b,
+                                 b.n > 0 ? g8 : 0);
+        return 1;
       }
-      return 1;
     }
-  }
-  if constexpr (Gen::DIRECTION == 0 && Gen::REFINE) {
-    if (P == 64) {
-      // the refined column sweeps of 64 chunks (columns of 256 to 511
-      // cells) in groups of 8 columns: a 512x256 step 0.185 -> 0.178 ms,
-      // 8 of them batched 0.576 -> 0.537 ms (the FP64 ones 3% slower that
-      // way alone, unchanged batched: they keep groups of 4)
-      const int g8 = cdiv(lines, XPB);
-      const long long total = (long long)g8 * std::max(b.n, 1);
-      launch_gen<Gen, 64, XPB>(G, st, (int)std::min<long long>(total, lslots / 2), 0, (int)total, b,
-                               b.n > 0 ? g8 : 0);
-      return 1;
-    }
-  }
-  if constexpr (Gen::DIRECTION == 0) {
     if (P == 128) {
       // column sweeps of 128 chunks: groups of 8 adjacent columns, one CTA
       // of 1024 threads per SM (a warp's loads cover 64 contiguous bytes of
@@ -462,29 +545,15 @@ static int launch_lines(const Gen& G, int P, int lines, int lslots, cudaStream_t
       }
       return 1;
     }
-  }
-  const int groups = cdiv(lines, LPB);
-  if (b.n > 0) {
-    const long long total = (long long)groups * b.n;
-    launch_any(G, P, st, (int)std::min<long long>(total, lslots), 0, (int)total, b, groups);
+    const int groups = cdiv(lines, LPB);
+    if (b.n > 0) {
+      const long long total = (long long)groups * b.n;
+      launch_any(G, P, st, (int)std::min<long long>(total, lslots), 0, (int)total, b, groups);
+      return 1;
+    }
+    launch_any(G, P, st, std::min(groups, lslots), 0, groups);
     return 1;
   }
-  if constexpr (Gen::DIRECTION == 1) {
-    if (P == 128) {
-      const int slots = std::min(resident_slots<Gen>(), lslots);
-      const int full = slots > 0 ? groups / slots : 0;
-      const int rem = groups - full * slots;
-      if (full >= 1 && rem > 0 && 2 * rem <= slots) {
-        launch_gen<Gen, 128>(G, st, slots, 0, full * slots);
-        const int line0 = full * slots * LPB;
-        const int g2 = cdiv(lines - line0, 2);
-        launch_gen<Gen, 256, 2>(G, st, std::min(g2, lslots), line0, g2);
-        return 2;
-      }
-    }
-  }
-  launch_any(G, P, st, std::min(groups, lslots), 0, groups);
-  return 1;
 }
 
 // Scratch slots for a sweep of lines of `unknowns` unknowns in P chunks:
@@ -511,7 +580,7 @@ static int launch_dir(const StateT<R>& S, const CoefT<R>& c, cudaStream_t st, in
   G.nl = DIR == 0 ? S.x_hi - S.x_lo + 1 : S.N - S.y_lo + 1;
   if (G.nl <= 0) return 0;
   const int ncells = DIR == 0 ? S.N - 1 : S.M - 1;
-  return launch_lines(G, P, G.nl, sweep_slots(S, ncells, P), st, b);
+  return launch_lines(G, P, ncells, G.nl, sweep_slots(S, ncells, P), st, b);
 }
 
 // ---------------------------------------------------------------------
@@ -554,19 +623,16 @@ struct FSGen {
     }
     if (!ok) return;
     const int n = DIR == 0 ? S.mocj[lp] : S.moci[lp];
+    const int first = (DIR == 0 ? S.dauj : S.daui)[lp * SEG + s];
+    const int last = (DIR == 0 ? S.cuoij : S.cuoii)[lp * SEG + s];
     if (s >= n) return;
     const int w = S.W;
     SegD& d = LS.s[s];
-    int first, last;
     bool br1, br2;
     if (DIR == 0) {
-      first = S.dauj[lp * SEG + s];
-      last = S.cuoij[lp * SEG + s];
       br1 = (first > 2) || ((first == 2) && ((S.h[1 * w + lp] + S.h[1 * w + lp - 1]) * 0.5 == c.NANGDAY));
       br2 = (last < S.N) || ((last == S.N) && ((S.h[S.N * w + lp] + S.h[S.N * w + lp - 1]) * 0.5 == c.NANGDAY));
     } else {
-      first = S.daui[lp * SEG + s];
-      last = S.cuoii[lp * SEG + s];
       br1 = (first > 2) || ((first == 2) && ((S.h[lp * w + first - 1] + S.h[(lp - 1) * w + first - 1]) * 0.5 == c.NANGDAY));
       br2 = (last < S.M) || ((last == S.M) && ((S.h[lp * w + last] + S.h[(lp - 1) * w + last]) * 0.5 == c.NANGDAY));
     }
@@ -577,6 +643,56 @@ struct FSGen {
     d.br1 = br1;
     d.br2 = br2;
     d.ran = d.qfirst = d.last_kind = d.xq_first = d.xq_last = 0;
+  }
+
+  // a cell's row for the staged row solver (rowsolve.cuh), from the fields
+  struct Ops {
+    R A, B, C, D;
+  };
+  __device__ int line_pos(int line) const { return line + 3; }
+  __device__ Ops load(int lp, int pos) const {
+    Ops o;
+    if (DIR == 0) fs_row<0>(S, c, pos, lp, o.A, o.B, o.C, o.D);
+    else fs_row<1>(S, c, lp, pos, o.A, o.B, o.C, o.D);
+    return o;
+  }
+  __device__ void row(const SegD& d, int lp, int pos, const Ops& o, R& A, R& B, R& C, R& D) const {
+    A = o.A;
+    B = o.B;
+    C = o.C;
+    D = o.D;
+    end_rows(d, lp, pos, A, B, C, D);
+  }
+  __device__ void keep(const SegD&, int, int, const Ops&) const {}
+  __device__ void prefetch(int lp) const {
+    const int w = S.W;
+    const size_t r = (size_t)lp * w;
+    prefetch_l2(S.Hmoi + r + 2 * w, w);
+    prefetch_l2(S.FS + r + w, w);
+    prefetch_l2(S.VTH + r, w);
+    prefetch_l2(S.Fw + r, w);
+    prefetch_l2(S.tv + r, w);
+    prefetch_l2(S.Htdv + r, w);
+    prefetch_l2(S.Ky + r, w);
+    prefetch_l2(S.tu + r, w);
+    prefetch_l2(S.Htdu + r, w);
+    prefetch_l2(S.Kx + r, w);
+  }
+  // the value stored for a solved concentration
+  __device__ R stored(double x) const { return (x < 0) ? c.NDnen : (R)x; }
+  // Writes tFS at cell pos, first <= pos <= last, of segment d, the ends as
+  // fixup does. value(p): the solved concentration of cell p.
+  template <class V>
+  __device__ void emit_cell(const SegD& d, int lp, int pos, V value) const {
+    if (d.rend < d.off) return;
+    const R* v = vel();
+    const int g = at(lp, pos);
+    if (pos == d.first)
+      S.tFS[g] = (d.br1 || v[g] == 0) ? stored(value(pos + 1)) : S.FS[g];
+    else if (pos == d.last)
+      S.tFS[g] = (d.br2 || v[g] == 0) ? stored(value(pos - 1)) : S.FS[g];
+    else
+      S.tFS[g] = stored(value(pos));
   }
 
   // Walks a chunk cell by cell; the rows come from k_fs_rows (one coalesced
@@ -693,6 +809,17 @@ struct FSGen {
   }
 };
 
+// whether the concentration row sweep forms its rows itself (else k_fs_rows
+// writes them ahead of it)
+template <class R>
+bool fs_rows_in_sweep(const StateT<R>& S, int dir) {
+  if (dir == 0) return false;
+  if constexpr (sizeof(R) == 4) {
+    if (S.refine) return row_fits<FSGen<1, R, true>>(S.M - 1);
+  }
+  return row_fits<FSGen<1, R, false>>(S.M - 1);
+}
+
 template <class R>
 int launch_fs_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t st,
                     const Batch<R>& b) {
@@ -701,12 +828,13 @@ int launch_fs_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t
   if (lines <= 0) return 0;
   const int P = line_chunks(ncells, 4);
   const int slots = sweep_slots(S, ncells, P);
-  if (dir == 0) {
-    if (S.refine) return launch_lines(FSGen<0, R, true>{S, c, S.lscratch}, P, lines, slots, st, b);
-    return launch_lines(FSGen<0, R, false>{S, c, S.lscratch}, P, lines, slots, st, b);
+  if constexpr (sizeof(R) == 4) {
+    if (S.refine && dir == 0)
+      return launch_lines(FSGen<0, R, true>{S, c, S.lscratch}, P, ncells, lines, slots, st, b);
+    if (S.refine) return launch_lines(FSGen<1, R, true>{S, c, S.lscratch}, P, ncells, lines, slots, st, b);
   }
-  if (S.refine) return launch_lines(FSGen<1, R, true>{S, c, S.lscratch}, P, lines, slots, st, b);
-  return launch_lines(FSGen<1, R, false>{S, c, S.lscratch}, P, lines, slots, st, b);
+  if (dir == 0) return launch_lines(FSGen<0, R, false>{S, c, S.lscratch}, P, ncells, lines, slots, st, b);
+  return launch_lines(FSGen<1, R, false>{S, c, S.lscratch}, P, ncells, lines, slots, st, b);
 }
 
 template <class R>
@@ -714,14 +842,18 @@ int launch_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t st
                  const Batch<R>& b) {
   const int ncells = dir == 0 ? S.N - 1 : S.M - 1;
   const int P = line_chunks(ncells, 4);
-  if (S.refine) {
-    if (dir == 0) return launch_dir<0, R, true>(S, c, st, P, b);
-    return launch_dir<1, R, true>(S, c, st, P, b);
+  if constexpr (sizeof(R) == 4) {  // (the refinement is of the FP32 form)
+    if (S.refine) {
+      if (dir == 0) return launch_dir<0, R, true>(S, c, st, P, b);
+      return launch_dir<1, R, true>(S, c, st, P, b);
+    }
   }
   if (dir == 0) return launch_dir<0, R, false>(S, c, st, P, b);
   return launch_dir<1, R, false>(S, c, st, P, b);
 }
 
+template bool fs_rows_in_sweep<double>(const StateT<double>&, int);
+template bool fs_rows_in_sweep<float>(const StateT<float>&, int);
 template int launch_sweep<double>(const StateT<double>&, const CoefT<double>&, int, cudaStream_t,
                                   const Batch<double>&);
 template int launch_sweep<float>(const StateT<float>&, const CoefT<float>&, int, cudaStream_t,

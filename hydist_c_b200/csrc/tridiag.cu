@@ -346,168 +346,10 @@ __host__ __device__ inline int bulk_region(int nmax) {
   return (nmax + 2 * E + E - 1) / E * E;
 }
 
-// the odd chunk length of a system of n rows on NT threads (at least 3)
-__device__ __forceinline__ int bulk_chunk(int n, int NT) {
-  int S = (n + NT - 1) / NT;
-  if (S < 3) S = 3;
-  return S | 1;
-}
-
 // waits of the staging barrier before a CTA gives a system up (each try
 // suspends the thread for a while; a stalled copy is reported, not waited
 // for without end)
 constexpr long GT_WAIT_TRIES = 1L << 22;
-
-// The rows of one chunk, eliminated forward (in place where KEEP): its
-// separator row, its first interior row in terms of both neighbouring
-// separators (yF, vF, wF) and its last one (yL, vL, wL).
-template <class T>
-struct ChunkEnds {
-  T as = 0, bs = 1, cs = 0, ds = 0;
-  T yF = 0, vF = 0, wF = 1, yL = 0, vL = 0, wL = 0;
-};
-
-// row(q, A, B, C, D) gives row q of the tile's rows
-template <bool KEEP, class T, class Row>
-__device__ __forceinline__ ChunkEnds<T> chunk_forward(T* rA, T* rC, T* rD, int q0, int nu, Row row) {
-  ChunkEnds<T> e;
-  T cp = 0, yp = 0, vp = 0;
-  for (int s = 0; s < nu - 1; ++s) {
-    T A, B, C, D;
-    row(q0 + s, A, B, C, D);
-    if (s == 0) {
-      const T m = T(1) / B;
-      cp = C * m;
-      yp = D * m;
-      vp = -A * m;
-    } else {
-      const T m = T(1) / (B - A * cp);
-      yp = (D - A * yp) * m;
-      vp = -A * vp * m;
-      cp = C * m;
-    }
-    if constexpr (KEEP) {
-      rC[q0 + s] = cp;
-      rD[q0 + s] = yp;
-      rA[q0 + s] = vp;
-    }
-    e.yF += e.wF * yp;
-    e.vF += e.wF * vp;
-    e.wF *= -cp;
-  }
-  if (nu > 0) row(q0 + nu - 1, e.as, e.bs, e.cs, e.ds);
-  e.yL = yp;
-  e.vL = vp;
-  e.wL = -cp;
-  return e;
-}
-
-// One level of parallel cyclic reduction on normalised rows (unit diagonal:
-// one reciprocal a level): a, c, d of this lane against the lanes st below
-// and above, where up / dn. A coupling with no partner stays: it is to the
-// unknown beyond the lanes' end.
-template <class T>
-__device__ __forceinline__ void pcr_level(T& a, T& c, T& d, int st, bool up, bool dn) {
-  constexpr unsigned full = 0xffffffffu;
-  T am = __shfl_up_sync(full, a, st), cm = __shfl_up_sync(full, c, st), dm = __shfl_up_sync(full, d, st);
-  T an = __shfl_down_sync(full, a, st), cn = __shfl_down_sync(full, c, st), dn_ = __shfl_down_sync(full, d, st);
-  const T au = up ? a : T(0), cd = dn ? c : T(0);
-  const T r = T(1) / (T(1) - au * cm - cd * an);
-  d = (d - au * dm - cd * dn_) * r;
-  a = (up ? -a * am : a) * r;
-  c = (dn ? -c * cn : c) * r;
-}
-
-// A tile's separators, one per thread of NT: each warp reduces the chunks of
-// its lanes by shuffles, lanes 0..30 to x = d - a XL - c XR (XL, XR the
-// previous and this warp's last separators: a coupling out of the warp stays
-// in its row), then every warp solves the warps' last separators, one lane
-// each, by shuffles again: one barrier, against two per level of a reduction
-// over the CTA in shared memory (16 of them for 256 chunks).
-// blk: NT / 32 rows of 8 values. FULL: the whole tile is solved here; x and xl
-// come back as this chunk's and the previous chunk's separators. Otherwise
-// the tile's last separator is the tile's own unknown and tile[0..6] gets the
-// first unknown's e0 + e1 XL + e2 X and the row A XL + B X + cs x_next = D
-// (written by thread 0).
-template <class T, int NT, bool FULL>
-__device__ __forceinline__ void tile_reduce(const ChunkEnds<T>& e, T (*blk)[8], T& x, T& xl, T* tile) {
-  constexpr unsigned full = 0xffffffffu;
-  constexpr int W = NT / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const T nyF = __shfl_down_sync(full, e.yF, 1), nvF = __shfl_down_sync(full, e.vF, 1),
-          nwF = __shfl_down_sync(full, e.wF, 1);
-  const T ra = e.as * e.vL, rb = e.bs + e.as * e.wL, rd = e.ds - e.as * e.yL;
-  T a, c, d;
-  {
-    const T inv = T(1) / (rb + e.cs * nvF);
-    a = ra * inv;
-    c = e.cs * nwF * inv;
-    d = (rd - e.cs * nyF) * inv;
-    // (lane 31 holds the warp's separator, whose row is completed below)
-    if (lane == 31) a = c = d = 0;
-  }
-#pragma unroll
-  for (int st = 1; st < 32; st <<= 1) pcr_level(a, c, d, st, lane >= st, lane + st < 31);
-  {
-    const T a30 = __shfl_up_sync(full, a, 1), c30 = __shfl_up_sync(full, c, 1), d30 = __shfl_up_sync(full, d, 1);
-    if (lane == 0) {
-      blk[warp][0] = e.yF + e.wF * d;
-      blk[warp][1] = e.vF - e.wF * a;
-      blk[warp][2] = -e.wF * c;
-    }
-    if (lane == 31) {
-      blk[warp][3] = -ra * a30;
-      blk[warp][4] = rb - ra * c30;
-      blk[warp][5] = e.cs;
-      blk[warp][6] = rd - ra * d30;
-    }
-  }
-  __syncthreads();
-  // the warps' separators: lane l takes warp l's (not the tile's last one
-  // where that is the tile's unknown)
-  constexpr int V = FULL ? W : W - 1;
-  T A = 0, B = 1, C = 0, D = 0;
-  if (lane < V) {
-    A = blk[lane][3];
-    B = blk[lane][4];
-    C = blk[lane][5];
-    D = blk[lane][6];
-    if (lane + 1 < W) {
-      B += C * blk[lane + 1][1];
-      D -= C * blk[lane + 1][0];
-      C *= blk[lane + 1][2];
-    } else {
-      C = 0;
-    }
-  }
-  {
-    const T inv = T(1) / B;
-    A *= inv;
-    C *= inv;
-    D *= inv;
-  }
-#pragma unroll
-  for (int st = 1; st < V; st <<= 1) pcr_level(A, C, D, st, lane >= st, lane + st < V);
-  if constexpr (FULL) {
-    T XL = __shfl_sync(full, D, warp > 0 ? warp - 1 : 0);
-    if (warp == 0) XL = 0;
-    const T XR = __shfl_sync(full, D, warp);
-    x = lane == 31 ? XR : d - a * XL - c * XR;
-    xl = __shfl_up_sync(full, x, 1);
-    if (lane == 0) xl = XL;
-  } else if (warp == 0) {
-    const T Av = __shfl_sync(full, A, V - 1), Cv = __shfl_sync(full, C, V - 1), Dv = __shfl_sync(full, D, V - 1);
-    if (lane == 0) {
-      tile[0] = blk[0][0] + blk[0][2] * D;
-      tile[1] = blk[0][1] - blk[0][2] * A;
-      tile[2] = -blk[0][2] * C;
-      tile[3] = -blk[V][3] * Av;
-      tile[4] = blk[V][4] - blk[V][3] * Cv;
-      tile[5] = blk[V][5];
-      tile[6] = blk[V][6] - blk[V][3] * Dv;
-    }
-  }
-}
 
 // rows [o, o + n) of the four arrays into a buffer's regions: the bulk copies
 // of the aligned part (thread 0) ...
@@ -551,28 +393,6 @@ __device__ __forceinline__ void stage_ends(const T* const src[4], T* buf, int re
   for (int q = threadIdx.x; q < head + (n - tail0); q += NT) {
     const int r = q < head ? q : tail0 + (q - head);
     for (int a = 0; a < 4; ++a) base[(size_t)a * region + r] = src[a][o + r];
-  }
-}
-
-// The partition solve of n staged rows, the solution over rD (threads of the
-// CTA: NT); row() reads a row, the chunks walked in odd lengths.
-template <class T, int NT, class Row>
-__device__ __forceinline__ void cta_solve(T* rA, T* rC, T* rD, int n, T (*blk)[8], Row row) {
-  const int tid = threadIdx.x, S = bulk_chunk(n, NT), P = max(1, n / S);
-  const int q0 = tid * S;
-  const int nu = tid < P ? (tid == P - 1 ? n - q0 : S) : 0;
-  const ChunkEnds<T> e = chunk_forward<true>(rA, rC, rD, q0, nu, row);
-  T x, xl;
-  tile_reduce<T, NT, true>(e, blk, x, xl, nullptr);
-  if (nu > 0) {
-    rD[q0 + nu - 1] = x;
-    T xn = x;
-#pragma unroll 4
-    for (int q = q0 + nu - 2; q >= q0; --q) {
-      const T xq = rD[q] + rA[q] * xl - rC[q] * xn;
-      rD[q] = xq;
-      xn = xq;
-    }
   }
 }
 
@@ -718,7 +538,7 @@ __global__ void __launch_bounds__(GT_TILE_NT) k_gt_tiles_pass(
       D = rD[q];
     };
     if (!last) {
-      const ChunkEnds<T> e = chunk_forward<false>(rA, rC, rD, tid * 9, 9, row);
+      const ChunkEnds<T> e = chunk_forward<false>((T*)nullptr, (T*)nullptr, (T*)nullptr, tid * 9, 9, row);
       T x0, x1;
       tile_reduce<T, NT, false>(e, sh.blk, x0, x1, v);
     } else {
@@ -728,7 +548,7 @@ __global__ void __launch_bounds__(GT_TILE_NT) k_gt_tiles_pass(
       const int nu = tid < P ? (tid == P - 1 ? n - q0 : S) : 0;
       T got[2];
       for (int g = 0; g < 2; ++g) {
-        const ChunkEnds<T> e = chunk_forward<false>(rA, rC, rD, q0, nu, [&](int q, T& A, T& B, T& C, T& D) {
+        const ChunkEnds<T> e = chunk_forward<false>((T*)nullptr, (T*)nullptr, (T*)nullptr, q0, nu, [&](int q, T& A, T& B, T& C, T& D) {
           row(q, A, B, C, D);
           if (g == 1) D = q == 0 ? -A : T(0);
           if (q == 0) A = 0;
