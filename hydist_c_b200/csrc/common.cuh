@@ -76,6 +76,7 @@ struct StateT {
   int x_lo, x_hi, y_lo;
   int reset_h;     // Reset_states_horizontal in the first half-step
   int bed_fb;      // the bed change feeds back into h, htaiz, Kx1, Ky1
+  int scan_always; // the mask may change outside the step (caller-owned arrays)
   double src_start;  // the concentration sweeps' erosion source from this time
   const double *h0, *htaiz0;  // the initial bed (with bed_fb)
   // static fields
@@ -95,7 +96,7 @@ struct StateT {
   // scratch
   R* tmp;        // smoothing buffer, (N+3)*(M+3)
   R *su, *sv;    // t_u / t_v after the smoothing of the current half-step
-  int* err;      // [0]: DevErr
+  int* err;      // [0]: DevErr; [1]: this half-step dried or wetted a cell
   R* lscratch;   // partitioned line solver: one slot per resident CTA
   // the rows of the next concentration sweep (A, B, C, D of every cell:
   // four arrays of (N+3)*(M+3), array k at pre + k*W*H)

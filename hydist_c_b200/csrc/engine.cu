@@ -660,6 +660,7 @@ void mirror_common(HydistHandle* h) {
   F.y_lo = S.y_lo;
   F.reset_h = S.reset_h;
   F.bed_fb = S.bed_fb;
+  F.scan_always = S.scan_always;
   F.src_start = S.src_start;
   F.h0 = S.h0;
   F.htaiz0 = S.htaiz0;
@@ -829,6 +830,7 @@ int hydist_create_external(const HydistExternal* e, const HydistParams* p, const
   int rc = new_handle(p, o, device, e->M, e->N, e->total_time, e->bienQ, &h);
   if (rc == HYDIST_OK) rc = [&]() -> int {
     State& S = h->S;
+    S.scan_always = 1;
     S.h = e->h;
     S.hsnham = e->hsnham;
     S.visco = e->visco;

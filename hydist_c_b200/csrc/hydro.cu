@@ -4,7 +4,8 @@
 //   k_onetime_init      [Onetime_init, support_funcs.cpp:21-69]
 //   k_interp_fs_rows    [Interpolate_FS_ng, support_funcs.cpp:191-213]
 //   k_interp_fs_col     [Interpolate_FS_d, support_funcs.cpp:215-237]
-//   k_runs_flags/sort   [Find_Calculation_limits_Horizontal/Vertical, :238-343]
+//   k_runs_flags/sort, k_runs_lines
+//                       [Find_Calculation_limits_Horizontal/Vertical, :238-343]
 //   k_htuongdoi         [Htuongdoi, :346-362] (set-up; per step in the commits)
 //   k_preprocess_sides  [preprocess_data, :482-601]
 //   k_boundary          [Update_Boundary_Value/Boundary_value/FS_boundary, :603-728;
@@ -26,6 +27,7 @@
 // Formulas keep the reference's structure; nvcc may fuse a multiply and an
 // add into one FMA, which the CPU oracle does not, so results agree to
 // rounding, not bit for bit.
+#include <algorithm>
 #include <cstdio>
 
 #include "assembly.cuh"
@@ -146,10 +148,21 @@ __device__ __forceinline__ void run_flags(bool wm1, bool w, bool wp1, bool wm2_l
 // reads as dried (1) and is written so. Reading a neighbour's mask while
 // its thread writes it is safe: the write turns 0 into 1 exactly when this
 // test gives 1.
+//
+// A scan within a step (always = 0) returns at once when no cell dried or was
+// wetted in this half-step (State::err[1], set by the wetting pass and the
+// commit, cleared by the boundary update): the tables hold for that mask
+// already. 19 + 3 us of a 2048x1024 step -> 2 + 2.
+template <class R>
+__device__ __forceinline__ bool scan_needed(const StateT<R>& S, int always) {
+  return always || S.scan_always || S.err[1] != 0;
+}
+
 template <class R, int BATCH = 0>
-__global__ void k_runs_flags(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int dry) {
+__global__ void k_runs_flags(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int dry, int always) {
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
+  if (!scan_needed(S, always)) return;
   int* seg_cnt = S.segcnt;
   const int j = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int i = blockIdx.y + 2;
@@ -235,8 +248,9 @@ __device__ __forceinline__ void sort_small(int* a, int n) {
 // One thread per line: order the claimed slots, set the counts, clear the
 // counters for the next scan.
 template <class R, int BATCH = 0>
-__global__ void k_runs_sort(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+__global__ void k_runs_sort(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int always) {
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
+  if (!scan_needed(S, always)) return;
   int* seg_cnt = S.segcnt;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int H = S.H, W = S.W;
@@ -268,6 +282,93 @@ __global__ void k_runs_sort(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
   *moc = n;
   *cs = 0;
   *ce = 0;
+}
+
+// The same tables in one launch on small meshes: a warp per line, which holds
+// the whole line's wet cells as words (one round of loads for up to 32 *
+// SCAN_WORDS cells) and numbers the runs in order by bit counts. Rows
+// write the dried cells' masks; the columns test them for themselves.
+constexpr int SCAN_WORDS = 8;
+constexpr int SCAN_MAX = 32 * SCAN_WORDS;  // positions 2..lim of a line
+
+template <class R, int BATCH = 0>
+__global__ void k_runs_lines(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int dry, int always) {
+  const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
+  const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
+  if (!scan_needed(S, always)) return;
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int nrow = S.N - 1, ncol = S.M - 1;
+  if (t >= nrow + ncol) return;
+  const bool isrow = t < nrow;
+  const int line = (isrow ? t : t - nrow) + 2, lim = isrow ? S.M : S.N, W = S.W;
+  int* K = S.khouot;
+  const int ilo = dry == 2 ? 1 : 2, jlo = dry == 2 ? 2 : 1;
+  // the mask at (i, j) after the drying pass
+  auto mask = [&](int i, int j, int k, R h) {
+    return dry && k == 0 && i >= ilo && i <= S.N && j >= jlo && j <= S.M && h <= c.H_TINH ? 1 : k;
+  };
+  int k[SCAN_WORDS];
+  R h[SCAN_WORDS];
+#pragma unroll
+  for (int w = 0; w < SCAN_WORDS; ++w) {
+    const int p = 2 + 32 * w + lane, g = isrow ? line * W + p : p * W + line;
+    k[w] = p <= lim ? K[g] : 2;
+    h[w] = dry && p <= lim ? S.Hmoi[g] : R(0);
+  }
+  if (dry && isrow) {
+    // the cells outside the scan's range that the drying pass reaches
+    if (dry == 1 && lane == 0) {
+      const int g = line * W + 1;
+      if (mask(line, 1, K[g], S.Hmoi[g]) != K[g]) K[g] = 1;
+    }
+    if (dry == 2 && line == 2)
+      for (int j = 2 + lane; j <= S.M; j += 32) {
+        const int g = W + j;
+        if (mask(1, j, K[g], S.Hmoi[g]) != K[g]) K[g] = 1;
+      }
+  }
+  unsigned word[SCAN_WORDS + 1];
+#pragma unroll
+  for (int w = 0; w < SCAN_WORDS; ++w) {
+    const int p = 2 + 32 * w + lane, i = isrow ? line : p, j = isrow ? p : line;
+    const int m = mask(i, j, k[w], h[w]);
+    if (isrow && m != k[w]) K[i * W + j] = m;
+    word[w] = __ballot_sync(0xffffffffu, m == 0);
+  }
+  word[SCAN_WORDS] = 0;
+  int* dau = (isrow ? S.daui : S.dauj) + line * SEG;
+  int* cuoi = (isrow ? S.cuoii : S.cuoij) + line * SEG;
+  // wet(p), p >= 2
+  auto wet = [&](int p) {
+    const int b = p - 2;
+    bool r = false;
+#pragma unroll
+    for (int w = 0; w < SCAN_WORDS; ++w)
+      if (w == b >> 5) r = word[w] >> (b & 31) & 1;
+    return b >= 0 && r;
+  };
+  const bool w2 = wet(lim - 2), w1 = wet(lim - 1);
+  int ns = 0, ne = 0;
+  const unsigned below = (1u << lane) - 1;
+#pragma unroll
+  for (int w = 0; w < SCAN_WORDS; ++w) {
+    const int p = 2 + 32 * w + lane;
+    const bool is = word[w] >> lane & 1;
+    const bool before = lane ? word[w] >> (lane - 1) & 1 : (w ? word[w - 1] >> 31 : 0);
+    const bool after = lane < 31 ? word[w] >> (lane + 1) & 1 : word[w + 1] & 1;
+    const bool st = is && !before && p <= lim - 2;
+    const bool en = is && !after && (p != lim - 1 || w2) && (p != lim || (w1 && w2));
+    const unsigned bs = __ballot_sync(0xffffffffu, st), be = __ballot_sync(0xffffffffu, en);
+    const int rs = ns + __popc(bs & below), re = ne + __popc(be & below);
+    if (st && rs < SEG) dau[rs] = p;
+    if (en && re < SEG) cuoi[re] = p;
+    ns += __popc(bs);
+    ne += __popc(be);
+  }
+  if (lane == 0) {
+    if (ns > SEG || ne != ns) atomicOr(S.err, DEV_SEG_OVERFLOW);
+    (isrow ? S.moci : S.mocj)[line] = min(ns, SEG);
+  }
 }
 
 template <class R>
@@ -401,6 +502,7 @@ __device__ __forceinline__ void boundary_cells(StateT<R> S_arg, CoefT<R> c_arg, 
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
   const int M = S.M, N = S.N, W = S.W;
   const double t_new = S.clock[0] + half;
+  if (half != 0 && blockIdx.x == 0 && threadIdx.x == 0) S.err[1] = 0;
   if (half != 0) {
     __syncthreads();  // every thread of the block has read the clock
     if (threadIdx.x == 0 && atomicAdd(&S.clock[1], 1.0) == (double)(gridDim.x - 1)) {
@@ -759,6 +861,7 @@ __global__ void k_wetting(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
   if (j > S.M) return;
   if (!colflag[j]) return;
   colflag[j] = 0;
+  S.err[1] = 1;  // (it may wet a cell)
   const int off = S.W, N = S.N;
   double* tz = S.tz;
   R* Hm = S.Hmoi;
@@ -792,6 +895,7 @@ __global__ void k_wetting_rows(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) 
   if (i > S.N) return;
   if (!rowflag[i]) return;
   rowflag[i] = 0;
+  S.err[1] = 1;  // (it may wet a cell)
   const int M = S.M;
   const size_t r = (size_t)i * S.W;
   double* tz = S.tz;
@@ -879,7 +983,10 @@ __device__ __forceinline__ void commit_b_cells(StateT<R> S_arg, CoefT<R> c_arg, 
   if (d0 || dright) tv = 0;
   S.tu[g] = tu;
   S.tv[g] = tv;
-  if (d0) S.FS[g] = 0;  // khouot is set by the segment scan after this pass
+  if (d0) {  // khouot is set by the segment scan after this pass
+    S.FS[g] = 0;
+    S.err[1] = 1;
+  }
   S.z[g] = tz;
   S.u[g] = tu * (1 - c.kenhhepd);
   S.v[g] = tv * (1 - c.kenhhepng);
@@ -997,11 +1104,26 @@ void launch_boundary(const StateT<R>& S, const CoefT<R>& c, cudaStream_t st) {
   launch2(HYD_K2B(k_boundary, R), dim3(cdiv(max(S.M, S.N), 128)), 128, st, S, c, Batch<R>{}, 0.0);
 }
 
+// the segment tables from the mask; dry: 0 none, 1 / 2 the vertical /
+// horizontal drying pass on the fly; always: whatever the half-step did to the
+// mask. Returns the launches.
+template <class R>
+static int scan(const StateT<R>& S, const CoefT<R>& c, int dry, bool always, cudaStream_t st,
+                const Batch<R>& b) {
+  const int a = always ? 1 : 0;
+  if (std::max(S.M, S.N) - 1 <= SCAN_MAX) {
+    launch2(HYD_K2(k_runs_lines, R), dim3(cdiv(S.N + S.M - 2, 4)), 128, st, S, c, b, dry, a);
+    return 1;
+  }
+  launch2(HYD_K2(k_runs_flags, R), grid2(S.M - 1, S.N - 1, 128), 128, st, S, c, b, dry, a);
+  launch2(HYD_K2(k_runs_sort, R), dim3(cdiv(S.N + S.M - 2, 128)), 128, st, S, c, b, a);
+  return 2;
+}
+
 template <class R>
 void launch_scan_segments(const StateT<R>& S, const CoefT<R>& c, bool dry, cudaStream_t st,
                           const Batch<R>& b) {
-  launch2(HYD_K2(k_runs_flags, R), grid2(S.M - 1, S.N - 1, 128), 128, st, S, c, b, dry ? 1 : 0);
-  launch2(HYD_K2(k_runs_sort, R), dim3(cdiv(S.N + S.M - 2, 128)), 128, st, S, c, b);
+  scan(S, c, dry ? 1 : 0, true, st, b);
 }
 
 template <class R>
@@ -1009,8 +1131,8 @@ void launch_find_limits(const StateT<R>& S, const CoefT<R>& c, bool dry, cudaStr
                         Trace* tr, const Batch<R>& b) {
   launch2(HYD_K2(k_interp_fs_rows, R), dim3(cdiv(S.M, 128), 2), 128, st, S, c, b);
   launch2(HYD_K2(k_interp_fs_col, R), dim3(cdiv(S.M, 128)), 128, st, S, c, b);
-  launch_scan_segments(S, c, dry, st, b);
-  if (tr) tr->launches += 4;
+  const int n = scan(S, c, dry ? 1 : 0, !dry, st, b);
+  if (tr) tr->launches += 2 + n;
 }
 
 template <class R>
@@ -1043,9 +1165,8 @@ void launch_half_x(const StateT<R>& S, const CoefT<R>& c, bool sed, cudaStream_t
     launch2(HYD_K2B(k_commit_b, R, 1), commit, 128, st, S, c, b, sed ? S.N : 0, 0);
     launch2(HYD_K2(k_interp_fs_rows, R), dim3(cdiv(S.M, 128), 2), 128, st, S, c, b);
     launch2(HYD_K2(k_interp_fs_col, R), dim3(cdiv(S.M, 128)), 128, st, S, c, b);
-    launch2(HYD_K2(k_runs_flags, R), grid2(S.M - 1, S.N - 1, 128), 128, st, S, c, b, 2);
-    launch2(HYD_K2(k_runs_sort, R), dim3(cdiv(S.N + S.M - 2, 128)), 128, st, S, c, b);
-    if (tr) tr->mark(st, PH_COMMIT_X, 6);
+    const int n = scan(S, c, 2, false, st, b);
+    if (tr) tr->mark(st, PH_COMMIT_X, 4 + n);
     return;
   }
   launch2(HYD_K2(k_smooth_full, R, 0, 0), smooth, 128, st, S, c, b);
