@@ -44,25 +44,29 @@ __device__ __forceinline__ MomF<R> mom_x(const StateT<R>& S, const CoefT<R>& c, 
   const R vtb = (v[g - 1] + v[g] + v[g + w - 1] + v[g + w]) * R(0.25);
   const R uu = u[g], VI = S.visco[g], Hu = S.Htdu[g];
   const R dT = c.dT;
+  // the cross-line stencil (columns j-2..j+2, inside the array for columns
+  // 2..M) loaded before the upwind tests choose from it
+  const R um1 = u[g - 1], um2 = u[g - 2], up1 = u[g + 1], up2 = u[g + 2];
+  const R hm1 = Hm[g - 1], hp1 = Hm[g + 1], hm2 = Hm[g - 2];
   const R rH = R(1) / Hu;
   const R visc = VI * c.dT_dXbp;
   P.f1 = c.dTchia2dX * uu + visc;
   P.f2 = -(2 + S.Kx1[g] * dT * sqrt(uu * uu + vtb * vtb) * rH + 2 * visc);
   P.f3 = visc - c.dTchia2dX * uu;
-  if (Hm[g - 1] <= c.H_TINH) {
+  if (hm1 <= c.H_TINH) {
     if (vtb < 0) {
-      p = vtb * (-3 * uu + 4 * u[g + 1] - u[g + 2]) * c.r_dY2;
-      q = (uu - 2 * u[g + 1] + u[g + 2]) * c.r_dYbp;
+      p = vtb * (-3 * uu + 4 * up1 - up2) * c.r_dY2;
+      q = (uu - 2 * up1 + up2) * c.r_dYbp;
     }
   } else {
-    if (Hm[g + 1] <= c.H_TINH) {
-      if ((Hm[g - 2] > c.H_TINH) && (vtb > 0)) {
-        p = vtb * (3 * uu - 4 * u[g - 1] + u[g - 2]) * c.r_dY2;
-        q = (uu - 2 * u[g - 1] + u[g - 2]) * c.r_dYbp;
+    if (hp1 <= c.H_TINH) {
+      if ((hm2 > c.H_TINH) && (vtb > 0)) {
+        p = vtb * (3 * uu - 4 * um1 + um2) * c.r_dY2;
+        q = (uu - 2 * um1 + um2) * c.r_dYbp;
       }
     } else {
-      p = vtb * (u[g + 1] - u[g - 1]) * c.r_dY2;
-      q = (u[g + 1] - 2 * uu + u[g - 1]) * c.r_dYbp;
+      p = vtb * (up1 - um1) * c.r_dY2;
+      q = (up1 - 2 * uu + um1) * c.r_dYbp;
     }
   }
   P.f5 = -2 * uu + dT * p - dT * c.CORIOLIS_FORCE * vtb - dT * VI * q -

@@ -7,13 +7,14 @@
 // continuity rows eliminated, make_row) on the fly (assembly.cuh) and write
 // the extraction of UZSolver_extract_solution / VZSolver_extract_solution
 // (UVZSolver_multithread.cpp:472-603) directly from the solution, each cell's
-// level by its continuity row. FP64 on 2048x1024, against the interleaved
-// system: XXX
+// level by its continuity row: against the interleaved system on 2048x1024
+// (FP64, the same chunked solver) x 0.151 -> 0.111 ms, y 0.172 -> 0.148.
 #include <algorithm>
 
 #include "assembly.cuh"
 #include "common.cuh"
 #include "hydro.cuh"
+#include "colsolve.cuh"
 #include "linesolve.cuh"
 #include "rowsolve.cuh"
 #include "sediment_cell.cuh"
@@ -69,21 +70,15 @@ struct HydroGen {
   // the VZ extraction reaches columns j <= N only (UVZSolver_multithread.cpp:851)
   __device__ bool extract_ok(int p) const { return DIR == 0 ? true : p <= S.N; }
 
-  __device__ void load_segment(LineSeg& LS, int line, int s) const {
-    const bool ok = line < lines();
-    const int lp = line + lp0;
-    if (s == SEG) {
-      LS.nseg = ok ? (DIR == 0 ? S.mocj[lp] : S.moci[lp]) : 0;
-      return;
-    }
-    if (!ok) return;
-    // (count and ends in one round of latency)
-    const int n = DIR == 0 ? S.mocj[lp] : S.moci[lp];
+  __device__ int segments(int lp) const { return DIR == 0 ? S.mocj[lp] : S.moci[lp]; }
+  // segment s of line position lp (false if the line has no such segment;
+  // count and ends in one round of latency)
+  __device__ bool segment(int lp, int s, SegD& d) const {
+    const int n = segments(lp);
     const int first = (DIR == 0 ? S.dauj : S.daui)[lp * SEG + s];
     const int last = (DIR == 0 ? S.cuoij : S.cuoii)[lp * SEG + s];
-    if (s >= n) return;
+    if (s >= n) return false;
     const int w = S.W;
-    SegD& d = LS.s[s];
     bool br1, br2;
     bool q1, q2;
     if (DIR == 0) {
@@ -111,6 +106,12 @@ struct HydroGen {
     d.last_kind = (unsigned char)L.last_kind;
     d.xq_first = q1;
     d.xq_last = q2;
+    return true;
+  }
+  __device__ void load_segment(LineSeg& LS, int line, int s) const {
+    const bool ok = line < lines();
+    if (s == SEG) LS.nseg = ok ? segments(line_pos(line)) : 0;
+    else if (ok) segment(line_pos(line), s, LS.s[s]);
   }
 
   // One cell's continuity values: depth at its velocity point, level, and the
@@ -421,17 +422,6 @@ static void launch_gen(const Gen& G, cudaStream_t st, int grid, int line0, int n
   }
 }
 
-template <class Gen>
-static void launch_any(const Gen& G, int P, cudaStream_t st, int grid, int line0, int ngroups,
-                       const Batch<typename Gen::Real>& b = {}, int gpm = 0) {
-  if (P == 128) launch_gen<Gen, 128>(G, st, grid, line0, ngroups, b, gpm);
-  else if (P == 64) launch_gen<Gen, 64>(G, st, grid, line0, ngroups, b, gpm);
-  else if (P == 32) launch_gen<Gen, 32>(G, st, grid, line0, ngroups, b, gpm);
-  else if (P == 16) launch_gen<Gen, 16>(G, st, grid, line0, ngroups, b, gpm);
-  else if (P == 4) launch_gen<Gen, 4>(G, st, grid, line0, ngroups, b, gpm);
-  else launch_gen<Gen, 1>(G, st, grid, line0, ngroups, b, gpm);
-}
-
 // Threads per row of the staged row solver: 5 to 9 cells each (odd chunks),
 // a warp for the shortest rows.
 static int row_threads(int ncells) {
@@ -499,6 +489,53 @@ static void launch_rows(const Gen& G, int ncells, int lines, cudaStream_t st,
   }
 }
 
+// The staged column solver takes columns of up to COL_MAX cells, a 32-byte
+// sector of them per CTA (4 in FP64 and refined, 8 in FP32; up to 8800 cells
+// and 106 KB). Hydraulic x sweep, chunked -> staged: 64x32 50 -> 13 us,
+// 256x128 31 -> 19, 512x256 32 -> 23, 1024x512 58 -> 42 (FP64; FP32 44 -> 37,
+// refined 54 -> 39); at 2048x1024 its 196 KB of rows in one CTA per SM lose
+// (111 -> 220, two columns per CTA 168), so longer columns keep the chunks.
+constexpr int COL_MAX = 1100;
+template <class Gen>
+constexpr int col_group() {
+  return sizeof(typename Gen::Real) == 8 || Gen::REFINE ? 4 : 8;
+}
+static bool cols_fit(int ncells) { return ncells <= COL_MAX; }
+
+template <class Gen, int NT, int L, int BATCH>
+static void launch_col_nt(const Gen& G, int ncells, int lines, cudaStream_t st,
+                          const Batch<typename Gen::Real>& b) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  static bool attr[64] = {};
+  if (dev < 64 && !attr[dev]) {
+    cudaFuncSetAttribute(k_col_solve<Gen, NT, L, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)col_smem<Gen, L>(COL_MAX));
+    attr[dev] = true;
+  }
+  k_col_solve<Gen, NT, L, BATCH>
+      <<<dim3(cdiv(lines, L), std::max(b.n, 1)), NT, col_smem<Gen, L>(ncells), st>>>(G, b);
+}
+
+// Threads of a column group: about eight cells each, four on short columns
+// (where the rounds of loads, not their number, count).
+template <class Gen, int L, int BATCH>
+static void launch_col_l(const Gen& G, int ncells, int lines, cudaStream_t st,
+                         const Batch<typename Gen::Real>& b) {
+  const int cells = ncells * L;
+  if (cells <= 512) launch_col_nt<Gen, 128, L, BATCH>(G, ncells, lines, st, b);
+  else if (cells <= 1536) launch_col_nt<Gen, 256, L, BATCH>(G, ncells, lines, st, b);
+  else if (L < 8 || cells <= 4096) launch_col_nt<Gen, 512, L, BATCH>(G, ncells, lines, st, b);
+  else if constexpr (L == 8) launch_col_nt<Gen, 1024, L, BATCH>(G, ncells, lines, st, b);
+}
+
+template <class Gen, int L>
+static void launch_cols(const Gen& G, int ncells, int lines, cudaStream_t st,
+                        const Batch<typename Gen::Real>& b) {
+  if (b.n > 0) launch_col_l<Gen, L, 1>(G, ncells, lines, st, b);
+  else launch_col_l<Gen, L, 0>(G, ncells, lines, st, b);
+}
+
 // Launches a sweep over `lines` lines and returns the number of launches.
 // With a batch, one launch walks the line groups of every member (the
 // persistent grid takes them in member order).
@@ -516,42 +553,16 @@ static int launch_lines(const Gen& G, int P, int ncells, int lines, int lslots, 
                          b.n > 0 ? groups : 0);
     return 1;
   } else {
-    if constexpr (Gen::REFINE) {
-      if (P == 64) {
-        // the refined column sweeps of 64 chunks (columns of 256 to 511
-        // cells) in groups of 8 columns: a 512x256 step 0.185 -> 0.178 ms,
-        // 8 of them batched 0.576 -> 0.537 ms (the FP64 ones 3% slower that
-        // way alone, unchanged batched: they keep groups of 4)
-        const int g8 = cdiv(lines, XPB);
-        const long long total = (long long)g8 * std::max(b.n, 1);
-        launch_gen<Gen, 64, XPB>(G, st, (int)std::min<long long>(total, lslots / 2), 0, (int)total, b,
-                                 b.n > 0 ? g8 : 0);
-        return 1;
-      }
-    }
-    if (P == 128) {
-      // column sweeps of 128 chunks: groups of 8 adjacent columns, one CTA
-      // of 1024 threads per SM (a warp's loads cover 64 contiguous bytes of
-      // each of 4 chunk rows; a group's scratch slot is two of the 4-line
-      // slots): 0.169 -> 0.153 ms for the FP64 hydraulic x sweep of
-      // 2048x1024, 0.216 -> 0.154 ms refined in FP32
-      const int g8 = cdiv(lines, XPB);
-      if (b.n > 0) {
-        const long long total = (long long)g8 * b.n;
-        launch_gen<Gen, 128, XPB>(G, st, (int)std::min<long long>(total, lslots / 2), 0, (int)total,
-                                  b, g8);
-      } else {
-        launch_gen<Gen, 128, XPB>(G, st, std::min(g8, lslots / 2), 0, g8);
-      }
+    if (cols_fit(ncells)) {
+      launch_cols<Gen, col_group<Gen>()>(G, ncells, lines, st, b);
       return 1;
     }
-    const int groups = cdiv(lines, LPB);
-    if (b.n > 0) {
-      const long long total = (long long)groups * b.n;
-      launch_any(G, P, st, (int)std::min<long long>(total, lslots), 0, (int)total, b, groups);
-      return 1;
-    }
-    launch_any(G, P, st, std::min(groups, lslots), 0, groups);
+    // groups of 8 adjacent columns of 128 chunks, one CTA of 1024 threads
+    // per SM (a group's scratch slot is two of the 4-line slots)
+    const int g8 = cdiv(lines, XPB);
+    const long long total = (long long)g8 * std::max(b.n, 1);
+    launch_gen<Gen, 128, XPB>(G, st, (int)std::min<long long>(total, lslots / 2), 0, (int)total, b,
+                              b.n > 0 ? g8 : 0);
     return 1;
   }
 }
@@ -614,20 +625,14 @@ struct FSGen {
   __device__ int at(int lp, int p) const { return DIR == 0 ? p * S.W + lp : lp * S.W + p; }
   __device__ const R* vel() const { return DIR == 0 ? S.tu : S.tv; }
 
-  __device__ void load_segment(LineSeg& LS, int line, int s) const {
-    const bool ok = line < lines();
-    const int lp = line + 3;
-    if (s == SEG) {
-      LS.nseg = ok ? (DIR == 0 ? S.mocj[lp] : S.moci[lp]) : 0;
-      return;
-    }
-    if (!ok) return;
-    const int n = DIR == 0 ? S.mocj[lp] : S.moci[lp];
+  __device__ int segments(int lp) const { return DIR == 0 ? S.mocj[lp] : S.moci[lp]; }
+  // segment s of line position lp (false if the line has no such segment)
+  __device__ bool segment(int lp, int s, SegD& d) const {
+    const int n = segments(lp);
     const int first = (DIR == 0 ? S.dauj : S.daui)[lp * SEG + s];
     const int last = (DIR == 0 ? S.cuoij : S.cuoii)[lp * SEG + s];
-    if (s >= n) return;
+    if (s >= n) return false;
     const int w = S.W;
-    SegD& d = LS.s[s];
     bool br1, br2;
     if (DIR == 0) {
       br1 = (first > 2) || ((first == 2) && ((S.h[1 * w + lp] + S.h[1 * w + lp - 1]) * 0.5 == c.NANGDAY));
@@ -643,6 +648,12 @@ struct FSGen {
     d.br1 = br1;
     d.br2 = br2;
     d.ran = d.qfirst = d.last_kind = d.xq_first = d.xq_last = 0;
+    return true;
+  }
+  __device__ void load_segment(LineSeg& LS, int line, int s) const {
+    const bool ok = line < lines();
+    if (s == SEG) LS.nseg = ok ? segments(line_pos(line)) : 0;
+    else if (ok) segment(line_pos(line), s, LS.s[s]);
   }
 
   // a cell's row for the staged row solver (rowsolve.cuh), from the fields
@@ -809,11 +820,11 @@ struct FSGen {
   }
 };
 
-// whether the concentration row sweep forms its rows itself (else k_fs_rows
+// whether the concentration sweep forms its rows itself (else k_fs_rows
 // writes them ahead of it)
 template <class R>
 bool fs_rows_in_sweep(const StateT<R>& S, int dir) {
-  if (dir == 0) return false;
+  if (dir == 0) return cols_fit(S.N - 1);
   if constexpr (sizeof(R) == 4) {
     if (S.refine) return row_fits<FSGen<1, R, true>>(S.M - 1);
   }
