@@ -140,6 +140,7 @@ struct HydistHandle {
   // one captured step per sediment phase: [bed*4 + sed_x*2 + sed_y]
   cudaGraphExec_t graph[8] = {};
   long long graph_launches[8] = {};
+  int eager_steps[8] = {};  // of hydist_step, before it captures the phase
   Trace trace;                                    // kernel launch counter
   cudaEvent_t ev[PH_COUNT + 1] = {};
   cudaEvent_t kev[2 * KS_COUNT] = {};
@@ -956,18 +957,74 @@ int hydist_destroy(HydistHandle* h) {
   return HYDIST_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// The sediment phase of the step from h->t: which sweeps run, and the index
+// of its graph.
+struct Phase3 {
+  bool sx, sy, bd;
+  double t2;
+  int index() const { return (bd ? 4 : 0) + (sx ? 2 : 0) + (sy ? 1 : 0); }
+};
+Phase3 next_phase(const HydistHandle* h) {
+  const double t1 = h->t + 0.5 * h->c.dT, t2 = t1 + h->c.dT * 0.5;
+  return Phase3{t1 >= h->o.sediment_start, t2 >= h->o.sediment_start, bed_on(h, t2), t2};
+}
+
+// One step by its phase's graph (the time advances on the device, so the
+// launches of a step are the same every step), captured on first use.
+int graph_step(HydistHandle* h, const Phase3& ph) {
+  const int gi = ph.index();
+  cudaGraphExec_t& ex = h->graph[gi];
+  if (!ex) {
+    cudaGraph_t g = nullptr;
+    Trace tr;
+    CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    enqueue_step(h, ph.sx, ph.sy, ph.bd, &tr);
+    CK(cudaStreamEndCapture(h->stream, &g));
+    h->graph_launches[gi] = tr.launches;
+    const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
+    cudaGraphDestroy(g);
+    CK(e);
+  }
+  CK(cudaGraphLaunch(ex, h->stream));
+  h->trace.launches += h->graph_launches[gi];
+  h->t = ph.t2;
+  return HYDIST_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+// A step launched kernel by kernel costs the host about 8 us per launch, more
+// than most kernels of a small mesh run (464x324 with sediment: 200 us per
+// step, 132 us by graph): from the eighth step of a phase on, or at once where
+// the call still has eight of them to go (what the capture then costs is
+// less than they save), hydist_step replays the phase's graph too. A caller
+// that captures the handle's stream itself gets the launches.
 int hydist_step(HydistHandle* h, int32_t nsteps) {
   if (!h) return fail(HYDIST_ERR_ARG, "null handle");
   if (h->next_half) return fail(HYDIST_ERR_STATE, "the second half-step is pending");
   if (nsteps < 0) return fail(HYDIST_ERR_ARG, "negative step count");
   CK(cudaSetDevice(h->device));
   TRY(check_horizon(h, nsteps));
+  constexpr int kCapture = 8;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(h->stream, &cap));
   for (int k = 0; k < nsteps; ++k) {
-    const double t1 = h->t + 0.5 * h->c.dT;
-    const double t2 = t1 + h->c.dT * 0.5;
-    enqueue_step(h, t1 >= h->o.sediment_start, t2 >= h->o.sediment_start, bed_on(h, t2),
-                 &h->trace);
-    h->t = t2;
+    const Phase3 ph = next_phase(h);
+    const int gi = ph.index();
+    if (cap == cudaStreamCaptureStatusNone &&
+        (h->graph[gi] || nsteps - k >= kCapture || h->eager_steps[gi] >= kCapture)) {
+      TRY(graph_step(h, ph));
+      continue;
+    }
+    ++h->eager_steps[gi];
+    enqueue_step(h, ph.sx, ph.sy, ph.bd, &h->trace);
+    h->t = ph.t2;
   }
   CK(cudaGetLastError());
   return HYDIST_OK;
@@ -1019,35 +1076,12 @@ int hydist_kernel_launches(HydistHandle* h, int64_t* count) {
 }
 
 int hydist_step_graph(HydistHandle* h, int32_t nsteps) {
-  // The time advances on the device, so the launches of a step are the same
-  // every step: one graph per sediment phase, captured on first use.
   if (!h) return fail(HYDIST_ERR_ARG, "null handle");
   if (h->next_half) return fail(HYDIST_ERR_STATE, "the second half-step is pending");
   if (nsteps < 0) return fail(HYDIST_ERR_ARG, "negative step count");
   CK(cudaSetDevice(h->device));
   TRY(check_horizon(h, nsteps));
-  for (int k = 0; k < nsteps; ++k) {
-    const double t1 = h->t + 0.5 * h->c.dT;
-    const double t2 = t1 + h->c.dT * 0.5;
-    const bool sx = t1 >= h->o.sediment_start, sy = t2 >= h->o.sediment_start;
-    const bool bd = bed_on(h, t2);
-    const int gi = (bd ? 4 : 0) + (sx ? 2 : 0) + (sy ? 1 : 0);
-    cudaGraphExec_t& ex = h->graph[gi];
-    if (!ex) {
-      cudaGraph_t g = nullptr;
-      Trace tr;
-      CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-      enqueue_step(h, sx, sy, bd, &tr);
-      CK(cudaStreamEndCapture(h->stream, &g));
-      h->graph_launches[gi] = tr.launches;
-      const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
-      cudaGraphDestroy(g);
-      CK(e);
-    }
-    CK(cudaGraphLaunch(ex, h->stream));
-    h->trace.launches += h->graph_launches[gi];
-    h->t = t2;
-  }
+  for (int k = 0; k < nsteps; ++k) TRY(graph_step(h, next_phase(h)));
   return HYDIST_OK;
 }
 
