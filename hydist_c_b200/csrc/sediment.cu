@@ -23,39 +23,50 @@ namespace hyd {
 // (:479).
 // _bed_load on rows 3..N-2 (BedLoad with the j-sweep's range,
 // engine.cpp:292), cells of the row's wet segments of at least 3 cells.
+//
+// The same pass commits the concentration (Update_FS, :654-663: FS = tFS on
+// rows 1..N, columns 1..M): its stencil reads tFS, which is what FS holds
+// there after the commit (and FS beyond column M, where the commit does not
+// reach).
 template <class R, int BATCH = 0>
 __device__ __forceinline__ void bed_load_cells(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
   __shared__ int s_first[SEG], s_last[SEG];
   __shared__ int s_n;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  const int i = blockIdx.y + 3;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int i = blockIdx.y + 1;
   if (threadIdx.x < SEG) {
     s_first[threadIdx.x] = S.daui[i * SEG + threadIdx.x];
     s_last[threadIdx.x] = S.cuoii[i * SEG + threadIdx.x];
   }
   if (threadIdx.x == 0) s_n = S.moci[i];
   __syncthreads();
-  if (i >= S.N - 1 || j > S.M) return;
+  if (j > S.M) return;
   const int w = S.W, pos = i * w + j, M = S.M, N = S.N;
+  const R* FS = S.tFS;
+  const R fs = FS[pos];
+  if (i < 3 || i >= N - 1 || j < 2) {
+    S.FS[pos] = fs;
+    if (!isfinite(fs)) atomicOr(S.err, DEV_NONFINITE);
+    return;
+  }
   const int* kh = S.khouot;
-  const R *Qbx = S.Qbx, *Qby = S.Qby, *FS = S.FS;
-  // every operand (all in bounds for rows 3..N-2, columns 2..M) before the
-  // segment lookup and the upwind tests that choose among them: one round
-  // of memory latency
+  const R *Qbx = S.Qbx, *Qby = S.Qby;
+  // every operand of a cell away from dried ones (all in bounds for rows
+  // 3..N-2, columns 2..M) before the segment lookup: one round of memory
+  // latency; what only the one-sided differences beside a dried cell take is
+  // read there
   const int kN = kh[pos - w], kS = kh[pos + w], kN2 = kh[pos - 2 * w], kS2 = kh[pos + 2 * w];
   const int kW = kh[pos - 1], kE = kh[pos + 1], kW2 = kh[pos - 2], kE2 = kh[pos + 2];
-  const R tu = S.tu[pos], tv = S.tv[pos];
-  const R qx0 = Qbx[pos], qxN = Qbx[pos - w], qxS = Qbx[pos + w], qxN2 = Qbx[pos - 2 * w],
-          qxS2 = Qbx[pos + 2 * w];
-  const R qy0 = Qby[pos], qyW = Qby[pos - 1], qyE = Qby[pos + 1], qyW2 = Qby[pos - 2],
-          qyE2 = Qby[pos + 2];
-  const R fs = FS[pos], fN = FS[pos - w], fS = FS[pos + w], fW = FS[pos - 1], fE = FS[pos + 1];
+  const R qxN = Qbx[pos - w], qxS = Qbx[pos + w], qyW = Qby[pos - 1], qyE = Qby[pos + 1];
+  const R fN = FS[pos - w], fS = FS[pos + w], fW = FS[pos - 1], fE = j < M ? FS[pos + 1] : S.FS[pos + 1];
   const R hu0 = S.Htdu[pos], huN = S.Htdu[pos - w], kx0 = S.Kx[pos], kxN = S.Kx[pos - w];
   const R hv0 = S.Htdv[pos], hvW = S.Htdv[pos - 1], ky0 = S.Ky[pos], kyW = S.Ky[pos - 1];
   const R Hm = S.Hmoi[pos], vth = S.VTH[pos];
   const R fw = S.ketdinh ? S.Fw[pos] : R(0);
+  S.FS[pos] = fs;
+  if (!isfinite(fs)) atomicOr(S.err, DEV_NONFINITE);
   int first = 0, last = 0;
   for (int k = 0; k < s_n; ++k)
     if (s_first[k] <= j && j <= s_last[k]) {
@@ -66,19 +77,19 @@ __device__ __forceinline__ void bed_load_cells(StateT<R> S_arg, CoefT<R> c_arg, 
   if (last - first < 2 || j < first || j > last) return;
   R p = 0, q = 0;
   if (kN == 1) {
-    if (tu < 0) p = (-3 * qx0 + 4 * qxS - qxS2) * c.r_dX2;
+    if (S.tu[pos] < 0) p = (-3 * Qbx[pos] + 4 * qxS - Qbx[pos + 2 * w]) * c.r_dX2;
   } else {
     if (kS == 1) {
-      if (tu > 0) p = (3 * qx0 - 4 * qxN + qxN2) * c.r_dX2;
+      if (S.tu[pos] > 0) p = (3 * Qbx[pos] - 4 * qxN + Qbx[pos - 2 * w]) * c.r_dX2;
     } else {
       p = (qxS - qxN) * c.r_dX2;
     }
   }
   if (kW == 1) {
-    if (tv < 0) q = (-3 * qy0 + 4 * qyE - qyE2) * c.r_dY2;
+    if (S.tv[pos] < 0) q = (-3 * Qby[pos] + 4 * qyE - Qby[pos + 2]) * c.r_dY2;
   } else {
     if (kE == 1) {
-      if (tv > 0) q = (3 * qy0 - 4 * qyW + qyW2) * c.r_dY2;
+      if (S.tv[pos] > 0) q = (3 * Qby[pos] - 4 * qyW + Qby[pos - 2]) * c.r_dY2;
     } else {
       q = (qyE - qyW) * c.r_dY2;
     }
@@ -252,17 +263,18 @@ void launch_sediment(const StateT<R>& S, const CoefT<R>& c, bool xdir, bool bed,
   }
   const int nfs = (rows ? 1 : 0) + launch_fs_sweep(S, c, xdir ? 0 : 1, st, b);
   if (tr) tr->kend(st, xdir ? KS_FS_X : KS_FS_Y);
-  const dim3 gfs(cdiv(S.M, 128), cdiv(S.N, FS_ROWS), z);
-  if (b.n > 0) k_update_fs<R, 1><<<gfs, 128, 0, st>>>(S, c, b);
-  else k_update_fs<R, 0><<<gfs, 128, 0, st>>>(S, c, b);
   int launched = nfs + 1;
-  if (bed && S.N >= 5) {
-    // the bed change once per step, after the j-sweep (engine.cpp:290-293)
-    // the flux Qb was computed by this step's second commit (k_commit_b)
-    const dim3 gl(cdiv(S.M - 1, 128), S.N - 4, z);
+  if (!bed || S.N < 5) {
+    const dim3 gfs(cdiv(S.M, 128), cdiv(S.N, FS_ROWS), z);
+    if (b.n > 0) k_update_fs<R, 1><<<gfs, 128, 0, st>>>(S, c, b);
+    else k_update_fs<R, 0><<<gfs, 128, 0, st>>>(S, c, b);
+  } else {
+    // the bed change once per step, after the j-sweep (engine.cpp:290-293),
+    // and with it the concentration's commit; the flux Qb was computed by
+    // this step's second commit (k_commit_b)
+    const dim3 gl(cdiv(S.M, 128), S.N, z);
     if (b.n > 0) k_bed_load_b<R><<<gl, 128, 0, st>>>(S, c, b);
     else k_bed_load<R, 0><<<gl, 128, 0, st>>>(S, c, b);
-    launched += 1;
     if (S.bed_fb) {
       launch_bed_feedback(S, c, st, b);
       ++launched;
