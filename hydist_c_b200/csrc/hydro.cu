@@ -2,8 +2,8 @@
 //
 // Kernels (reference kernel each one replaces in brackets):
 //   k_onetime_init      [Onetime_init, support_funcs.cpp:21-69]
-//   k_interp_fs_rows    [Interpolate_FS_ng, support_funcs.cpp:191-213]
-//   k_interp_fs_col     [Interpolate_FS_d, support_funcs.cpp:215-237]
+//   k_interp_fs         [Interpolate_FS_ng, support_funcs.cpp:191-213,
+//                        Interpolate_FS_d, :215-237]
 //   k_runs_flags/sort, k_runs_lines
 //                       [Find_Calculation_limits_Horizontal/Vertical, :238-343]
 //   k_htuongdoi         [Htuongdoi, :346-362] (set-up; per step in the commits)
@@ -14,8 +14,8 @@
 //                        UVZSolver_multithread.cpp:19-139, 142-603, 798-933]:
 //                        sweep.cu on the partitioned solver of linesolve.cuh
 //   k_smooth_full       [Normalize/_normalize/update_buffer, :761-808]
-//   k_solve_v/k_solve_u [solveV/vSolver, solveU/uSolver, :607-795, 938-978]
-//   k_margin_v/k_margin_u [update_margin_elem_V/U, :980-1060]
+//   k_solve_v/k_solve_u [solveV/vSolver, solveU/uSolver, :607-795, 938-978;
+//                        update_margin_elem_V/U, :980-1060]
 //   k_commit_a          [update_h_moi + update_uvz + Htuongdoi, :71-86, 732-759, 346-362;
 //                        before a concentration step also Find_VTH + hesoK,
 //                        sediment_transport.cpp:575-602, 539-573]
@@ -76,14 +76,14 @@ __global__ void k_onetime_init(StateT<R> S, CoefT<R> c) {
 }
 
 // ------------------------------------------------------- segment tables
-template <class R, int BATCH = 0>
-__global__ void k_interp_fs_rows(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
-  const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
-  const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
-  // Interpolate_FS_ng at row N (offset N-1, sign -1) and row 2 (offset 2, +1)
-  const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  const int which = blockIdx.y;
-  if (j >= S.M) return;
+// The boundary concentration's interpolation in one launch: the first blocks
+// take rows N and 2 (Interpolate_FS_ng: offset N-1, sign -1; offset 2, sign
+// +1), the last of them to finish (counted in State::err[2]) then the two
+// cells of column M that read those rows, the other blocks the rest of column
+// M (Interpolate_FS_d: offset M-1, sign -1; rows 1..M-1 as the reference
+// loops them, support_funcs.cpp:227).
+template <class R>
+__device__ __forceinline__ void interp_fs_row(const StateT<R>& S, const CoefT<R>& c, int which, int j) {
   const int W = S.W;
   const int loc = which == 0 ? S.N : 2;
   const int offset = which == 0 ? S.N - 1 : 2;
@@ -102,14 +102,8 @@ __global__ void k_interp_fs_rows(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg
   }
 }
 
-template <class R, int BATCH = 0>
-__global__ void k_interp_fs_col(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
-  const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
-  const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
-  // Interpolate_FS_d at column M (offset M-1, sign -1); rows 1..M-1 as the
-  // reference loops them (support_funcs.cpp:227)
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (i >= S.M || i >= S.H) return;
+template <class R>
+__device__ __forceinline__ void interp_fs_col(const StateT<R>& S, const CoefT<R>& c, int i) {
   const int W = S.W, loc = S.M, offset = S.M - 1, sign = -1;
   if (S.tv[i * W + loc] > 0) {
     const double deltaY = (S.v[i * W + loc] + S.tv[i * W + loc]) * 0.25 * c.dT;
@@ -120,6 +114,33 @@ __global__ void k_interp_fs_col(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg)
     const int j_dY = __double2int_rn(c.dY);
     S.FS[i * W + loc] = S.FS[i * W + j + 1] +
                         (S.FS[i * W + j + 1] - S.FS[i * W + j]) * (deltaY / c.dY - j_deltaY / j_dY);
+  }
+}
+
+template <class R, int BATCH = 0>
+__global__ void __launch_bounds__(128) k_interp_fs(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
+  const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
+  const int rows = min(S.M, S.H);  // column M: rows 1 .. rows - 1
+  const int per = cdiv(S.M - 1, 128);  // blocks of a row
+  if ((int)blockIdx.x >= 2 * per) {
+    const int i = (blockIdx.x - 2 * per) * 128 + threadIdx.x + 1;
+    if (i < rows && i != 2 && i != S.N) interp_fs_col(S, c, i);
+    return;
+  }
+  const int j = (int)(blockIdx.x % per) * 128 + threadIdx.x + 1;
+  if (j < S.M) interp_fs_row(S, c, (int)blockIdx.x / per, j);
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&S.err[2], 1) == 2 * per - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) S.err[2] = 0;
+  if (threadIdx.x < 2) {
+    const int i = threadIdx.x ? S.N : 2;
+    if (i < rows) interp_fs_col(S, c, i);
   }
 }
 
@@ -677,20 +698,9 @@ __global__ void __launch_bounds__(128, BATCH ? 8 : 10)
 }
 
 // ---------------------------------------------------- explicit updates
-__device__ __forceinline__ bool find_seg(const int* dau, const int* cuoi, int n, int pos, int& first,
-                                         int& last) {
-  for (int k = 0; k < n; ++k) {
-    if (dau[k] <= pos && pos <= cuoi[k]) {
-      first = dau[k];
-      last = cuoi[k];
-      return true;
-    }
-  }
-  return false;
-}
-
-// vSolver driven by solveV (UVZSolver_multithread.cpp:607-663, 961-978);
-// the cell's arithmetic is v_new (explicit.cuh).
+// vSolver driven by solveV (UVZSolver_multithread.cpp:607-663, 961-978) with
+// update_margin_elem_V (:1018-1060); the cell's arithmetic is v_new
+// (explicit.cuh).
 template <class R, int BATCH = 0>
 __device__ __forceinline__ void solve_v_cells(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
@@ -698,11 +708,11 @@ __device__ __forceinline__ void solve_v_cells(StateT<R> S_arg, CoefT<R> c_arg, B
   // the block's cells share one row: its segment table goes to shared memory
   __shared__ int s_first[SEG], s_last[SEG];
   __shared__ int s_n;
-  const int col = blockIdx.x * blockDim.x + threadIdx.x + 2;
+  const int col = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int row = blockIdx.y + 2;
   const bool ok = row <= S.N && col <= S.M;
   const int g = row * S.W + col;
-  // every operand, in bounds for rows 2..N and columns 2..M, is loaded
+  // every operand, in bounds for rows 2..N and columns 1..M, is loaded
   // with the segment table, before the lookup that decides whether the
   // cell is updated: one round of memory latency
   VOps<R> o;
@@ -714,14 +724,21 @@ __device__ __forceinline__ void solve_v_cells(StateT<R> S_arg, CoefT<R> c_arg, B
   if (threadIdx.x == 0) s_n = S.moci[row];
   __syncthreads();
   if (!ok) return;
-  int first, last;
-  if (!find_seg(s_first, s_last, s_n, col, first, last)) return;
-  if (first >= last || col >= last || col < first) return;
-  S.tv[g] = v_new(o, c);
+  const SegHit h = seg_hit(s_first, s_last, s_n, col);
+  if (h.what == 1) {
+    S.tv[g] = v_new(o, S, c, g);
+  } else if (h.what) {
+    bool br1, br2;
+    ends_v(S, (double)c.NANGDAY, row, h.first, h.last, br1, br2);
+    const int r = row * S.W;
+    seg_ends<R>(h, br1, br2, [&](int p) { return v_new(v_ops(S, S.su, r + p), S, c, r + p); },
+                [&](int p) { return S.tv[r + p]; }, [&](int p, R x) { S.tv[r + p] = x; });
+  }
 }
 
-// uSolver driven by solveU (UVZSolver_multithread.cpp:724-795, 938-959);
-// the cell's arithmetic is u_new (explicit.cuh).
+// uSolver driven by solveU (UVZSolver_multithread.cpp:724-795, 938-959) with
+// update_margin_elem_U (:980-1016); the cell's arithmetic is u_new
+// (explicit.cuh).
 template <class R, int BATCH = 0>
 __device__ __forceinline__ void solve_u_cells(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
@@ -733,32 +750,16 @@ __device__ __forceinline__ void solve_u_cells(StateT<R> S_arg, CoefT<R> c_arg, B
   // every operand is loaded before the segment lookup (all in bounds for
   // rows 1..N, columns 2..M), so both take one round of memory latency
   const UOps<R> o = u_ops(S, S.sv, ij);  // t_v after its smoothing
-  int first, last;
-  if (!find_seg(S.dauj + col * SEG, S.cuoij + col * SEG, S.mocj[col], row, first, last)) return;
-  if (first > last || row < first - 1 || row >= last) return;
-  S.tu[ij] = u_new(o, c);
-}
-
-// update_margin_elem_V (UVZSolver_multithread.cpp:1018-1060), one row per
-// thread.
-template <class R, int BATCH = 0>
-__global__ void k_margin_v(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
-  const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
-  const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  if (i > S.N) return;
-  margin_v(S, (double)c.NANGDAY, i);
-}
-
-// update_margin_elem_U (UVZSolver_multithread.cpp:980-1016), one column per
-// thread.
-template <class R, int BATCH = 0>
-__global__ void k_margin_u(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
-  const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
-  const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
-  const int j = blockIdx.x * blockDim.x + threadIdx.x + 2;
-  if (j > S.M) return;
-  margin_u(S, (double)c.NANGDAY, j);
+  const SegHit h = seg_hit(S.dauj + col * SEG, S.cuoij + col * SEG, S.mocj[col], row);
+  if (h.what == 1) {
+    S.tu[ij] = u_new(o, S, c, ij);
+  } else if (h.what) {
+    bool br1, br2;
+    ends_u(S, (double)c.NANGDAY, col, h.first, h.last, br1, br2);
+    const int w = S.W;
+    seg_ends<R>(h, br1, br2, [&](int p) { return u_new(u_ops(S, S.sv, p * w + col), S, c, p * w + col); },
+                [&](int p) { return S.tu[p * w + col]; }, [&](int p, R x) { S.tu[p * w + col] = x; });
+  }
 }
 
 // ------------------------------------------------------ fused commits
@@ -769,6 +770,21 @@ __global__ void k_margin_u(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
 // (the sediment launch shape: N after half-step A, N-1 after B), VTH from
 // row and column 2.
 // Returns the speed stored at (i, j) (0 where none is, i or j below 2).
+//
+// The diffusivity min(100, max(5, n / (18 log(12 H / Ks)))), n >= 0. Whether
+// it is the lower bound is decided with a single-precision logarithm where
+// that is clear of its error (the quotient below 5 by more than a thousandth,
+// against 1e-5 for the logarithm of an argument not within a hundredth of 1):
+// the same value, without the FP64 logarithm and division of nearly every
+// cell. (A NaN takes the plain path.)
+template <class R>
+__device__ __forceinline__ R diffusivity(R n, R H, R Ks) {
+  const R q = 12 * H / Ks;
+  const float cz = 18.0f * __logf((float)q);
+  if (cz > 0.2f && cz < 1e30f && n < R(4.99) * R(cz)) return R(5);
+  return fmin(R(100), fmax(R(5), n / (18 * log(q))));
+}
+
 template <class R>
 __device__ __forceinline__ R vth_heso_cell(const StateT<R>& S, const CoefT<R>& c, int i, int j,
                                            int g, R tu, R tv, R tu_up, R tv_left, R Hm,
@@ -784,14 +800,10 @@ __device__ __forceinline__ R vth_heso_cell(const StateT<R>& S, const CoefT<R>& c
     S.VTH[g] = vthv;
   }
   if (Hu > 0) {
-    const R Cz = 18 * log(12 * Hu / c.Ks);
-    const R k = R(5.93) * c.sqrt_g * R(hl + hp) * R(0.25) * fabs(tu) / Cz;
-    S.Kx[g] = fmin(R(100), fmax(R(5), k));
+    S.Kx[g] = diffusivity(R(5.93) * c.sqrt_g * R(hl + hp) * R(0.25) * fabs(tu), Hu, c.Ks);
   }
   if (Hv > 0) {
-    const R Cz = 18 * log(12 * Hv / c.Ks);
-    const R k = R(5.93) * c.sqrt_g * R(hup + hp) * R(0.25) * fabs(tv) / Cz;
-    S.Ky[g] = fmin(R(100), fmax(R(5), k));
+    S.Ky[g] = diffusivity(R(5.93) * c.sqrt_g * R(hup + hp) * R(0.25) * fabs(tv), Hv, c.Ks);
   }
   return vthv;
 }
@@ -1031,8 +1043,10 @@ __global__ void HYD_CELL_BOUNDS k_boundary_b(StateT<R> S_arg, CoefT<R> c_arg, Ba
   boundary_cells<R, 1>(S_arg, c_arg, b_arg, half);
 }
 
+// (the explicit updates bounded: with the segments' end velocities they would
+// take 66 registers in FP64 and 64 in FP32)
 template <class R, int BATCH = 0>
-__global__ void k_solve_v(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 8 : 10) k_solve_v(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
   solve_v_cells<R, BATCH>(S_arg, c_arg, b_arg);
 }
 template <class R>
@@ -1041,7 +1055,7 @@ __global__ void HYD_CELL_BOUNDS k_solve_v_b(StateT<R> S_arg, CoefT<R> c_arg, Bat
 }
 
 template <class R, int BATCH = 0>
-__global__ void k_solve_u(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 8 : 10) k_solve_u(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
   solve_u_cells<R, BATCH>(S_arg, c_arg, b_arg);
 }
 template <class R>
@@ -1127,18 +1141,22 @@ void launch_scan_segments(const StateT<R>& S, const CoefT<R>& c, bool dry, cudaS
 }
 
 template <class R>
+static void launch_interp_fs(const StateT<R>& S, const CoefT<R>& c, cudaStream_t st, const Batch<R>& b) {
+  launch2(HYD_K2(k_interp_fs, R), dim3(3 * cdiv(S.M - 1, 128)), 128, st, S, c, b);
+}
+
+template <class R>
 void launch_find_limits(const StateT<R>& S, const CoefT<R>& c, bool dry, cudaStream_t st,
                         Trace* tr, const Batch<R>& b) {
-  launch2(HYD_K2(k_interp_fs_rows, R), dim3(cdiv(S.M, 128), 2), 128, st, S, c, b);
-  launch2(HYD_K2(k_interp_fs_col, R), dim3(cdiv(S.M, 128)), 128, st, S, c, b);
+  launch_interp_fs(S, c, st, b);
   const int n = scan(S, c, dry ? 1 : 0, !dry, st, b);
-  if (tr) tr->launches += 2 + n;
+  if (tr) tr->launches += 1 + n;
 }
 
 template <class R>
 void launch_half_x(const StateT<R>& S, const CoefT<R>& c, bool sed, cudaStream_t st, Trace* tr,
                    const Batch<R>& b) {
-  const dim3 cells(cdiv(S.M - 1, 128), S.N - 1);
+  const dim3 cells(cdiv(S.M, 128), S.N - 1);
   const dim3 smooth(cdiv(S.W, 128), cdiv(S.H, SMOOTH_ROWS));
   const dim3 commit(cdiv(S.M + 1, 128), S.N + 1);
   launch2(HYD_K2B(k_boundary, R), dim3(cdiv(max(S.M, S.N), 128)), 128, st, S, c, b, 0.5 * (double)c.dT);
@@ -1147,12 +1165,11 @@ void launch_half_x(const StateT<R>& S, const CoefT<R>& c, bool sed, cudaStream_t
   const int nx = launch_sweep(S, c, 0, st, b);
   if (tr) tr->kend(st, KS_SWEEP_X);
   if (tr) tr->mark(st, PH_SWEEP_X, nx);
-  // smoothing of t_u into su, explicit v from it, margins, smoothing of t_v
+  // smoothing of t_u into su, explicit v from it with its margins, smoothing of t_v
   // into sv; k_commit_a writes both back (Normalize/update_buffer pairs,
   // engine.cpp:109-124)
   launch2(HYD_K2(k_smooth_full, R, 1, 0), smooth, 128, st, S, c, b);
   launch2(HYD_K2B(k_solve_v, R), cells, 128, st, S, c, b);
-  launch2(HYD_K2(k_margin_v, R), dim3(cdiv(S.N - 1, 128)), 128, st, S, c, b);
   if (S.reset_h) {
     // wetting and drying along rows (Reset_states_horizontal after
     // update_h_moi): the smoothing of t_v also does update_h_moi and flags
@@ -1160,25 +1177,23 @@ void launch_half_x(const StateT<R>& S, const CoefT<R>& c, bool sed, cudaStream_t
     // drying per cell in the commit, the mask is written by the segment
     // scan (the mask can change, so the tables are rescanned)
     launch2(HYD_K2(k_smooth_full, R, 0, 2), smooth, 128, st, S, c, b);
-    if (tr) tr->mark(st, PH_EXPLICIT_V, 4);
+    if (tr) tr->mark(st, PH_EXPLICIT_V, 3);
     launch2(HYD_K2(k_wetting_rows, R), dim3(cdiv(S.N, 128)), 128, st, S, c, b);
     launch2(HYD_K2B(k_commit_b, R, 1), commit, 128, st, S, c, b, sed ? S.N : 0, 0);
-    launch2(HYD_K2(k_interp_fs_rows, R), dim3(cdiv(S.M, 128), 2), 128, st, S, c, b);
-    launch2(HYD_K2(k_interp_fs_col, R), dim3(cdiv(S.M, 128)), 128, st, S, c, b);
+    launch_interp_fs(S, c, st, b);
     const int n = scan(S, c, 2, false, st, b);
-    if (tr) tr->mark(st, PH_COMMIT_X, 4 + n);
+    if (tr) tr->mark(st, PH_COMMIT_X, 3 + n);
     return;
   }
   launch2(HYD_K2(k_smooth_full, R, 0, 0), smooth, 128, st, S, c, b);
-  if (tr) tr->mark(st, PH_EXPLICIT_V, 4);
+  if (tr) tr->mark(st, PH_EXPLICIT_V, 3);
   // update_h_moi + update_uvz + Htuongdoi; the wet/dry mask does not change
   // in this half-step, so the segment tables are not rescanned, only the
   // boundary concentration is interpolated (support_funcs.cpp:255-258, 311)
   // with sed, also Find_VTH + hesoK of the concentration step (rows to N)
   launch2(HYD_K2B(k_commit_a, R), commit, 128, st, S, c, b, sed ? S.N : 0);
-  launch2(HYD_K2(k_interp_fs_rows, R), dim3(cdiv(S.M, 128), 2), 128, st, S, c, b);
-  launch2(HYD_K2(k_interp_fs_col, R), dim3(cdiv(S.M, 128)), 128, st, S, c, b);
-  if (tr) tr->mark(st, PH_COMMIT_X, 3);
+  launch_interp_fs(S, c, st, b);
+  if (tr) tr->mark(st, PH_COMMIT_X, 2);
 }
 
 template <class R>
@@ -1194,10 +1209,9 @@ void launch_half_y(const StateT<R>& S, const CoefT<R>& c, bool sed, cudaStream_t
   if (tr) tr->mark(st, PH_SWEEP_Y, ny);
   launch2(HYD_K2(k_smooth_full, R, 0, 0), smooth, 128, st, S, c, b);
   launch2(HYD_K2B(k_solve_u, R), dim3(cdiv(S.M - 1, 128), S.N), 128, st, S, c, b);
-  launch2(HYD_K2(k_margin_u, R), dim3(cdiv(S.M - 1, 128)), 128, st, S, c, b);
   // with update_h_moi and the wetting pass's column flags
   launch2(HYD_K2(k_smooth_full, R, 1, 1), smooth, 128, st, S, c, b);
-  if (tr) tr->mark(st, PH_EXPLICIT_U, 4);
+  if (tr) tr->mark(st, PH_EXPLICIT_U, 3);
   // update_h_moi, Reset_states_vertical (wetting on flagged columns, drying
   // per cell), update_uvz, Htuongdoi, then the segment tables
   launch2(HYD_K2(k_wetting, R), dim3(cdiv(S.M, 128)), 128, st, S, c, b);

@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(1024) solveV(double t, int startidx, int endid
   const State S = state_of(arg);
   const Coef c = coef_of(coeffs);
   const int g = i * S.W + j;
-  arg->t_v[g] = hyd::v_new(hyd::v_ops(S, static_cast<const double*>(arg->t_u), g), c);
+  arg->t_v[g] = hyd::v_new(hyd::v_ops(S, static_cast<const double*>(arg->t_u), g), S, c, g);
 }
 
 // update_margin_elem_V (UVZSolver_multithread.cpp:1018-1060): row
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(1024) solveU(double t, int startidx, int endid
   const State S = state_of(arg);
   const Coef c = coef_of(coeffs);
   const int ij = i * S.W + j;
-  arg->t_u[ij] = hyd::u_new(hyd::u_ops(S, static_cast<const double*>(arg->t_v), ij), c);
+  arg->t_u[ij] = hyd::u_new(hyd::u_ops(S, static_cast<const double*>(arg->t_v), ij), S, c, ij);
 }
 
 // update_margin_elem_U (UVZSolver_multithread.cpp:980-1016): column
