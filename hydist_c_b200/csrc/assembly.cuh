@@ -25,9 +25,11 @@ using Pre = PreT<double>;
 
 // The momentum part of the preindex step: f1 u_{-} + f2 u + f3 u_{+} +
 // f4 (z - z_{+}) = f5 along the line, before the continuity rows enter it.
+// g2, g5: f2 and f5 without the time derivative's terms, f2 = -(2 + g2),
+// f5 = -2 u + g5.
 template <class R>
 struct MomF {
-  R f1, f2, f3, f5;
+  R f1, f2, f3, f5, g2, g5;
 };
 
 // _uzSolver_calculate_preindex (UVZSolver_multithread.cpp:210-278): the
@@ -51,7 +53,9 @@ __device__ __forceinline__ MomF<R> mom_x(const StateT<R>& S, const CoefT<R>& c, 
   const R rH = R(1) / Hu;
   const R visc = VI * c.dT_dXbp;
   P.f1 = c.dTchia2dX * uu + visc;
-  P.f2 = -(2 + S.Kx1[g] * dT * sqrt(uu * uu + vtb * vtb) * rH + 2 * visc);
+  const R fr = S.Kx1[g] * dT * sqrt(uu * uu + vtb * vtb) * rH;
+  P.f2 = -(2 + fr + 2 * visc);
+  P.g2 = fr + 2 * visc;
   P.f3 = visc - c.dTchia2dX * uu;
   if (hm1 <= c.H_TINH) {
     if (vtb < 0) {
@@ -71,6 +75,7 @@ __device__ __forceinline__ MomF<R> mom_x(const StateT<R>& S, const CoefT<R>& c, 
   }
   P.f5 = -2 * uu + dT * p - dT * c.CORIOLIS_FORCE * vtb - dT * VI * q -
          dT * (c.Windx - S.Tsxw[g]) * rH;
+  P.g5 = dT * p - dT * c.CORIOLIS_FORCE * vtb - dT * VI * q - dT * (c.Windx - S.Tsxw[g]) * rH;
   return P;
 }
 
@@ -109,7 +114,9 @@ __device__ __forceinline__ MomF<R> mom_y(const StateT<R>& S, const CoefT<R>& c, 
   const R rH = R(1) / Hv;
   const R visc = VI * c.dT_dYbp;
   P.f1 = c.dTchia2dY * vv + visc;
-  P.f2 = -(2 + S.Ky1[g] * dT * sqrt(vv * vv + utb * utb) * rH + 2 * visc);
+  const R fr = S.Ky1[g] * dT * sqrt(vv * vv + utb * utb) * rH;
+  P.f2 = -(2 + fr + 2 * visc);
+  P.g2 = fr + 2 * visc;
   P.f3 = visc - c.dTchia2dY * vv;
   if (hm1 <= c.H_TINH) {
     if (utb < 0) {
@@ -129,6 +136,7 @@ __device__ __forceinline__ MomF<R> mom_y(const StateT<R>& S, const CoefT<R>& c, 
   }
   P.f5 = -2 * vv + dT * q + dT * c.CORIOLIS_FORCE * utb - dT * VI * p -
          dT * (c.Windy - S.Tsyw[g]) * rH;
+  P.g5 = dT * q + dT * c.CORIOLIS_FORCE * utb - dT * VI * p - dT * (c.Windy - S.Tsyw[g]) * rH;
   return P;
 }
 

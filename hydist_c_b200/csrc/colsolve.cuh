@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT < 1 ? 1 : (sizeof(typename Gen::
     R* rA = reinterpret_cast<R*>(smem_raw);
     R* rC = rA + nc * L;
     R* rD = rC + nc * L;
-    R* rB = rD + nc * L;  // (REFINE)
+    R* rB = rD + nc * L;  // (where the rows are not normalised)
     typename Gen::Ops o;
     if (act && r0 < nc) o = G.load(lp, r0 + 2);
     for (int e = tid; e < L * (SEG + 1); e += NT)
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT < 1 ? 1 : (sizeof(typename Gen::
       if (w.at(LS, pos)) {
         G.row(w.d, lp, pos, o, A, B, C, D);
         G.keep(w.d, lp, pos, o);
-        if constexpr (!Gen::REFINE) {
+        if constexpr (row_normal<Gen>()) {
           const R m = R(1) / B;
           A *= m;
           C *= m;
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT < 1 ? 1 : (sizeof(typename Gen::
       rA[q] = A;
       rC[q] = C;
       rD[q] = D;
-      if constexpr (Gen::REFINE) rB[q] = B;
+      if constexpr (!row_normal<Gen>()) rB[q] = B;
       r += NT / L;
       if (act && r < nc) o = G.load(lp, r + 2);
     }
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT < 1 ? 1 : (sizeof(typename Gen::
     if constexpr (!Gen::REFINE) {
       cols_solve<R, NT, L>(rA, rC, rD, nc, sh, [&](int q, R& A, R& B, R& C, R& D) {
         A = rA[q];
-        B = 1;
+        B = row_normal<Gen>() ? R(1) : rB[q];
         C = rC[q];
         D = rD[q];
       });

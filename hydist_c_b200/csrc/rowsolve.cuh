@@ -10,8 +10,8 @@
 // (distinct banks) and reduced by shuffles with one barrier (cta_solve), and
 // the solution and the segments' ends are emitted with neighbouring threads
 // on neighbouring cells. What bounds it is the latency of a row's rounds of
-// loads times the rounds of CTAs: the rows are kept normalised (three arrays)
-// so that seven FP64 rows of 1023 cells share an SM and 2047 of them take two
+// loads times the rounds of CTAs: the FP64 rows are kept normalised (three
+// arrays) so that seven of 1023 cells share an SM and 2047 of them take two
 // rounds (four arrays, six rows, three rounds: 0.107 ms, hydraulic). The solve
 // itself is a tenth of the time, the rounds of loads half (ablation). On
 // 2048x1024, from the chunks in global memory: hydraulic y sweep 0.148 ->
@@ -31,11 +31,20 @@
 
 namespace hyd {
 
-// arrays of a row's cells in shared memory: a = A/B, c = C/B, d = D/B; with
-// refinement A, B, C, D, v', c' and the first solution
+// Rows normalised to a unit diagonal (a = A/B, c = C/B, d = D/B: one array
+// less) in FP64. In FP32 their rounding would add to the result's error (the
+// concentration's 2.0e-7 -> 2.5e-7 against 64 bits after ten steps), and the
+// fourth array costs no resident CTA.
+template <class Gen>
+constexpr bool row_normal() {
+  return sizeof(typename Gen::Real) == 8;
+}
+
+// arrays of a row's cells in shared memory: a, c, d or A, C, D, B; with
+// refinement also v', c' and the first solution
 template <class Gen>
 constexpr int row_arrays() {
-  return Gen::REFINE ? 7 : 3;
+  return Gen::REFINE ? 7 : (row_normal<Gen>() ? 3 : 4);
 }
 
 template <class Gen>
@@ -94,7 +103,7 @@ __global__ void __launch_bounds__(NT, row_min_blocks<typename Gen::Real, NT>())
     R* rA = reinterpret_cast<R*>(smem_raw);
     R* rC = rA + nc;
     R* rD = rC + nc;
-    R* rB = rD + nc;  // (REFINE)
+    R* rB = rD + nc;  // (where the rows are not normalised)
     // the row's own new field rows towards L2 at once, so that the rounds of
     // loads after the first find them there (0.115 -> 0.107 ms, hydraulic)
     if (tid == 0) G.prefetch(lp);
@@ -110,7 +119,7 @@ __global__ void __launch_bounds__(NT, row_min_blocks<typename Gen::Real, NT>())
       if (w.at(LS, pos)) {
         G.row(w.d, lp, pos, o, A, B, C, D);
         G.keep(w.d, lp, pos, o);
-        if constexpr (!Gen::REFINE) {
+        if constexpr (row_normal<Gen>()) {
           const R m = R(1) / B;
           A *= m;
           C *= m;
@@ -120,7 +129,7 @@ __global__ void __launch_bounds__(NT, row_min_blocks<typename Gen::Real, NT>())
       rA[c] = A;
       rC[c] = C;
       rD[c] = D;
-      if constexpr (Gen::REFINE) rB[c] = B;
+      if constexpr (!row_normal<Gen>()) rB[c] = B;
       c += NT;
       if (c < nc) o = G.load(lp, c + 2);
     }
@@ -129,7 +138,7 @@ __global__ void __launch_bounds__(NT, row_min_blocks<typename Gen::Real, NT>())
     if constexpr (!Gen::REFINE) {
       cta_solve<R, NT>(rA, rC, rD, nc, blk, [&](int q, R& A, R& B, R& C, R& D) {
         A = rA[q];
-        B = 1;
+        B = row_normal<Gen>() ? R(1) : rB[q];
         C = rC[q];
         D = rD[q];
       });
