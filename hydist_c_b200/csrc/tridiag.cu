@@ -10,9 +10,9 @@
 //
 // Four solvers, chosen per length band:
 //   Thomas      one thread per system, in place in global memory (any length);
-//   warp        one warp per system staged in shared memory, partition
-//               method with a shuffle PCR of the 32 chunk separators
-//               (systems up to GT_WARP_MAX rows);
+//   warp        one warp (two beyond 256 rows) per system staged in shared
+//               memory, partition method with a shuffle PCR of the 32 chunk
+//               separators (systems up to GT_WARP_MAX rows);
 //   CTA         one CTA of 128, 256 or 512 threads per system, its rows staged
 //               in shared memory by TMA bulk copies (the next system's while
 //               one is solved, where two fit), partition method over chunks,
@@ -63,24 +63,27 @@ __host__ __device__ inline int gt_band_hi(int b) {
 
 // Length classes of the lists: the bands, those above 512 rows split where
 // the systems' rows in shared memory set how many CTAs an SM holds (three of
-// 2048 FP64 rows, six of 1024).
-constexpr int GT_NC = 10;
+// 2048 FP64 rows, six of 1024), the warp solver's at 256 for the same reason.
+constexpr int GT_NC = 11;
 __host__ __device__ inline int gt_class_hi(int k) {
   switch (k) {
     case 0: return 32;
     case 1: return 128;
-    case 2: return 512;
-    case 3: return 1024;
-    case 4: return 1536;
-    case 5: return 2048;
-    case 6: return 3072;
-    case 7: return 4096;
-    case 8: return 6144;
+    case 2: return 256;
+    case 3: return 512;
+    case 4: return 1024;
+    case 5: return 1536;
+    case 6: return 2048;
+    case 7: return 3072;
+    case 8: return 4096;
+    case 9: return 6144;
     default: return INT_MAX;
   }
 }
 // the band of class k
-inline int gt_class_band(int k) { return k < 3 ? k : (k < 6 ? 3 : (k < 8 ? 4 : k - 3)); }
+inline int gt_class_band(int k) {
+  return k < 2 ? k : (k < 4 ? 2 : (k < 7 ? 3 : (k < 9 ? 4 : k - 4)));
+}
 // what the classification counts: systems per class, the packed extent, a
 // negative offset seen, tiles of the open class; then a flag that stays set
 // until read (a CTA gave its systems up)
@@ -399,7 +402,7 @@ __device__ __forceinline__ void stage_ends(const T* const src[4], T* buf, int re
 // Systems of one class, a CTA of NT threads each (about 9 to 17 rows a
 // thread). Bound by the chunks' dependent chains and the rows resident in
 // shared memory. 16384 systems of 16..4096 rows (12 M) on a B200: FP64 434 ->
-// 193 us a batch (2.5 of the 6.6 TB/s at 40 B a row), FP32 280 -> 116 us,
+// 178 us a batch (2.7 of the 6.6 TB/s at 40 B a row), FP32 280 -> 114 us,
 // against a reduction over the CTA in shared memory on 512 threads.
 template <class T, int NT, int NBUF>
 __global__ void __launch_bounds__(NT) k_gtsv_bulk(const T* __restrict__ dl, const T* __restrict__ d,
@@ -812,8 +815,10 @@ int cta_max_rows(const DevInfo& D) {
 }
 
 // the tile solver of the open band (not a public algo: what the shared-memory
-// solvers become for systems that fit no CTA)
+// solvers become for systems that fit no CTA), and the warp solver on rows
+// staged by bulk copies
 constexpr int GTSV_TILES = 100;
+constexpr int GTSV_WARP_BULK = 101;
 
 struct Caps {
   int cta128, cta256, cta512;  // longest systems of the three CTA tiles
@@ -972,6 +977,10 @@ int launch_class(int algo, int cls, const T* dl, const T* d, const T* du, const 
     rc = launch_cta<T, 512>(hi, dl, d, du, b, x, off, len, list, count, stalled, nsys_band, D, st);
   } else if (algo == HYDIST_GTSV_WARP) {
     rc = launch_warp<T>(cls, cls, dl, d, du, b, x, off, len, nsys_band, D, st);
+  } else if (algo == GTSV_WARP_BULK && hi <= 256) {
+    rc = launch_cta<T, 32>(hi, dl, d, du, b, x, off, len, list, count, stalled, nsys_band, D, st);
+  } else if (algo == GTSV_WARP_BULK) {
+    rc = launch_cta<T, 64>(hi, dl, d, du, b, x, off, len, list, count, stalled, nsys_band, D, st);
   } else if (algo == GTSV_TILES) {
     rc = launch_tiles<T>(dl, d, du, b, x, off, len, list, count, nsys_band, D.scr.host[hyd::GT_TILES],
                          stalled, D, st);
@@ -1044,7 +1053,7 @@ bool band_streams(DevInfo& D) {
 
 bool staged_algo(int a) {
   return a == HYDIST_GTSV_PARTITION || a == HYDIST_GTSV_PARTITION_512 || a == HYDIST_GTSV_PARTITION_128 ||
-         a == GTSV_TILES;
+         a == GTSV_TILES || a == GTSV_WARP_BULK;
 }
 
 // one batched solve with a given solver per band (table[b])
@@ -1075,7 +1084,6 @@ int solve_batch(const T* dl, const T* d, const T* du, const T* b, T* x, const in
     ++nonempty;
     thomas |= tab[k] == HYDIST_GTSV_THOMAS;
     pivot |= tab[k] == HYDIST_GTSV_PIVOT;
-    staged |= staged_algo(tab[k]);
     if (tab[k] == HYDIST_GTSV_WARP) {
       top_warp = k;
       short_sys += counts[k];
@@ -1094,6 +1102,20 @@ int solve_batch(const T* dl, const T* d, const T* du, const T* b, T* x, const in
   for (int k = 0; k < top_warp; ++k) merge = merge && (counts[k] == 0 || tab[k] == HYDIST_GTSV_WARP);
   if (merge)
     for (int k = 0; k < top_warp; ++k) nonempty -= counts[k] > 0 && tab[k] == HYDIST_GTSV_WARP;
+  // Otherwise systems of more than 32 rows are staged by bulk copies, a warp
+  // each (two beyond 256 rows), where the warps' own 8-byte copies
+  // (k_gtsv_warp) keep the load units busy: 16384 systems on a B200, a call on
+  // a cold cache, FP64 / FP32: 257..512 rows 164 -> 92 us / 106 -> 74, 129..256
+  // 94 -> 76 / 71 -> 57, 33..128 58 -> 51 / 52 -> 51; up to 32 rows the copies
+  // are too short (46 / 43 against 50 / 49). Their stall flag costs a batch
+  // without longer systems 10 to 14 us more, so there only many systems of
+  // more than 256 rows pay (2048 in FP64: 66 -> 64 us, 51 -> 57 in FP32; 16384
+  // in FP32: 105 -> 86). Misaligned arrays keep the warps' own copies.
+  bool bulk = counts[3] >= (sizeof(T) == 8 ? 2048 : 8192);
+  for (int k = 4; k < GT_NC; ++k) bulk |= counts[k] > 0 && staged_algo(tab[k]);
+  for (int k = 1; k <= top_warp && bulk && aligned && !merge; ++k)
+    if (tab[k] == HYDIST_GTSV_WARP) tab[k] = GTSV_WARP_BULK;
+  for (int k = 0; k < GT_NC; ++k) staged |= counts[k] > 0 && staged_algo(tab[k]);
   // the classes' solves are independent (disjoint systems, per-class lists,
   // per-system scratch): each on its own stream, so that the short classes'
   // launches and the long classes' tails overlap; the longest first

@@ -59,3 +59,33 @@ def test_batches_on_two_streams_share_the_scratch(hyd, oracle_mod):
     torch.cuda.synchronize()
     for x, w in zip(xs, work):
         assert np.abs(x.cpu().numpy() - w[3]).max() <= 1e-13 * max(1.0, np.abs(w[3]).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_many_short_systems_beside_a_long_one(hyd, oracle_mod, dtype, shift):
+    """Short systems staged by bulk copies (more of them than one wave of
+    warps, and a longer system in the batch), at the classes' edges, from
+    offsets of every alignment; with arrays that are not 16-byte aligned the
+    warps' own copies. Rows around the systems stay as they were."""
+    import torch
+    from hydist_c_b200 import scenario as S
+    edges = [1, 2, 3, 31, 32, 33, 34, 65, 95, 127, 128, 129, 191, 255, 256, 257, 320, 511, 512]
+    a, d, c, b, off, ln = S.tridiag_batch(lengths=np.array(edges * 40 + [600]), seed=77)
+    ref = oracle_mod.thomas_batched(a, d, c, b, off, ln)
+    dt = getattr(torch, dtype)
+
+    def place(v):
+        t = torch.full((len(v) + 2,), float("nan"), dtype=dt, device="cuda")
+        t[shift:shift + len(v)] = torch.from_numpy(v).to(dt).cuda()
+        return t[shift:shift + len(v)]
+
+    t = [place(v) for v in (a, d, c, b)]
+    full = torch.full((len(b) + 8,), float("nan"), dtype=dt, device="cuda")
+    x = full[4:4 + len(b)]
+    hyd.gtsv_batched(*t, torch.from_numpy(off), torch.from_numpy(ln), x=x)
+    torch.cuda.synchronize()
+    assert torch.isnan(full[:4]).all() and torch.isnan(full[-4:]).all()
+    err = np.abs(x.double().cpu().numpy() - ref) / np.maximum(np.abs(ref), 1.0)
+    assert np.isfinite(err).all() and err.max() <= (1e-14 if dtype == "float64" else 5e-6), err.max()
