@@ -142,6 +142,7 @@ __device__ __forceinline__ void cols_solve(T* oV, T* oC, T* X, int n, ColShared<
 template <class Gen, int NT, int L, int BATCH>
 __global__ void __launch_bounds__(NT, 1024 / NT < 1 ? 1 : (sizeof(typename Gen::Real) == 8 && NT < 1024 ? 768 : 1024) / NT)
     k_col_solve(Gen G0, Batch<typename Gen::Real> bt) {
+  step_begin<BATCH>();
   using R = typename Gen::Real;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LineSeg seg[L];
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT < 1 ? 1 : (sizeof(typename Gen::
     for (int pos = r0 + 2; pos < nc + 2; pos += NT / L)
       if (e.at(LS, pos)) G.emit_cell(e.d, lp, pos, value);
   };
-  if constexpr (BATCH != 0) {
+  if constexpr ((BATCH & 1) != 0) {
     Gen Gm = G0;
     Gm.bind(bt.S[blockIdx.y], bt.c[blockIdx.y]);
     solve(Gm);

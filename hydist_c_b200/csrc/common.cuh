@@ -134,12 +134,12 @@ struct Batch {
 // with BATCH those of member blockIdx.z.
 template <int BATCH, class R>
 __device__ __forceinline__ StateT<R> member_state(const StateT<R>& S0, const Batch<R>& b) {
-  if constexpr (BATCH != 0) return b.S[blockIdx.z];
+  if constexpr ((BATCH & 1) != 0) return b.S[blockIdx.z];
   else return S0;
 }
 template <int BATCH, class R>
 __device__ __forceinline__ CoefT<R> member_coef(const CoefT<R>& c0, const Batch<R>& b) {
-  if constexpr (BATCH != 0) return b.c[blockIdx.z];
+  if constexpr ((BATCH & 1) != 0) return b.c[blockIdx.z];
   else return c0;
 }
 
@@ -196,5 +196,67 @@ struct Trace {
     }
   }
 };
+
+// The kernels of a small mesh's step start while the one before them still
+// runs (programmatic dependent launch; BATCH & 2): step_begin, first in each of
+// them, waits for all of the previous kernel's results and then lets the next
+// one start once every block of this one has come so far, so that a launch's
+// latency falls into the tail of the kernel before. A step on a B200, without
+// -> with: 64x32 49.2 -> 47.1 us, 256x128 63.7 -> 59.4, 464x324 with sediment
+// 129 -> 127, 24 members of 256x128 in FP32 306 -> 298; 2048x1024 706 -> 715
+// and 8 members of 1024x512 1583 -> 1625 (the waiting blocks take places in
+// which the kernel's own would have been spread), so only up to
+// DEPENDENT_CELLS cells in all, by kernels of their own: the two instructions,
+// or a branch around them, cost the large meshes 9 us too. (Letting the next
+// one start before the wait: 53.3, 63.5 and 138 us.)
+constexpr size_t DEPENDENT_CELLS = (size_t)1 << 20;
+template <class R>
+inline bool dependent_launches(const StateT<R>& S, const Batch<R>& b) {
+  return (size_t)S.M * S.N * (b.n > 0 ? b.n : 1) <= DEPENDENT_CELLS;
+}
+template <int BATCH>
+__device__ __forceinline__ void step_begin() {
+  if constexpr ((BATCH & 2) != 0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
+}
+// launches a kernel whose BATCH & 2 is set
+template <class... P, class... A>
+inline void launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
+                             cudaStream_t st, const A&... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(a)...);
+}
+
+// One scenario's kernel (ks; where launches are dependent ksd) or every
+// member's of a batch (kb, kbd; grid z = members).
+template <class R, class KS, class KB, class KSD, class KBD, class... A>
+inline void launch2(KS ks, KB kb, KSD ksd, KBD kbd, dim3 g, int bs, cudaStream_t st,
+                    const StateT<R>& S, const CoefT<R>& c, const Batch<R>& b, A... a) {
+  const bool dep = dependent_launches(S, b);
+  if (b.n > 0) {
+    g.z = (unsigned)b.n;
+    if (dep) launch_dependent(kbd, g, bs, 0, st, S, c, b, a...);
+    else kb<<<g, bs, 0, st>>>(S, c, b, a...);
+  } else {
+    if (dep) launch_dependent(ksd, g, bs, 0, st, S, c, b, a...);
+    else ks<<<g, bs, 0, st>>>(S, c, b, a...);
+  }
+}
+#define HYD_K2(name, ...) \
+  name<__VA_ARGS__, 0>, name<__VA_ARGS__, 1>, name<__VA_ARGS__, 2>, name<__VA_ARGS__, 3>
+// the same for the passes with separate batch entry points (name_b)
+#define HYD_K2B(name, ...) \
+  name<__VA_ARGS__, 0>, name##_b<__VA_ARGS__, 1>, name<__VA_ARGS__, 2>, name##_b<__VA_ARGS__, 3>
 
 }  // namespace hyd

@@ -119,6 +119,7 @@ __device__ __forceinline__ void interp_fs_col(const StateT<R>& S, const CoefT<R>
 
 template <class R, int BATCH = 0>
 __global__ void __launch_bounds__(128) k_interp_fs(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  step_begin<BATCH>();
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
   const int rows = min(S.M, S.H);  // column M: rows 1 .. rows - 1
@@ -181,6 +182,7 @@ __device__ __forceinline__ bool scan_needed(const StateT<R>& S, int always) {
 
 template <class R, int BATCH = 0>
 __global__ void k_runs_flags(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int dry, int always) {
+  step_begin<BATCH>();
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
   if (!scan_needed(S, always)) return;
@@ -270,6 +272,7 @@ __device__ __forceinline__ void sort_small(int* a, int n) {
 // counters for the next scan.
 template <class R, int BATCH = 0>
 __global__ void k_runs_sort(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int always) {
+  step_begin<BATCH>();
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   if (!scan_needed(S, always)) return;
   int* seg_cnt = S.segcnt;
@@ -314,6 +317,7 @@ constexpr int SCAN_MAX = 32 * SCAN_WORDS;  // positions 2..lim of a line
 
 template <class R, int BATCH = 0>
 __global__ void k_runs_lines(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int dry, int always) {
+  step_begin<BATCH>();
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
   if (!scan_needed(S, always)) return;
@@ -617,8 +621,9 @@ constexpr int SMOOTH_ROWS = 4;
 // are template parameters: each launch compiles to its own variant.
 // (ten CTAs per SM, eight for a batch: 3 us less per FP32 step on 2048x1024)
 template <class R, int isU, int hmoi, int BATCH = 0>
-__global__ void __launch_bounds__(128, BATCH ? 8 : 10)
+__global__ void __launch_bounds__(128, (BATCH & 1) ? 8 : 10)
     k_smooth_full(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  step_begin<BATCH>();
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
   constexpr int RB = SMOOTH_ROWS;
@@ -866,6 +871,7 @@ __device__ __forceinline__ void commit_a_cells(StateT<R> S_arg, CoefT<R> c_arg, 
 // sequential along i, on flagged columns only.
 template <class R, int BATCH = 0>
 __global__ void k_wetting(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  step_begin<BATCH>();
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
   int* colflag = S.colflag;
@@ -900,6 +906,7 @@ __global__ void k_wetting(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
 // sequential along j, on flagged rows 1..N only.
 template <class R, int BATCH = 0>
 __global__ void k_wetting_rows(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  step_begin<BATCH>();
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
   int* rowflag = S.rowflag;
@@ -1028,48 +1035,54 @@ __device__ __forceinline__ void commit_b_cells(StateT<R> S_arg, CoefT<R> c_arg, 
 // ------------------------------------------------------------- launchers
 static inline dim3 grid2(int nx, int ny, int bx) { return dim3(cdiv(nx, bx), ny); }
 
-// Launches a step kernel for one scenario (ks, b.n == 0) or for every
-// member of a batch (kb, grid z = members).
 // Entry points of the passes above: the single-scenario kernels unbounded,
 // the batch ones (suffix _b) under HYD_CELL_BOUNDS. A bound changes ptxas's
 // register choice even where it does not bind, so the two are separate
 // kernels.
 template <class R, int BATCH = 0>
 __global__ void k_boundary(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, double half) {
+  step_begin<BATCH>();
   boundary_cells<R, BATCH>(S_arg, c_arg, b_arg, half);
 }
-template <class R>
+template <class R, int BATCH = 1>
 __global__ void HYD_CELL_BOUNDS k_boundary_b(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, double half) {
-  boundary_cells<R, 1>(S_arg, c_arg, b_arg, half);
+  step_begin<BATCH>();
+  boundary_cells<R, BATCH>(S_arg, c_arg, b_arg, half);
 }
 
 // (the explicit updates bounded: with the segments' end velocities they would
 // take 66 registers in FP64 and 64 in FP32)
 template <class R, int BATCH = 0>
 __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 8 : 10) k_solve_v(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  step_begin<BATCH>();
   solve_v_cells<R, BATCH>(S_arg, c_arg, b_arg);
 }
-template <class R>
+template <class R, int BATCH = 1>
 __global__ void HYD_CELL_BOUNDS k_solve_v_b(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
-  solve_v_cells<R, 1>(S_arg, c_arg, b_arg);
+  step_begin<BATCH>();
+  solve_v_cells<R, BATCH>(S_arg, c_arg, b_arg);
 }
 
 template <class R, int BATCH = 0>
 __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 8 : 10) k_solve_u(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  step_begin<BATCH>();
   solve_u_cells<R, BATCH>(S_arg, c_arg, b_arg);
 }
-template <class R>
+template <class R, int BATCH = 1>
 __global__ void HYD_CELL_BOUNDS k_solve_u_b(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
-  solve_u_cells<R, 1>(S_arg, c_arg, b_arg);
+  step_begin<BATCH>();
+  solve_u_cells<R, BATCH>(S_arg, c_arg, b_arg);
 }
 
 template <class R, int BATCH = 0>
 __global__ void k_commit_a(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int vth_hi) {
+  step_begin<BATCH>();
   commit_a_cells<R, BATCH>(S_arg, c_arg, b_arg, vth_hi);
 }
-template <class R>
+template <class R, int BATCH = 1>
 __global__ void HYD_CELL_BOUNDS k_commit_a_b(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int vth_hi) {
-  commit_a_cells<R, 1>(S_arg, c_arg, b_arg, vth_hi);
+  step_begin<BATCH>();
+  commit_a_cells<R, BATCH>(S_arg, c_arg, b_arg, vth_hi);
 }
 
 // (the single-scenario second commit under the bound too: 66 -> 64 registers
@@ -1078,26 +1091,14 @@ __global__ void HYD_CELL_BOUNDS k_commit_a_b(StateT<R> S_arg, CoefT<R> c_arg, Ba
 template <class R, int HORIZ, int BATCH = 0>
 __global__ void HYD_CELL_BOUNDS k_commit_b(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int vth_hi,
                                            int qb) {
+  step_begin<BATCH>();
   commit_b_cells<R, HORIZ, BATCH>(S_arg, c_arg, b_arg, vth_hi, qb);
 }
-template <class R, int HORIZ>
+template <class R, int HORIZ, int BATCH = 1>
 __global__ void HYD_CELL_BOUNDS k_commit_b_b(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg, int vth_hi, int qb) {
-  commit_b_cells<R, HORIZ, 1>(S_arg, c_arg, b_arg, vth_hi, qb);
+  step_begin<BATCH>();
+  commit_b_cells<R, HORIZ, BATCH>(S_arg, c_arg, b_arg, vth_hi, qb);
 }
-
-template <class R, class KS, class KB, class... A>
-static void launch2(KS ks, KB kb, dim3 g, int bs, cudaStream_t st, const StateT<R>& S,
-                    const CoefT<R>& c, const Batch<R>& b, A... a) {
-  if (b.n > 0) {
-    g.z = (unsigned)b.n;
-    kb<<<g, bs, 0, st>>>(S, c, b, a...);
-  } else {
-    ks<<<g, bs, 0, st>>>(S, c, b, a...);
-  }
-}
-#define HYD_K2(name, ...) name<__VA_ARGS__, 0>, name<__VA_ARGS__, 1>
-// the same for the passes with separate batch entry points (name_b)
-#define HYD_K2B(name, ...) name<__VA_ARGS__, 0>, name##_b<__VA_ARGS__>
 
 template <class R>
 void launch_init(const StateT<R>& S, const CoefT<R>& c, cudaStream_t st) {

@@ -94,6 +94,7 @@ struct SegWalk {
 template <class Gen, int NT, int BATCH>
 __global__ void __launch_bounds__(NT, row_min_blocks<typename Gen::Real, NT>())
     k_row_solve(Gen G0, Batch<typename Gen::Real> bt) {
+  step_begin<BATCH>();
   using R = typename Gen::Real;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LineSeg LS;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(NT, row_min_blocks<typename Gen::Real, NT>())
     for (int pos = tid + 2; pos < nc + 2; pos += NT)
       if (e.at(LS, pos)) G.emit_cell(e.d, lp, pos, value);
   };
-  if constexpr (BATCH != 0) {
+  if constexpr ((BATCH & 1) != 0) {
     Gen Gm = G0;
     Gm.bind(bt.S[blockIdx.y], bt.c[blockIdx.y]);
     solve(Gm);

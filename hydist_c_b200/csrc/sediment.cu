@@ -197,6 +197,7 @@ constexpr int FS_ROWS = 8;
 
 template <class R, int BATCH = 0>
 __global__ void k_update_fs(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  step_begin<BATCH>();
   const StateT<R> S = member_state<BATCH>(S_arg, b_arg);
   const CoefT<R> c = member_coef<BATCH>(c_arg, b_arg);
   // FS = tFS on rows 1..N, columns 1..M; FS_ROWS rows per thread, every
@@ -227,11 +228,13 @@ __global__ void k_update_fs(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
 template <class R, int BATCH = 0>
 __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 7 : 10)
     k_bed_load(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
+  step_begin<BATCH>();
   bed_load_cells<R, BATCH>(S_arg, c_arg, b_arg);
 }
-template <class R>
+template <class R, int BATCH = 1>
 __global__ void HYD_CELL_BOUNDS k_bed_load_b(StateT<R> S_arg, CoefT<R> c_arg, Batch<R> b_arg) {
-  bed_load_cells<R, 1>(S_arg, c_arg, b_arg);
+  step_begin<BATCH>();
+  bed_load_cells<R, BATCH>(S_arg, c_arg, b_arg);
 }
 
 template <class R, int DIR, int BATCH = 0>
@@ -266,15 +269,13 @@ void launch_sediment(const StateT<R>& S, const CoefT<R>& c, bool xdir, bool bed,
   int launched = nfs + 1;
   if (!bed || S.N < 5) {
     const dim3 gfs(cdiv(S.M, 128), cdiv(S.N, FS_ROWS), z);
-    if (b.n > 0) k_update_fs<R, 1><<<gfs, 128, 0, st>>>(S, c, b);
-    else k_update_fs<R, 0><<<gfs, 128, 0, st>>>(S, c, b);
+    launch2(HYD_K2(k_update_fs, R), gfs, 128, st, S, c, b);
   } else {
     // the bed change once per step, after the j-sweep (engine.cpp:290-293),
     // and with it the concentration's commit; the flux Qb was computed by
     // this step's second commit (k_commit_b)
     const dim3 gl(cdiv(S.M, 128), S.N, z);
-    if (b.n > 0) k_bed_load_b<R><<<gl, 128, 0, st>>>(S, c, b);
-    else k_bed_load<R, 0><<<gl, 128, 0, st>>>(S, c, b);
+    launch2(HYD_K2B(k_bed_load, R), gl, 128, st, S, c, b);
     if (S.bed_fb) {
       launch_bed_feedback(S, c, st, b);
       ++launched;

@@ -521,14 +521,19 @@ static void launch_row_nt(const Gen& G, int ncells, int lines, cudaStream_t st,
                          lim.optin - 8192);
     attr[dev] = true;
   }
-  k_row_solve<Gen, NT, BATCH>
-      <<<dim3(lines, std::max(b.n, 1)), NT, row_smem<Gen>(ncells), st>>>(G, b);
+  const dim3 grid(lines, std::max(b.n, 1));
+  const size_t smem = row_smem<Gen>(ncells);
+  if constexpr ((BATCH & 2) != 0) launch_dependent(k_row_solve<Gen, NT, BATCH>, grid, NT, smem, st, G, b);
+  else k_row_solve<Gen, NT, BATCH><<<grid, NT, smem, st>>>(G, b);
 }
 
 template <class Gen, int NT>
 static void launch_row_b(const Gen& G, int ncells, int lines, cudaStream_t st,
                          const Batch<typename Gen::Real>& b) {
-  if (b.n > 0) launch_row_nt<Gen, NT, 1>(G, ncells, lines, st, b);
+  const bool dep = dependent_launches(G.S, b);
+  if (b.n > 0 && dep) launch_row_nt<Gen, NT, 3>(G, ncells, lines, st, b);
+  else if (b.n > 0) launch_row_nt<Gen, NT, 1>(G, ncells, lines, st, b);
+  else if (dep) launch_row_nt<Gen, NT, 2>(G, ncells, lines, st, b);
   else launch_row_nt<Gen, NT, 0>(G, ncells, lines, st, b);
 }
 
@@ -568,8 +573,12 @@ static void launch_col_nt(const Gen& G, int ncells, int lines, cudaStream_t st,
                          (int)col_smem<Gen, L>(COL_MAX));
     attr[dev] = true;
   }
-  k_col_solve<Gen, NT, L, BATCH>
-      <<<dim3(cdiv(lines, L), std::max(b.n, 1)), NT, col_smem<Gen, L>(ncells), st>>>(G, b);
+  const dim3 grid(cdiv(lines, L), std::max(b.n, 1));
+  const size_t smem = col_smem<Gen, L>(ncells);
+  if constexpr ((BATCH & 2) != 0)
+    launch_dependent(k_col_solve<Gen, NT, L, BATCH>, grid, NT, smem, st, G, b);
+  else
+    k_col_solve<Gen, NT, L, BATCH><<<grid, NT, smem, st>>>(G, b);
 }
 
 // Threads of a column group: about eight cells each, four on short columns
@@ -587,7 +596,10 @@ static void launch_col_l(const Gen& G, int ncells, int lines, cudaStream_t st,
 template <class Gen, int L>
 static void launch_cols(const Gen& G, int ncells, int lines, cudaStream_t st,
                         const Batch<typename Gen::Real>& b) {
-  if (b.n > 0) launch_col_l<Gen, L, 1>(G, ncells, lines, st, b);
+  const bool dep = dependent_launches(G.S, b);
+  if (b.n > 0 && dep) launch_col_l<Gen, L, 3>(G, ncells, lines, st, b);
+  else if (b.n > 0) launch_col_l<Gen, L, 1>(G, ncells, lines, st, b);
+  else if (dep) launch_col_l<Gen, L, 2>(G, ncells, lines, st, b);
   else launch_col_l<Gen, L, 0>(G, ncells, lines, st, b);
 }
 
