@@ -11,8 +11,8 @@ bathymetry, sediment from t=600 s. The state is spun up to t=600 s before
 timing so that every timed step runs the sediment sweeps. value is
 cell-steps/s (N*M interior cells x steps / device seconds), whole job. Each
 step is one replay of the step's CUDA graph (hydist_step_graph), the path the
-ensembles and the server take; --eager launches the kernels one by one
-(hydist_step).
+ensembles and the server take; --eager launches the kernels one by one (the
+two hydist_half_step of each step).
 
 Multi-GPU: scenarios are independent, so N GPUs run N replicas with no
 data-path collective (weak scaling); the time is the max over ranks.
@@ -50,10 +50,10 @@ BYTES_PER_CELL_STEP = {  # algorithmic bytes per interior cell and full step
 #     Tsxw (Tsyw) = 9 x 8 B; write t_z and t_u (t_v) = 2 x 8 B  -> 88 B
 #   concentration sweeps: read FS, H_moi, VTH, Fw, t_u, t_v, Htdu, Htdv, Kx,
 #     Ky = 10 x 8 B; write tFS = 8 B                             -> 88 B
-#     (a concentration sweep is timed over its two launches: the per-cell
-#     row kernel k_fs_rows and the line solve)
-# The line-solver scratch (3 doubles per unknown) and the concentration rows
-# passed between the two launches (4 doubles per cell) are not counted.
+#     (the concentration sweep of columns of more than 1100 cells is timed
+#     over its two launches: the per-cell row kernel k_fs_rows and the solve)
+# The chunked solver's scratch (3 doubles per unknown) and the concentration
+# rows passed between those two launches (4 doubles per cell) are not counted.
 # In the FP32 form z is read (8 B) and t_z written (8 B) in FP64, the other
 # fields are 4 B: hydraulic 8 + 8 x 4 + 8 + 4 = 52 B, concentration 11 x 4 = 44 B.
 SWEEP_BYTES_PER_CELL = {
@@ -61,6 +61,15 @@ SWEEP_BYTES_PER_CELL = {
              "line_solve_conc_x": 88, "line_solve_conc_y": 88},
     "fp32": {"line_solve_hydro_x": 52, "line_solve_hydro_y": 52,
              "line_solve_conc_x": 44, "line_solve_conc_y": 44}}
+
+
+def eager_steps(sim):
+    """Steps of `sim` launch by launch (hydist_step replays a graph)."""
+    def step(n):
+        for _ in range(n):
+            sim.half_step(0)
+            sim.half_step(1)
+    return step
 
 
 def sweep_cells(name, N, M):
@@ -563,7 +572,9 @@ def run_tridiag(args):
     lib.hydist_gtsv_band_bounds(bands)
     nonempty = 0
     lo = 0
-    for hi in list(bands):
+    # one launch per non-empty length class (a batch of this many short systems
+    # is not merged into one)
+    for hi in (32, 128, 256, 512, 1024, 1536, 2048, 3072, 4096, 6144, 1 << 30):
         nonempty += int(((ln > lo) & (ln <= hi)).sum() > 0)
         lo = hi
     # accuracy against the FP64 oracle, and e2e through host buffers
@@ -712,7 +723,8 @@ def run_ours(args):
     if spin:
         sim.step(spin)
     # warm-up in the timed mode (a graph is captured on its first step)
-    (sim.step_graph if args.graph else sim.step)(max(args.warmup, 3))
+    step = sim.step_graph if args.graph else eager_steps(sim)
+    step(max(args.warmup, 3))
     sim.sync()
     l0 = sim.kernel_launches
     stream = torch.cuda.ExternalStream(sim.stream, device=dev)
@@ -726,10 +738,7 @@ def run_ours(args):
     e0.record(stream)
     step_ev[0].record(stream)
     for k in range(args.steps):
-        if args.graph:
-            sim.step_graph(1)
-        else:
-            sim.step(1)
+        step(1)
         step_ev[k + 1].record(stream)
     e1.record(stream)
     torch.cuda.synchronize(dev)
@@ -990,7 +999,7 @@ def measure_e2e(H, bundle, dev, prec, args):
     t1 = time.perf_counter()
     create = {k: round(v, 3) for k, v in sim.create_phases().items()}
     for _ in range(args.steps):
-        (sim.step_graph if args.graph else sim.step)(1)
+        (sim.step_graph if args.graph else eager_steps(sim))(1)
         sim.mass()
     t2 = time.perf_counter()
     for f, o in outs.items():
@@ -1028,7 +1037,7 @@ def main():
                          "HydistGtsvAlgo; 0: the autotuned one per band)")
     ap.add_argument("--eager", action="store_true",
                     help="launch each step's kernels one by one instead of replaying the "
-                         "step's CUDA graph (hydist_step instead of hydist_step_graph)")
+                         "step's CUDA graph (hydist_half_step instead of hydist_step_graph)")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--no-forms", action="store_true",

@@ -98,9 +98,10 @@ struct StateT {
   R *su, *sv;    // t_u / t_v after the smoothing of the current half-step
   int* err;      // [0]: DevErr; [1]: this half-step dried or wetted a cell;
                  // [2]: blocks of k_interp_fs done (0 between launches)
-  R* lscratch;   // partitioned line solver: one slot per resident CTA
-  // the rows of the next concentration sweep (A, B, C, D of every cell:
-  // four arrays of (N+3)*(M+3), array k at pre + k*W*H)
+  R* lscratch;   // chunked line solver: one slot per resident CTA
+  // the rows of the next concentration sweep where its solver does not form
+  // them itself (A, B, C, D of every cell: four arrays of (N+3)*(M+3), array k
+  // at pre + k*W*H); the transfers of FP32 fields convert in it
   R* pre;
   int lslots;    // number of slots (CTAs of the persistent sweep grid)
   int* colflag;  // per column: holds a cell dried during the run

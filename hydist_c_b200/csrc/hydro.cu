@@ -12,7 +12,7 @@
 //                        it also advances the device clock]
 //   the line sweeps     [UZSolver_*/VZSolver_* + tridiagSolver,
 //                        UVZSolver_multithread.cpp:19-139, 142-603, 798-933]:
-//                        sweep.cu on the partitioned solver of linesolve.cuh
+//                        sweep.cu
 //   k_smooth_full       [Normalize/_normalize/update_buffer, :761-808]
 //   k_solve_v/k_solve_u [solveV/vSolver, solveU/uSolver, :607-795, 938-978;
 //                        update_margin_elem_V/U, :980-1060]

@@ -1,11 +1,12 @@
-// linesolve.cuh -- partitioned tridiagonal line solver for the ADI sweeps.
+// linesolve.cuh -- chunked tridiagonal line solver for the lines that the
+// staged solvers (rowsolve.cuh, colsolve.cuh) do not take: columns of more than
+// 1100 cells, rows of more than one CTA's shared memory holds.
 //
-// One CTA solves L adjacent lines at a time (LPB = 4; XPB = 8 for the
-// 128-chunk column sweeps; a persistent loop walks the line groups). Each
-// line is split into P chunks of consecutive cells; thread (chunk k, line l)
-// = threadIdx.x = k*L + l, so with L = 4 a warp covers 8 chunks x 4 adjacent
-// lines and every global access of a column sweep reads 4 adjacent columns
-// (one 32-byte sector), with L = 8 4 chunks x 8 columns (64 bytes).
+// One CTA solves L adjacent lines at a time (LPB = 4 rows, XPB = 8 columns; a
+// persistent loop walks the line groups). Each line is split into P = 128
+// chunks of consecutive cells; thread (chunk k, line l) = threadIdx.x = k*L + l,
+// so with L = 8 a warp covers 4 chunks x 8 adjacent columns and every global
+// access of a column sweep reads whole sectors (64 bytes in FP64).
 //
 // The line's tridiagonal system (all wet segments of the line, identity rows
 // between them) is solved by the partition method:
@@ -32,8 +33,8 @@
 
 namespace hyd {
 
-constexpr int LPB = 4;  // lines per CTA
-constexpr int XPB = 8;  // lines per CTA of the 128-chunk column sweeps
+constexpr int LPB = 4;  // rows per CTA
+constexpr int XPB = 8;  // columns per CTA
 
 // One wet segment of a line, with its system layout.
 struct SegD {
@@ -73,18 +74,11 @@ constexpr size_t line_smem(bool refine) {
   return sizeof(LSShared<R, P, L>) + (refine ? (size_t)2 * pcr_levels(P) * P * L * sizeof(R) : 0);
 }
 
-// Gen::MIN_BLOCKS: resident CTAs per SM the P = 128 solver is compiled for
-// (2 caps registers at 64 per thread). The solvers for shorter lines (fewer
-// chunks, smaller CTAs) are compiled for at least 512 threads per SM, the
-// row sweeps' for as many as their P = 128 solver (at most 32 CTAs): left
-// uncapped, the row sweeps' short-line solvers took up to 198 registers and
-// ran 8 warps per SM; the column sweeps' spill under the 64-register cap.
+// resident CTAs per SM: one of the columns' 1024 threads (64 registers each),
+// Gen::MIN_BLOCKS of the rows' 512 (2 caps registers at 64 per thread)
 template <class Gen, int P, int L>
 constexpr int line_min_blocks() {
-  constexpr int k = (L * P >= 512) ? 1 : 512 / (L * P);
-  constexpr int b = Gen::DIRECTION == 1 ? k * Gen::MIN_BLOCKS : k;
-  if (L * P >= 1024) return 1;  // one CTA per SM, 64 registers per thread
-  return (P == 128 && L == LPB) ? Gen::MIN_BLOCKS : (b > 32 ? 32 : b);
+  return L * P >= 1024 ? 1 : Gen::MIN_BLOCKS;
 }
 
 // The launch solves line groups 0 .. ngroups-1 of L lines from line0 on.

@@ -4,9 +4,9 @@
 //   Find_VTH + hesoK [sediment_transport.cpp:575-602, 539-573] run in the
 //                  hydraulic commits (hydro.cu: k_commit_a, k_commit_b)
 //   the sweeps     [Scan_FSj/Scan_FSi + tridiagSolver + FSj/FSi_extract_
-//                   solution, :51-349, 604-651]: the partitioned line solver
-//                   with FSGen (sweep.cu), cell rows in sediment_cell.cuh
-//   k_update_fs    [Update_FS, :654-663]
+//                   solution, :51-349, 604-651]: FSGen (sweep.cu), cell rows in
+//                   sediment_cell.cuh (k_fs_rows ahead of the chunked solver)
+//   k_update_fs    [Update_FS, :654-663; with the bed change in k_bed_load]
 //   Calculate_Qb   [:352-434] runs in the second commit (hydro.cu k_commit_b)
 //   k_bed_load     [_bed_load / BedLoad, :436-537, :664-673]
 #include "common.cuh"

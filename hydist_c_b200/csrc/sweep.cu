@@ -1,4 +1,4 @@
-// sweep.cu -- the hydraulic ADI line sweeps on the partitioned line solver.
+// sweep.cu -- the ADI line sweeps: what they solve, and which solver takes them.
 //
 // HydroGen<0> is the x sweep (UZ half-step: lines are columns j, cells run
 // along i, unknowns u_i); HydroGen<1> is the y sweep (VZ half-step: lines are
@@ -21,17 +21,6 @@
 
 namespace hyd {
 
-// chunks per line: as many as keep at least `min_cells` cells per chunk (of
-// 128, 64, 32, 16, 4 or 1), so that no chunk of a short line is empty or
-// holds its separator alone
-int line_chunks(int ncells, int min_cells) {
-  int P = 128;
-  while (P > 1 && ncells < P * min_cells) P >>= 1;
-  if (P == 8) P = 4;
-  if (P == 2) P = 1;
-  return P;
-}
-
 // REF: refine each line solve once with an FP64 residual (FP32 forms)
 template <int DIR, class R, bool REF = false>
 struct HydroGen {
@@ -44,10 +33,9 @@ struct HydroGen {
   static constexpr int SCRATCH_ARRAYS = AUX + 1;
   static constexpr bool HYDRO = true;
   static constexpr int DIRECTION = DIR;
-  // x sweeps (columns, 4 adjacent per warp) run faster with two CTAs per SM
-  // despite the register cap, and so do the FP32 y sweeps; the FP64 and the
-  // refined FP32 y sweeps slower
-  static constexpr int MIN_BLOCKS = (DIR == 0 || (sizeof(R) == 4 && !REF)) ? 2 : 1;
+  // resident CTAs per SM the chunked row solver is compiled for: the FP32 rows
+  // run faster with two despite the register cap, the FP64 and refined slower
+  static constexpr int MIN_BLOCKS = sizeof(R) == 4 && !REF ? 2 : 1;
   StateT<R> S;
   CoefT<R> c;
   R* scratch;
@@ -603,12 +591,13 @@ static void launch_cols(const Gen& G, int ncells, int lines, cudaStream_t st,
   else launch_col_l<Gen, L, 0>(G, ncells, lines, st, b);
 }
 
-// Launches a sweep over `lines` lines and returns the number of launches.
-// With a batch, one launch walks the line groups of every member (the
-// persistent grid takes them in member order).
+// Launches a sweep over `lines` lines and returns the number of launches: rows
+// by the staged row solver, columns by the staged column solver, what these do
+// not take by the chunked one, whose launch walks the line groups of every
+// member of a batch (its persistent grid takes them in member order).
 template <class Gen>
-static int launch_lines(const Gen& G, int P, int ncells, int lines, int lslots, cudaStream_t st,
-                        const Batch<typename Gen::Real>& b = {}) {
+static int launch_lines(const Gen& G, int ncells, int lines, cudaStream_t st,
+                        const Batch<typename Gen::Real>& b) {
   if constexpr (Gen::DIRECTION == 1) {
     if (row_fits<Gen>(ncells)) {
       launch_rows(G, ncells, lines, st, b);
@@ -616,7 +605,7 @@ static int launch_lines(const Gen& G, int P, int ncells, int lines, int lslots, 
     }
     const int groups = cdiv(lines, LPB);
     const long long total = (long long)groups * std::max(b.n, 1);
-    launch_gen<Gen, 128>(G, st, (int)std::min<long long>(total, lslots), 0, (int)total, b,
+    launch_gen<Gen, 128>(G, st, (int)std::min<long long>(total, G.S.lslots), 0, (int)total, b,
                          b.n > 0 ? groups : 0);
     return 1;
   } else {
@@ -628,37 +617,21 @@ static int launch_lines(const Gen& G, int P, int ncells, int lines, int lslots, 
     // per SM (a group's scratch slot is two of the 4-line slots)
     const int g8 = cdiv(lines, XPB);
     const long long total = (long long)g8 * std::max(b.n, 1);
-    launch_gen<Gen, 128, XPB>(G, st, (int)std::min<long long>(total, lslots / 2), 0, (int)total, b,
+    launch_gen<Gen, 128, XPB>(G, st, (int)std::min<long long>(total, G.S.lslots / 2), 0, (int)total, b,
                               b.n > 0 ? g8 : 0);
     return 1;
   }
 }
 
-// Scratch slots for a sweep of lines of `unknowns` unknowns in P chunks:
-// the scratch holds StateT::lslots slots of lines of max(M, N) unknowns,
-// so a sweep of shorter lines has proportionally more. Only the solvers of
-// fewer than 128 chunks (smaller CTAs, more of them resident per SM) use
-// them: their grid may then exceed the CTAs resident at once, the extra
-// CTAs starting as earlier ones finish. (For the 128-chunk solvers the
-// persistent grid of lslots CTAs measured as fast or faster.)
-template <class R>
-static int sweep_slots(const StateT<R>& S, int unknowns, int P) {
-  if (P >= 128) return S.lslots;
-  const int umax = std::max(S.M, S.N);
-  return S.lslots * std::max(1, umax / std::max(unknowns, 1));
-}
-
 template <int DIR, class R, bool REF>
-static int launch_dir(const StateT<R>& S, const CoefT<R>& c, cudaStream_t st, int P,
-                      const Batch<R>& b) {
+static int launch_dir(const StateT<R>& S, const CoefT<R>& c, cudaStream_t st, const Batch<R>& b) {
   HydroGen<DIR, R, REF> G;
   G.bind(S, c);
   G.scratch = S.lscratch;
   G.lp0 = DIR == 0 ? S.x_lo : S.y_lo;
   G.nl = DIR == 0 ? S.x_hi - S.x_lo + 1 : S.N - S.y_lo + 1;
   if (G.nl <= 0) return 0;
-  const int ncells = DIR == 0 ? S.N - 1 : S.M - 1;
-  return launch_lines(G, P, ncells, G.nl, sweep_slots(S, ncells, P), st, b);
+  return launch_lines(G, DIR == 0 ? S.N - 1 : S.M - 1, G.nl, st, b);
 }
 
 // ---------------------------------------------------------------------
@@ -676,8 +649,7 @@ struct FSGen {
   static constexpr int SCRATCH_ARRAYS = REFINE ? 4 : 3;
   static constexpr bool HYDRO = false;
   static constexpr int DIRECTION = DIR;
-  // two CTAs per SM in both directions and precisions
-  static constexpr int MIN_BLOCKS = 2;
+  static constexpr int MIN_BLOCKS = 2;  // in both precisions
   StateT<R> S;
   CoefT<R> c;
   R* scratch;
@@ -904,30 +876,26 @@ int launch_fs_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t
   const int ncells = dir == 0 ? S.N - 1 : S.M - 1;
   const int lines = dir == 0 ? S.M - 3 : S.N - 3;
   if (lines <= 0) return 0;
-  const int P = line_chunks(ncells, 4);
-  const int slots = sweep_slots(S, ncells, P);
   if constexpr (sizeof(R) == 4) {
     if (S.refine && dir == 0)
-      return launch_lines(FSGen<0, R, true>{S, c, S.lscratch}, P, ncells, lines, slots, st, b);
-    if (S.refine) return launch_lines(FSGen<1, R, true>{S, c, S.lscratch}, P, ncells, lines, slots, st, b);
+      return launch_lines(FSGen<0, R, true>{S, c, S.lscratch}, ncells, lines, st, b);
+    if (S.refine) return launch_lines(FSGen<1, R, true>{S, c, S.lscratch}, ncells, lines, st, b);
   }
-  if (dir == 0) return launch_lines(FSGen<0, R, false>{S, c, S.lscratch}, P, ncells, lines, slots, st, b);
-  return launch_lines(FSGen<1, R, false>{S, c, S.lscratch}, P, ncells, lines, slots, st, b);
+  if (dir == 0) return launch_lines(FSGen<0, R, false>{S, c, S.lscratch}, ncells, lines, st, b);
+  return launch_lines(FSGen<1, R, false>{S, c, S.lscratch}, ncells, lines, st, b);
 }
 
 template <class R>
 int launch_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t st,
                  const Batch<R>& b) {
-  const int ncells = dir == 0 ? S.N - 1 : S.M - 1;
-  const int P = line_chunks(ncells, 4);
   if constexpr (sizeof(R) == 4) {  // (the refinement is of the FP32 form)
     if (S.refine) {
-      if (dir == 0) return launch_dir<0, R, true>(S, c, st, P, b);
-      return launch_dir<1, R, true>(S, c, st, P, b);
+      if (dir == 0) return launch_dir<0, R, true>(S, c, st, b);
+      return launch_dir<1, R, true>(S, c, st, b);
     }
   }
-  if (dir == 0) return launch_dir<0, R, false>(S, c, st, P, b);
-  return launch_dir<1, R, false>(S, c, st, P, b);
+  if (dir == 0) return launch_dir<0, R, false>(S, c, st, b);
+  return launch_dir<1, R, false>(S, c, st, b);
 }
 
 template bool fs_rows_in_sweep<double>(const StateT<double>&, int);

@@ -226,7 +226,9 @@ int hydist_create_external(const HydistExternal* ext, const HydistParams* p,
 
 /* Advance nsteps full ADI steps (two half-steps each): the body of the time
  * loop of Hydraulic_Calculation (engine.cpp:65-295). Stream-ordered on the
- * handle's stream; returns once the work is enqueued. */
+ * handle's stream; returns once the work is enqueued. Steps of a call of eight
+ * or more, and those after eight single ones, replay a CUDA graph of the step
+ * that the first of them captures (except inside a capture of the caller's). */
 int hydist_step(HydistHandle* h, int32_t nsteps);
 
 /* One half of a step: half 0 = t += dT/2, the x sweep (UZ), explicit v,
@@ -254,8 +256,8 @@ int hydist_upload(HydistHandle* h, int32_t field, const void* host);
 /* Water volume sum over wet cells of (htaiz + z) * dX * dY, accumulated in
  * FP64 on the device (mass-conservation check). */
 int hydist_mass(HydistHandle* h, double* volume);
-/* Run nsteps with each step captured once into a CUDA graph and replayed.
- * Same results as hydist_step. */
+/* Run nsteps with each step captured once into a CUDA graph and replayed
+ * from the first on. Same results as hydist_step. */
 int hydist_step_graph(HydistHandle* h, int32_t nsteps);
 /* The CUDA stream the handle enqueues on (a cudaStream_t). */
 void* hydist_stream(HydistHandle* h);

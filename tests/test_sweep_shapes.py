@@ -3,8 +3,8 @@ one-launch and skipped forms.
 
 Meshes: rows of one to sixteen warps a row and columns of four to sixteen
 warps a group, the last column group ragged, columns one cell below and above
-the staged solver's limit (1100 cells), islands that leave several segments in
-rows and columns, more columns than rows (the reference's y sweep writes
+the staged solver's limit (1100 cells), rows beyond the staged solver's in
+every form, islands that leave several segments in rows and columns, more columns than rows (the reference's y sweep writes
 columns up to N only). From the oracle's state after 8 steps one step on each
 agrees to 1e-10 of a field's magnitude in FP64, to 1e-4 in the FP32 forms
 (the bounds of the parity tests)."""
@@ -15,7 +15,7 @@ from hydist_c_b200 import scenario as S
 
 STATE = ["u", "v", "z", "t_u", "t_v", "t_z", "H_moi", "Htdu", "Htdv", "FS", "tFS"]
 MESHES = [(9, 8), (33, 30), (66, 34), (131, 67), (162, 161), (259, 353), (354, 64), (520, 1155),
-          (1101, 41), (1102, 41), (2307, 24)]
+          (1101, 41), (1102, 41), (2307, 24), (20, 18200)]
 
 
 def _mesh(N, M):
