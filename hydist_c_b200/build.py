@@ -21,7 +21,7 @@ LIB = PKG / "libhydist_b200.so"
 SOURCES = ["engine.cu", "hydro.cu", "sweep.cu", "sediment.cu", "tridiag.cu", "compat.cu", "server.cu",
            "uvz_compat.cu"]
 HEADERS = ["common.cuh", "hydro.cuh", "assembly.cuh", "linesolve.cuh", "partsolve.cuh", "sediment_cell.cuh",
-           "explicit.cuh", "rowsolve.cuh", "colsolve.cuh"]
+           "explicit.cuh", "rowsolve.cuh", "colsolve.cuh", "pairgen.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
               "-Xptxas", "-v"]

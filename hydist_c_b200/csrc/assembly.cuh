@@ -25,11 +25,9 @@ using Pre = PreT<double>;
 
 // The momentum part of the preindex step: f1 u_{-} + f2 u + f3 u_{+} +
 // f4 (z - z_{+}) = f5 along the line, before the continuity rows enter it.
-// g2, g5: f2 and f5 without the time derivative's terms, f2 = -(2 + g2),
-// f5 = -2 u + g5.
 template <class R>
 struct MomF {
-  R f1, f2, f3, f5, g2, g5;
+  R f1, f2, f3, f5;
 };
 
 // _uzSolver_calculate_preindex (UVZSolver_multithread.cpp:210-278): the
@@ -53,9 +51,7 @@ __device__ __forceinline__ MomF<R> mom_x(const StateT<R>& S, const CoefT<R>& c, 
   const R rH = R(1) / Hu;
   const R visc = VI * c.dT_dXbp;
   P.f1 = c.dTchia2dX * uu + visc;
-  const R fr = S.Kx1[g] * dT * sqrt(uu * uu + vtb * vtb) * rH;
-  P.f2 = -(2 + fr + 2 * visc);
-  P.g2 = fr + 2 * visc;
+  P.f2 = -(2 + S.Kx1[g] * dT * sqrt(uu * uu + vtb * vtb) * rH + 2 * visc);
   P.f3 = visc - c.dTchia2dX * uu;
   if (hm1 <= c.H_TINH) {
     if (vtb < 0) {
@@ -75,7 +71,6 @@ __device__ __forceinline__ MomF<R> mom_x(const StateT<R>& S, const CoefT<R>& c, 
   }
   P.f5 = -2 * uu + dT * p - dT * c.CORIOLIS_FORCE * vtb - dT * VI * q -
          dT * (c.Windx - S.Tsxw[g]) * rH;
-  P.g5 = dT * p - dT * c.CORIOLIS_FORCE * vtb - dT * VI * q - dT * (c.Windx - S.Tsxw[g]) * rH;
   return P;
 }
 
@@ -86,12 +81,48 @@ __device__ __forceinline__ R flux_x(const StateT<R>& S, const CoefT<R>& c, int g
   return c.dTchia2dY * (S.Htdv[g] * S.v[g] - S.Htdv[g - 1] * S.v[g - 1]);
 }
 
+// All of the preindex step as one statement: put together from mom_x, its sums
+// and products are contracted otherwise, and the FP32 sweeps depend on their
+// bits (pairgen.cuh).
 template <class R>
 __device__ __forceinline__ PreT<R> pre_x(const StateT<R>& S, const CoefT<R>& c, int i, int j) {
-  const int g = i * S.W + j;
-  const MomF<R> m = mom_x(S, c, i, j);
-  return PreT<R>{m.f1, m.f2, m.f3, m.f5, -c.dTchia2dX * S.Htdu[g - S.W], c.dTchia2dX * S.Htdu[g],
-                 R(S.z[g]) - flux_x(S, c, g)};
+  const int w = S.W;
+  const int g = i * w + j;
+  const R* u = S.u;
+  const R* v = S.v;
+  const R* Hm = S.Hmoi;
+  PreT<R> P;
+  R p = 0, q = 0;
+  const R vtb = (v[g - 1] + v[g] + v[g + w - 1] + v[g + w]) * R(0.25);
+  const R uu = u[g], VI = S.visco[g], Hu = S.Htdu[g];
+  const R dT = c.dT;
+  const R rH = R(1) / Hu;
+  const R visc = VI * c.dT_dXbp;
+  P.f1 = c.dTchia2dX * uu + visc;
+  P.f2 = -(2 + S.Kx1[g] * dT * sqrt(uu * uu + vtb * vtb) * rH + 2 * visc);
+  P.f3 = visc - c.dTchia2dX * uu;
+  if (Hm[g - 1] <= c.H_TINH) {
+    if (vtb < 0) {
+      p = vtb * (-3 * uu + 4 * u[g + 1] - u[g + 2]) * c.r_dY2;
+      q = (uu - 2 * u[g + 1] + u[g + 2]) * c.r_dYbp;
+    }
+  } else {
+    if (Hm[g + 1] <= c.H_TINH) {
+      if ((Hm[g - 2] > c.H_TINH) && (vtb > 0)) {
+        p = vtb * (3 * uu - 4 * u[g - 1] + u[g - 2]) * c.r_dY2;
+        q = (uu - 2 * u[g - 1] + u[g - 2]) * c.r_dYbp;
+      }
+    } else {
+      p = vtb * (u[g + 1] - u[g - 1]) * c.r_dY2;
+      q = (u[g + 1] - 2 * uu + u[g - 1]) * c.r_dYbp;
+    }
+  }
+  P.f5 = -2 * uu + dT * p - dT * c.CORIOLIS_FORCE * vtb - dT * VI * q -
+         dT * (c.Windx - S.Tsxw[g]) * rH;
+  P.c2 = c.dTchia2dX * Hu;
+  P.a2 = -c.dTchia2dX * S.Htdu[g - w];
+  P.d2 = R(S.z[g]) - c.dTchia2dY * (S.Htdv[g] * v[g] - S.Htdv[g - 1] * v[g - 1]);
+  return P;
 }
 
 // _vzSolver_calculate_preindex (UVZSolver_multithread.cpp:142-208).
@@ -114,9 +145,7 @@ __device__ __forceinline__ MomF<R> mom_y(const StateT<R>& S, const CoefT<R>& c, 
   const R rH = R(1) / Hv;
   const R visc = VI * c.dT_dYbp;
   P.f1 = c.dTchia2dY * vv + visc;
-  const R fr = S.Ky1[g] * dT * sqrt(vv * vv + utb * utb) * rH;
-  P.f2 = -(2 + fr + 2 * visc);
-  P.g2 = fr + 2 * visc;
+  P.f2 = -(2 + S.Ky1[g] * dT * sqrt(vv * vv + utb * utb) * rH + 2 * visc);
   P.f3 = visc - c.dTchia2dY * vv;
   if (hm1 <= c.H_TINH) {
     if (utb < 0) {
@@ -136,7 +165,6 @@ __device__ __forceinline__ MomF<R> mom_y(const StateT<R>& S, const CoefT<R>& c, 
   }
   P.f5 = -2 * vv + dT * q + dT * c.CORIOLIS_FORCE * utb - dT * VI * p -
          dT * (c.Windy - S.Tsyw[g]) * rH;
-  P.g5 = dT * q + dT * c.CORIOLIS_FORCE * utb - dT * VI * p - dT * (c.Windy - S.Tsyw[g]) * rH;
   return P;
 }
 
@@ -147,10 +175,47 @@ __device__ __forceinline__ R flux_y(const StateT<R>& S, const CoefT<R>& c, int g
 
 template <class R>
 __device__ __forceinline__ PreT<R> pre_y(const StateT<R>& S, const CoefT<R>& c, int i, int j) {
-  const int g = i * S.W + j;
-  const MomF<R> m = mom_y(S, c, i, j);
-  return PreT<R>{m.f1, m.f2, m.f3, m.f5, -c.dTchia2dY * S.Htdv[g - 1], c.dTchia2dY * S.Htdv[g],
-                 R(S.z[g]) - flux_y(S, c, g)};
+  const int w = S.W;
+  const int g = i * w + j;
+  const R* u = S.u;
+  const R* v = S.v;
+  const R* Hm = S.Hmoi;
+  PreT<R> P;
+  R p = 0, q = 0;
+  const R utb = (u[g - w] + u[g] + u[g - w + 1] + u[g + 1]) * R(0.25);
+  const R vv = v[g], VI = S.visco[g], Hv = S.Htdv[g];
+  const R dT = c.dT;
+  // the cross-line stencil (rows i-2..i+2, inside the array for rows 2..N)
+  // loaded before the upwind tests choose from it
+  const R vm1 = v[g - w], vm2 = v[g - 2 * w], vp1 = v[g + w], vp2 = v[g + 2 * w];
+  const R hm1 = Hm[g - w], hp1 = Hm[g + w], hm2 = Hm[g - 2 * w];
+  const R rH = R(1) / Hv;
+  const R visc = VI * c.dT_dYbp;
+  P.f1 = c.dTchia2dY * vv + visc;
+  P.f2 = -(2 + S.Ky1[g] * dT * sqrt(vv * vv + utb * utb) * rH + 2 * visc);
+  P.f3 = visc - c.dTchia2dY * vv;
+  if (hm1 <= c.H_TINH) {
+    if (utb < 0) {
+      q = utb * (-3 * vv + 4 * vp1 - vp2) * c.r_dX2;
+      p = (vv - 2 * vp1 + vp2) * c.r_dXbp;
+    }
+  } else {
+    if (hp1 <= c.H_TINH) {
+      if ((hm2 > c.H_TINH) && (utb > 0)) {
+        q = utb * (3 * vv - 4 * vm1 + vm2) * c.r_dX2;
+        p = (vv - 2 * vm1 + vm2) * c.r_dXbp;
+      }
+    } else {
+      q = utb * (vp1 - vm1) * c.r_dX2;
+      p = (vp1 - 2 * vv + vm1) * c.r_dXbp;
+    }
+  }
+  P.f5 = -2 * vv + dT * q + dT * c.CORIOLIS_FORCE * utb - dT * VI * p -
+         dT * (c.Windy - S.Tsyw[g]) * rH;
+  P.c2 = c.dTchia2dY * Hv;
+  P.a2 = -c.dTchia2dY * S.Htdv[g - 1];
+  P.d2 = R(S.z[g]) - c.dTchia2dX * (S.Htdu[g] * u[g] - S.Htdu[g - w] * u[g - w]);
+  return P;
 }
 
 template <class R>

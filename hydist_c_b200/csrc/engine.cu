@@ -547,8 +547,9 @@ int new_handle(const HydistParams* p, const HydistOptions* o, int device, int M,
 // The arrays only this library uses: smoothing buffers, boundary weights,
 // line-solver scratch, flags, counters, the device clock.
 // The FP64 / FP32 arrays only this library uses: smoothing buffers and the
-// line-solver scratch (4 values per unknown, 4 lines per slot, one slot per
-// CTA of the persistent sweep grid).
+// line-solver scratch (4 values per unknown, in the FP32 forms 3 for each of two
+// unknowns per cell; 4 lines per slot, one slot per CTA of the persistent sweep
+// grid).
 template <class R>
 int bulk_private(HydistHandle* h, StateT<R>& B) {
   const State& S = h->S;
@@ -562,9 +563,9 @@ int bulk_private(HydistHandle* h, StateT<R>& B) {
   B.lslots = 2 * nsm;
   const size_t U = (size_t)std::max(S.M, S.N);
   // at least 4 (max(M,N)+3) doubles: preprocess_data borrows it as FP64;
-  // the refined FP32 form keeps 8 values per unknown (its refinement stores
+  // the refined FP32 form keeps 7 values per unknown (its refinement stores
   // the rows)
-  const size_t arrays = S.refine ? 8 : 4;
+  const size_t arrays = S.refine ? 14 : sizeof(R) == 4 ? 6 : 4;
   TRY(dalloc(h, &B.lscratch, std::max((size_t)B.lslots * arrays * U * 4, 16 * U + 128)));
   return HYDIST_OK;
 }

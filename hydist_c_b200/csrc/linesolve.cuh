@@ -1,12 +1,14 @@
-// linesolve.cuh -- chunked tridiagonal line solver for the lines that the
-// staged solvers (rowsolve.cuh, colsolve.cuh) do not take: columns of more than
-// 1100 cells, rows of more than one CTA's shared memory holds.
+// linesolve.cuh -- chunked tridiagonal line solver: the hydraulic sweeps of the
+// FP32 forms (pairgen.cuh), and of the other sweeps the lines that the staged
+// solvers (rowsolve.cuh, colsolve.cuh) do not take: columns of more than 1100
+// cells, rows of more than one CTA's shared memory holds.
 //
-// One CTA solves L adjacent lines at a time (LPB = 4 rows, XPB = 8 columns; a
-// persistent loop walks the line groups). Each line is split into P = 128
-// chunks of consecutive cells; thread (chunk k, line l) = threadIdx.x = k*L + l,
-// so with L = 8 a warp covers 4 chunks x 8 adjacent columns and every global
-// access of a column sweep reads whole sectors (64 bytes in FP64).
+// One CTA solves L adjacent lines at a time (LPB = 4 or XPB = 8; a persistent
+// loop walks the line groups). Each line is split into P chunks of consecutive
+// cells (P = 128, fewer for the FP32 forms' short lines); thread (chunk k, line
+// l) = threadIdx.x = k*L + l, so with L = 8 a warp covers 4 chunks x 8 adjacent
+// columns and every global access of a column sweep reads whole sectors (64
+// bytes in FP64).
 //
 // The line's tridiagonal system (all wet segments of the line, identity rows
 // between them) is solved by the partition method:
@@ -33,13 +35,15 @@
 
 namespace hyd {
 
-constexpr int LPB = 4;  // rows per CTA
-constexpr int XPB = 8;  // columns per CTA
+constexpr int LPB = 4;  // lines per CTA
+constexpr int XPB = 8;  // lines per CTA of the wider groups
 
 // One wet segment of a line, with its system layout.
 struct SegD {
   int first, last;
-  int off, rend;  // cells off..rend hold the segment's unknowns
+  // cells off..rend hold the segment's unknowns; with two unknowns per cell
+  // (pairgen.cuh) rows off..rend of the line system are the segment's
+  int off, rend;
   unsigned char br1, br2, ran, qfirst, last_kind, xq_first, xq_last, pad;
 };
 
@@ -74,11 +78,19 @@ constexpr size_t line_smem(bool refine) {
   return sizeof(LSShared<R, P, L>) + (refine ? (size_t)2 * pcr_levels(P) * P * L * sizeof(R) : 0);
 }
 
-// resident CTAs per SM: one of the columns' 1024 threads (64 registers each),
-// Gen::MIN_BLOCKS of the rows' 512 (2 caps registers at 64 per thread)
+// Resident CTAs per SM: one of 1024 threads (64 registers each), Gen::MIN_BLOCKS
+// of 4 lines of 128 chunks (2 caps registers at 64 per thread). The solvers for
+// shorter lines (fewer chunks, smaller CTAs) are compiled for at least 512
+// threads per SM, the row sweeps' for as many as their P = 128 solver (at most
+// 32 CTAs): left uncapped, the row sweeps' short-line solvers took up to 198
+// registers and ran 8 warps per SM; the column sweeps' spill under the
+// 64-register cap.
 template <class Gen, int P, int L>
 constexpr int line_min_blocks() {
-  return L * P >= 1024 ? 1 : Gen::MIN_BLOCKS;
+  constexpr int k = (L * P >= 512) ? 1 : 512 / (L * P);
+  constexpr int b = Gen::DIRECTION == 1 ? k * Gen::MIN_BLOCKS : k;
+  if (L * P >= 1024) return 1;
+  return (P == 128 && L == LPB) ? Gen::MIN_BLOCKS : (b > 32 ? 32 : b);
 }
 
 // The launch solves line groups 0 .. ngroups-1 of L lines from line0 on.
@@ -108,6 +120,7 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
   R* sc_y = scr + UL;
   R* sc_v = scr + 2 * UL;
   const int ncells = G0.cells_per_line();
+  const int upc = Gen::UPC;  // unknowns per cell
 
   // one group of L lines: gg-th of its scenario, with that scenario's G
   auto solve_group = [&](const Gen& G, int gg) {
@@ -122,7 +135,7 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
     // ---- chunk bounds (balanced split of the line's cells)
     const int c0 = (int)(((long long)k * ncells) / P);
     const int c1 = (int)(((long long)(k + 1) * ncells) / P);
-    const int q0 = c0, nu = c1 - c0;  // chunk unknowns [q0, q0+nu)
+    const int q0 = c0 * upc, nu = (c1 - c0) * upc;  // chunk unknowns [q0, q0+nu)
 
     // ---- pass A: forward elimination of the interior, separator row
     {
@@ -133,43 +146,47 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
       // first interior row in terms of both separators, accumulated forward:
       // x_0 = sum_k P_k (y'_k + v'_k x_L) + P_L x_R, P_0 = 1, P_{k+1} = -c'_k P_k
       R Pk = 1, fy = 0, fv = 0;
+      int s = 0;
       for (int c = c0; c < c1; ++c) {
         W.cell(G, LS, c);
-        R A, B, C, D;
-        W.row(G, LS, A, B, C, D);
-        const size_t o = (size_t)c * L + l;
-        if constexpr (Gen::AUX != 0) scr[Gen::AUX * UL + o] = W.aux;
-        if (c == c1 - 1) {
-          sh.sep[0][cidx] = A;
-          sh.sep[1][cidx] = B;
-          sh.sep[2][cidx] = C;
-          sh.sep[3][cidx] = D;
-        } else {
-          R m;
-          if (c == c0) {
-            m = rcp(B);
-            cp = C * m;
-            yp = D * m;
-            vp = -A * m;
+#pragma unroll
+        for (int e = 0; e < Gen::UPC; ++e, ++s) {
+          R A, B, C, D;
+          W.row(G, LS, e, A, B, C, D);
+          if constexpr (Gen::AUX != 0) scr[Gen::AUX * UL + (size_t)(q0 + s) * L + l] = W.aux;
+          if (s == nu - 1) {
+            sh.sep[0][cidx] = A;
+            sh.sep[1][cidx] = B;
+            sh.sep[2][cidx] = C;
+            sh.sep[3][cidx] = D;
           } else {
-            m = rcp(B - A * cp);
-            yp = (D - A * yp) * m;
-            vp = -A * vp * m;
-            cp = C * m;
+            R m;
+            if (s == 0) {
+              m = rcp(B);
+              cp = C * m;
+              yp = D * m;
+              vp = -A * m;
+            } else {
+              m = rcp(B - A * cp);
+              yp = (D - A * yp) * m;
+              vp = -A * vp * m;
+              cp = C * m;
+            }
+            const size_t o = (size_t)(q0 + s) * L + l;
+            if constexpr (Gen::REFINE && !Gen::ROWS_AGAIN) {
+              // the interior rows, for the residual
+              scr[3 * UL + o] = A;
+              scr[4 * UL + o] = B;
+              scr[5 * UL + o] = C;
+              scr[6 * UL + o] = D;
+            }
+            sc_c[o] = cp;
+            sc_y[o] = yp;
+            sc_v[o] = vp;
+            fy += Pk * yp;
+            fv += Pk * vp;
+            Pk *= -cp;
           }
-          if constexpr (Gen::REFINE && !Gen::ROWS_AGAIN) {
-            // the interior rows, for the residual
-            scr[3 * UL + o] = A;
-            scr[4 * UL + o] = B;
-            scr[5 * UL + o] = C;
-            scr[6 * UL + o] = D;
-          }
-          sc_c[o] = cp;
-          sc_y[o] = yp;
-          sc_v[o] = vp;
-          fy += Pk * yp;
-          fv += Pk * vp;
-          Pk *= -cp;
         }
       }
       // first and last interior rows in terms of the neighbouring separators
@@ -244,18 +261,32 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
       const R xl = (k > 0) ? sh.xsep[cidx - L] : R(0);
       typename Gen::Emitter E;
       E.init(G, LS, line);
-      // an unknown is emitted once the one before it is known
-      R xn = xr, ax = 0;
+      if constexpr (Gen::AUX == 0) {
+        // (the FP32 forms' bits hang on this loop's shape: with the other one's
+        // delayed emission the compiler contracts the substitution differently)
+        E.emit(G, LS, sh.xlast[l], q0 + nu - 1, xr, 0.0, R(0));
+        R xn = xr;
 #pragma unroll 4
-      for (int t = nu - 2; t >= 0; --t) {
-        const size_t o = (size_t)(q0 + t) * L + l;
-        const R x = sc_y[o] + sc_v[o] * xl - sc_c[o] * xn;
-        if constexpr (Gen::AUX != 0) ax = scr[Gen::AUX * UL + o + L];
-        E.emit(G, LS, sh.xlast[l], q0 + t + 1, xn, x, ax);
-        xn = x;
+        for (int t = nu - 2; t >= 0; --t) {
+          const size_t o = (size_t)(q0 + t) * L + l;
+          const R x = sc_y[o] + sc_v[o] * xl - sc_c[o] * xn;
+          E.emit(G, LS, sh.xlast[l], q0 + t, x, 0.0, R(0));
+          xn = x;
+        }
+      } else {
+        // an unknown is emitted once the one before it is known
+        R xn = xr, ax = 0;
+#pragma unroll 4
+        for (int t = nu - 2; t >= 0; --t) {
+          const size_t o = (size_t)(q0 + t) * L + l;
+          const R x = sc_y[o] + sc_v[o] * xl - sc_c[o] * xn;
+          ax = scr[Gen::AUX * UL + o + L];
+          E.emit(G, LS, sh.xlast[l], q0 + t + 1, xn, x, ax);
+          xn = x;
+        }
+        ax = scr[Gen::AUX * UL + (size_t)q0 * L + l];
+        E.emit(G, LS, sh.xlast[l], q0, xn, xl, ax);
       }
-      if constexpr (Gen::AUX != 0) ax = scr[Gen::AUX * UL + (size_t)q0 * L + l];
-      E.emit(G, LS, sh.xlast[l], q0, xn, xl, ax);
     } else {
       // one refinement pass. The back substitution stores x over y' and, as
       // soon as x_{t-1..t+1} are known, takes row t's residual
@@ -332,7 +363,8 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
         // the unknown left of the separator: the chunk's last interior one,
         // or the previous chunk's separator; right of it: the next chunk's
         // first unknown, its separator where that chunk holds nothing else
-        const int nu_next = (k + 1 < P) ? (int)(((long long)(k + 2) * ncells) / P) - c1 : 0;
+        const int nu_next = (k + 1 < P)
+            ? ((int)(((long long)(k + 2) * ncells) / P) - c1) * upc : 0;
         const R xm = nu >= 2 ? x_before_sep : (q > 0 ? xl : R(0));
         const R xp = q + 1 < U ? (nu_next >= 2 ? sc_y[o + L] : sh.xsep[cidx + L]) : R(0);
         const R as = sh.sep[0][cidx], bs = sh.sep[1][cidx], cs = sh.sep[2][cidx],
@@ -362,21 +394,15 @@ __global__ void __launch_bounds__(L * P, line_min_blocks<Gen, P, L>())
         const R dl = (k > 0) ? sh.xsep[cidx - L] : R(0);
         typename Gen::Emitter E;
         E.init_fwd(G, LS, line);
-        R dp = dl, ax = 0;
-        double xm = (double)xl + (double)dl;  // the refined unknown before
+        R dp = dl;
         for (int t = 0; t <= nu - 2; ++t) {
           const size_t o = (size_t)(q0 + t) * L + l;
           const R d = sD[o] - sA[o] * dp - sC[o] * dr;
-          const double x = (double)sc_y[o] + (double)d;
-          if constexpr (Gen::AUX != 0) ax = scr[Gen::AUX * UL + o];
-          E.template emit<true>(G, LS, sh.xlast[l], q0 + t, x, xm, ax);
+          E.template emit<true>(G, LS, sh.xlast[l], q0 + t, (double)sc_y[o] + (double)d, 0.0, R(0));
           dp = d;
-          xm = x;
         }
-        if (nu >= 1) {
-          if constexpr (Gen::AUX != 0) ax = scr[Gen::AUX * UL + (size_t)(q0 + nu - 1) * L + l];
-          E.template emit<true>(G, LS, sh.xlast[l], q0 + nu - 1, (double)xr + (double)dr, xm, ax);
-        }
+        if (nu >= 1)
+          E.template emit<true>(G, LS, sh.xlast[l], q0 + nu - 1, (double)xr + (double)dr, 0.0, R(0));
       }
     }
     __syncthreads();

@@ -15,9 +15,9 @@
 // rounds (four arrays, six rows, three rounds: 0.107 ms, hydraulic). The solve
 // itself is a tenth of the time, the rounds of loads half (ablation). On
 // 2048x1024, from the chunks in global memory: hydraulic y sweep 0.148 ->
-// 0.080 ms in FP64, 0.111 -> 0.065 in FP32, 0.153 -> 0.077 refined; the
+// 0.080 ms (FP64; the FP32 forms' has its own solver, pairgen.cuh); the
 // concentration y sweep, whose rows a per-cell kernel wrote to four arrays
-// first, 0.126 -> 0.084, 0.079 -> 0.062, 0.108 -> 0.072.
+// first, 0.126 -> 0.084 in FP64, 0.079 -> 0.062 in FP32, 0.108 -> 0.072 refined.
 //
 // REFINE: the rows stay in shared memory as they are; the residual is taken
 // in FP64 and the correction solved from them again.

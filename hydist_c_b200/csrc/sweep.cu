@@ -1,5 +1,6 @@
 // sweep.cu -- the ADI line sweeps: what they solve, and which solver takes them.
 //
+// The FP64 form's hydraulic sweeps (the FP32 forms': pairgen.cuh).
 // HydroGen<0> is the x sweep (UZ half-step: lines are columns j, cells run
 // along i, unknowns u_i); HydroGen<1> is the y sweep (VZ half-step: lines are
 // rows i, cells along j, unknowns v_j). Both generate the rows of the
@@ -16,26 +17,25 @@
 #include "hydro.cuh"
 #include "colsolve.cuh"
 #include "linesolve.cuh"
+#include "pairgen.cuh"
 #include "rowsolve.cuh"
 #include "sediment_cell.cuh"
 
 namespace hyd {
 
-// REF: refine each line solve once with an FP64 residual (FP32 forms)
-template <int DIR, class R, bool REF = false>
+template <int DIR>
 struct HydroGen {
+  using R = double;
   using Real = R;
-  static constexpr bool REFINE = REF;
-  // the rows are generated from the stencils: the refinement keeps them
-  static constexpr bool ROWS_AGAIN = false;
-  // c', y', v', with refinement the rows A, B, C, D, and the emitter's value
-  static constexpr int AUX = REFINE ? 7 : 3;
+  static constexpr bool REFINE = false, ROWS_AGAIN = false;
+  static constexpr int UPC = 1;
+  static constexpr int AUX = 3;  // c', y', v', then the emitter's value
   static constexpr int SCRATCH_ARRAYS = AUX + 1;
   static constexpr bool HYDRO = true;
   static constexpr int DIRECTION = DIR;
-  // resident CTAs per SM the chunked row solver is compiled for: the FP32 rows
-  // run faster with two despite the register cap, the FP64 and refined slower
-  static constexpr int MIN_BLOCKS = sizeof(R) == 4 && !REF ? 2 : 1;
+  // resident CTAs per SM the chunked row solver is compiled for (two, with
+  // their register cap, are slower)
+  static constexpr int MIN_BLOCKS = 1;
   StateT<R> S;
   CoefT<R> c;
   R* scratch;
@@ -127,25 +127,8 @@ struct HydroGen {
   // the unknowns, and one division per cell instead of four. Ends: a solid or
   // discharge end prescribes the velocity beyond it; at an open end (level
   // given) the reference keeps the substituted f1/a2 (f3/c2) term.
-  //
-  // INC (the FP32 forms): the unknown is the velocity's change over the
-  // half-step. The row's diagonal is -2 among terms of g H (dT/dX)^2 / 2, so
-  // rounding its coefficients moves the velocity itself by a few 1e-7, its
-  // change by a few 1e-7 of the change; the right-hand side is the residual
-  // of the old velocities (vm, v0, vp; beyond a solid or discharge end the
-  // prescribed one), formed from differences. 700x300 with sediment, ten
-  // steps, largest relative error of u, v, z against 64 bits over three seeds:
-  // the interleaved system 6.4e-7 (refined 3.5e-7), velocities 7.6e-7
-  // (4.9e-7), their changes 3.6e-7 (3.6e-7), for 4 to 8 us of a 2048x1024
-  // sweep.
-  static constexpr bool INC = sizeof(R) == 4;
-  __device__ R vel_old(int g) const { return DIR == 0 ? S.u[g] : S.v[g]; }
-  // the velocity before cell pos: the one prescribed beyond the first cell
-  __device__ R before(const SegD& d, int lp, int pos, R vm) const {
-    return pos == d.first && d.ran ? (d.qfirst ? q_first(lp) : R(0)) : vm;
-  }
   __device__ void make_row(const SegD& d, int lp, int pos, MomF<R> m, R Hm, const Cont& c0,
-                           const Cont& c1, R vm, R v0, R vp, R& A, R& B, R& C, R& D) const {
+                           const Cont& c1, R& A, R& B, R& C, R& D) const {
     const R kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY, e = f4 * kk;
     const bool at0 = pos == d.first, at1 = pos == d.last - 1;
     if (d.last - 1 <= d.first) m.f1 = m.f3 = 0;  // a two-cell segment
@@ -153,15 +136,6 @@ struct HydroGen {
     B = m.f2 - 2 * e * c0.H;
     C = m.f3 + e * c1.H;
     const R dd = R(c1.z - c0.z) - (c1.w - c0.w);
-    if (INC && !(at0 && !d.ran) && !(at1 && d.last_kind == 2)) {
-      const R p = before(d, lp, pos, vm);
-      const R n = at1 ? (d.last_kind == 1 ? q_last(lp) : R(0)) : vp;
-      D = ((m.g5 + m.g2 * v0) - m.f1 * p - m.f3 * n) +
-          f4 * (dd - kk * ((Hm * p - c0.H * v0) - (c0.H * v0 - c1.H * n)));
-      if (at0) A = 0;
-      if (at1) C = 0;
-      return;
-    }
     D = m.f5 + f4 * dd;
     if (at0) {
       if (d.qfirst) {
@@ -189,23 +163,12 @@ struct HydroGen {
       }
       C = 0;
     }
-    if (INC) D -= A * vm + B * v0 + C * vp;
-  }
-  // the part of a cell's new level that does not depend on the solution, less
-  // its old level: -w, with INC also what the old velocities give
-  __device__ double level_base(const SegD& d, int lp, int pos, R Hm, const Cont& c0, R vm, R v0) const {
-    double q = -(double)c0.w;
-    if (INC) {
-      const double kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
-      q += kk * ((double)Hm * before(d, lp, pos, vm) - (double)c0.H * v0);
-    }
-    return q;
   }
 
   // a cell's operands and row for the staged row solver (rowsolve.cuh); load
   // is in bounds for every cell of the mesh, wet or not
   struct Ops {
-    R Hm, vm, v0, vp;
+    R Hm;
     Cont c0, c1;
     MomF<R> m;
   };
@@ -216,17 +179,11 @@ struct HydroGen {
     o.Hm = depth(g - s);
     o.c0 = cont(g);
     o.c1 = cont(g + s);
-    o.vm = o.v0 = o.vp = 0;
-    if (INC) {
-      o.vm = vel_old(g - s);
-      o.v0 = vel_old(g);
-      o.vp = vel_old(g + s);
-    }
     o.m = DIR == 0 ? mom_x(S, c, pos, lp) : mom_y(S, c, lp, pos);
     return o;
   }
   __device__ void row(const SegD& d, int lp, int pos, const Ops& o, R& A, R& B, R& C, R& D) const {
-    make_row(d, lp, pos, o.m, o.Hm, o.c0, o.c1, o.vm, o.v0, o.vp, A, B, C, D);
+    make_row(d, lp, pos, o.m, o.Hm, o.c0, o.c1, A, B, C, D);
   }
   // the part of a cell's new level that does not depend on the solution is
   // kept where the level goes, if the emission will write it there (nothing
@@ -235,8 +192,7 @@ struct HydroGen {
     return (pos > d.first || d.ran) && extract_ok(pos);
   }
   __device__ void keep(const SegD& d, int lp, int pos, const Ops& o) const {
-    if (level_out(d, pos))
-      S.tz[at(lp, pos)] = o.c0.z + level_base(d, lp, pos, o.Hm, o.c0, o.vm, o.v0);
+    if (level_out(d, pos)) S.tz[at(lp, pos)] = o.c0.z - o.c0.w;
   }
   __device__ void prefetch(int lp) const {
     const int w = S.W;
@@ -260,18 +216,18 @@ struct HydroGen {
     if (!extract_ok(pos)) return;
     R* v = vel_ptr();
     if (pos < d.last) {
-      const R x = INC ? (double)vel_old(g) + value(pos) : value(pos);
+      const R x = value(pos);
       v[g] = x;
       if (level_out(d, pos)) {
-        const double xm = pos > d.first ? value(pos - 1) : (!INC && d.qfirst ? (double)q_first(lp) : 0.0);
-        const double kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
-        S.tz[g] = S.tz[g] + kk * ((double)depth(g - s) * xm - (double)depth(g) * value(pos));
+        const R xm = pos > d.first ? value(pos - 1) : (d.qfirst ? q_first(lp) : 0.0);
+        const R kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
+        S.tz[g] = S.tz[g] + kk * (depth(g - s) * xm - depth(g) * x);
       }
       if (pos == d.first) end_first(d, lp, x);
     } else {
       const bool two = d.last > d.first;
-      const double x = two ? (INC ? (double)vel_old(g - s) : 0.0) + value(pos - 1) : 0.0;
-      end_last(d, lp, x, two ? (R)x : v[g - s]);
+      const R x = two ? value(pos - 1) : 0.0;
+      end_last(d, lp, x, two ? x : v[g - s]);
     }
   }
 
@@ -279,8 +235,7 @@ struct HydroGen {
   struct Walker {
     int lp, si, pos, prev;
     bool in;
-    R Hm, aux;  // depth before c0; what the emitter needs to form the level
-    R vm, v0, vp;
+    R Hm, aux;  // depth before c0; the level without the solution's part
     Cont c0, c1;
     MomF<R> m;
     __device__ void init(const HydroGen& G, const LineSeg& LS, int line, int first_cell) {
@@ -300,58 +255,37 @@ struct HydroGen {
       if (prev == pos - 1) {
         Hm = c0.H;
         c0 = c1;
-        vm = v0;
-        v0 = vp;
       } else {
         Hm = G.depth(G.at(lp, pos - 1));
         c0 = G.cont(G.at(lp, pos));
-        vm = INC ? G.vel_old(G.at(lp, pos - 1)) : R(0);
-        v0 = INC ? G.vel_old(G.at(lp, pos)) : R(0);
       }
       c1 = G.cont(G.at(lp, pos + 1));
-      vp = INC ? G.vel_old(G.at(lp, pos + 1)) : R(0);
       m = DIR == 0 ? mom_x(G.S, G.c, pos, lp) : mom_y(G.S, G.c, lp, pos);
       prev = pos;
-      aux = sizeof(R) == 8 ? R(c0.z - c0.w) : R(G.level_base(LS.s[si], lp, pos, Hm, c0, vm, v0));
+      aux = c0.z - c0.w;
     }
-    __device__ void row(const HydroGen& G, const LineSeg& LS, R& A, R& B, R& C, R& D) const {
+    __device__ void row(const HydroGen& G, const LineSeg& LS, int, R& A, R& B, R& C, R& D) const {
       if (!in) {
         A = 0; B = 1; C = 0; D = 0;
         return;
       }
-      G.make_row(LS.s[si], lp, pos, m, Hm, c0, c1, vm, v0, vp, A, B, C, D);
+      G.make_row(LS.s[si], lp, pos, m, Hm, c0, c1, A, B, C, D);
     }
   };
 
-  // (the refinement reads the stored rows: no cursor over them)
-  struct RowCursor {
-    __device__ void init(const HydroGen&, const LineSeg&, int) {}
-    __device__ void row(const HydroGen&, const LineSeg&, int, R&, R&, R&, R&) {}
-  };
-
   // Writes each solved velocity and its cell's level to t_u (t_v) / t_z as
-  // the extraction does. FWD: the unknowns come in increasing order
-  // (init_fwd), else decreasing.
+  // the extraction does; the unknowns come in decreasing order.
   struct Emitter {
     int lp, si;
     __device__ void init(const HydroGen& G, const LineSeg& LS, int line) {
       lp = line + G.lp0;
       si = LS.nseg - 1;
     }
-    __device__ void init_fwd(const HydroGen& G, const LineSeg& LS, int line) {
-      lp = line + G.lp0;
-      si = -1;
-    }
     // unknown q with value x, the one before it xm, its cell's aux
-    template <bool FWD = false>
     __device__ void emit(const HydroGen& G, const LineSeg& LS, double* xlast, int q, double x,
                          double xm, R aux) {
       const int pos = q + 2;
-      if constexpr (FWD) {
-        while (si + 1 < LS.nseg && LS.s[si + 1].first <= pos) ++si;
-      } else {
-        while (si >= 0 && LS.s[si].first > pos) --si;
-      }
+      while (si >= 0 && LS.s[si].first > pos) --si;
       if (si < 0) return;
       G.store_in(LS.s[si], xlast + si, lp, pos, x, xm, aux);
     }
@@ -360,21 +294,18 @@ struct HydroGen {
   // The extraction of the velocity x of cell pos of segment d on line position
   // lp, and of the cell's level by continuity (the first cell's where it is
   // not given); the segment's last velocity also goes to *xl for the end
-  // fix-up. aux: the level without the solution's part, in FP32 less the old
-  // level (which stays FP64).
+  // fix-up. aux: the level without the solution's part.
   __device__ void store_in(const SegD& d, double* xl, int lp, int pos, double x, double xm,
                            R aux) const {
     if (pos >= d.last) return;
     const int g = at(lp, pos);
-    const double xn = INC ? (double)vel_old(g) + x : x;
-    if (pos == d.last - 1) *xl = xn;
+    if (pos == d.last - 1) *xl = x;
     if (!extract_ok(pos)) return;
-    vel_ptr()[g] = xn;
+    vel_ptr()[g] = x;
     if (pos > d.first || d.ran) {
-      if (pos == d.first) xm = !INC && d.qfirst ? (double)q_first(lp) : 0.0;
-      const double kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
-      const double base = sizeof(R) == 8 ? (double)aux : S.z[g] + (double)aux;
-      S.tz[g] = base + kk * ((double)depth(DIR == 0 ? g - S.W : g - 1) * xm - (double)depth(g) * x);
+      if (pos == d.first) xm = d.qfirst ? q_first(lp) : 0.0;
+      const R kk = DIR == 0 ? c.dTchia2dX : c.dTchia2dY;
+      S.tz[g] = aux + kk * (depth(DIR == 0 ? g - S.W : g - 1) * xm - depth(g) * x);
     }
   }
 
@@ -540,8 +471,8 @@ static void launch_rows(const Gen& G, int ncells, int lines, cudaStream_t st,
 // The staged column solver takes columns of up to COL_MAX cells, a 32-byte
 // sector of them per CTA (4 in FP64 and refined, 8 in FP32; up to 8800 cells
 // and 106 KB). Hydraulic x sweep, chunked -> staged: 64x32 50 -> 13 us,
-// 256x128 31 -> 19, 512x256 32 -> 23, 1024x512 58 -> 42 (FP64; FP32 44 -> 37,
-// refined 54 -> 39); at 2048x1024 its 196 KB of rows in one CTA per SM lose
+// 256x128 31 -> 19, 512x256 32 -> 23, 1024x512 58 -> 42 (FP64); at 2048x1024 its
+// 196 KB of rows in one CTA per SM lose
 // (111 -> 220, two columns per CTA 168), so longer columns keep the chunks.
 constexpr int COL_MAX = 1100;
 template <class Gen>
@@ -623,9 +554,67 @@ static int launch_lines(const Gen& G, int ncells, int lines, cudaStream_t st,
   }
 }
 
-template <int DIR, class R, bool REF>
-static int launch_dir(const StateT<R>& S, const CoefT<R>& c, cudaStream_t st, const Batch<R>& b) {
-  HydroGen<DIR, R, REF> G;
+// The FP32 forms' hydraulic sweeps: chunks per line, as many as keep at least
+// four cells per chunk (of 128, 64, 32, 16, 4 or 1), so that no chunk of a short
+// line is empty or holds its separator alone.
+static int pair_chunks(int ncells) {
+  int P = 128;
+  while (P > 1 && ncells < P * 4) P >>= 1;
+  return P == 8 ? 4 : P == 2 ? 1 : P;
+}
+
+// Groups of L lines of P chunks, a CTA each; a group of eight takes two of the
+// scratch's 4-line slots. The scratch holds StateT::lslots slots of lines of
+// 2*max(M, N) unknowns, so a sweep of shorter lines has proportionally more.
+// Only the solvers of fewer than 128 chunks (smaller CTAs, more of them resident
+// per SM) use them: their grid may then exceed the CTAs resident at once. (For
+// the 128-chunk solvers the persistent grid of lslots CTAs measured as fast or
+// faster.)
+template <class Gen, int P, int L>
+static int launch_pairs_p(const Gen& G, int ncells, int chunks, cudaStream_t st, const Batch<float>& b) {
+  const int groups = cdiv(G.nl, L);
+  const long long total = (long long)groups * std::max(b.n, 1);
+  int slots = G.S.lslots;
+  if (chunks < 128) slots *= std::max(1, std::max(G.S.M, G.S.N) / ncells);
+  launch_gen<Gen, P, L>(G, st, (int)std::min<long long>(total, slots * LPB / L), 0, (int)total, b,
+                        b.n > 0 ? groups : 0);
+  return 1;
+}
+
+// Groups of eight lines where a line has 64 or 128 chunks (columns 64: only
+// refined), else of four. On 2048x1024 (128 chunks of columns and rows), four ->
+// eight: x refined 0.216 -> 0.154 ms, y 0.130 -> 0.121; the refined rows, alone, as
+// 64 chunks 0.210 -> 0.204 (as 128 in a batch).
+template <int DIR, bool REF>
+static int launch_pairs(const StateT<float>& S, const CoefT<float>& c, cudaStream_t st,
+                        const Batch<float>& b) {
+  using Gen = PairGen<DIR, REF>;
+  Gen G;
+  G.bind(S, c);
+  G.scratch = S.lscratch;
+  G.lp0 = DIR == 0 ? S.x_lo : S.y_lo;
+  G.nl = DIR == 0 ? S.x_hi - S.x_lo + 1 : S.N - S.y_lo + 1;
+  if (G.nl <= 0) return 0;
+  const int ncells = DIR == 0 ? S.N - 1 : S.M - 1, P = pair_chunks(ncells);
+  switch (P) {
+    case 128:
+      if constexpr (DIR == 1 && REF) {
+        if (b.n > 0) return launch_pairs_p<Gen, 128, LPB>(G, ncells, P, st, b);
+        return launch_pairs_p<Gen, 64, XPB>(G, ncells, P, st, b);
+      } else {
+        return launch_pairs_p<Gen, 128, XPB>(G, ncells, P, st, b);
+      }
+    case 64: return launch_pairs_p<Gen, 64, (DIR == 1 || REF) ? XPB : LPB>(G, ncells, P, st, b);
+    case 32: return launch_pairs_p<Gen, 32, LPB>(G, ncells, P, st, b);
+    case 16: return launch_pairs_p<Gen, 16, LPB>(G, ncells, P, st, b);
+    case 4: return launch_pairs_p<Gen, 4, LPB>(G, ncells, P, st, b);
+    default: return launch_pairs_p<Gen, 1, LPB>(G, ncells, P, st, b);
+  }
+}
+
+template <int DIR>
+static int launch_dir(const State& S, const Coef& c, cudaStream_t st, const Batch<double>& b) {
+  HydroGen<DIR> G;
   G.bind(S, c);
   G.scratch = S.lscratch;
   G.lp0 = DIR == 0 ? S.x_lo : S.y_lo;
@@ -647,6 +636,7 @@ struct FSGen {
   static constexpr bool ROWS_AGAIN = true;
   static constexpr int AUX = 0;  // the emitter needs nothing but the solution
   static constexpr int SCRATCH_ARRAYS = REFINE ? 4 : 3;
+  static constexpr int UPC = 1;
   static constexpr bool HYDRO = false;
   static constexpr int DIRECTION = DIR;
   static constexpr int MIN_BLOCKS = 2;  // in both precisions
@@ -760,7 +750,7 @@ struct FSGen {
       while (si < LS.nseg && LS.s[si].last < pos) ++si;
       in = si < LS.nseg && LS.s[si].off <= pos && pos <= LS.s[si].rend;
     }
-    __device__ void row(const FSGen& G, const LineSeg& LS, R& A, R& B, R& C, R& D) const {
+    __device__ void row(const FSGen& G, const LineSeg& LS, int, R& A, R& B, R& C, R& D) const {
       if (!in) {
         A = 0; B = 1; C = 0; D = 0;
         return;
@@ -888,14 +878,15 @@ int launch_fs_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t
 template <class R>
 int launch_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t st,
                  const Batch<R>& b) {
-  if constexpr (sizeof(R) == 4) {  // (the refinement is of the FP32 form)
-    if (S.refine) {
-      if (dir == 0) return launch_dir<0, R, true>(S, c, st, b);
-      return launch_dir<1, R, true>(S, c, st, b);
-    }
+  if constexpr (sizeof(R) == 4) {
+    if (S.refine && dir == 0) return launch_pairs<0, true>(S, c, st, b);
+    if (S.refine) return launch_pairs<1, true>(S, c, st, b);
+    if (dir == 0) return launch_pairs<0, false>(S, c, st, b);
+    return launch_pairs<1, false>(S, c, st, b);
+  } else {
+    if (dir == 0) return launch_dir<0>(S, c, st, b);
+    return launch_dir<1>(S, c, st, b);
   }
-  if (dir == 0) return launch_dir<0, R, false>(S, c, st, b);
-  return launch_dir<1, R, false>(S, c, st, b);
 }
 
 template bool fs_rows_in_sweep<double>(const StateT<double>&, int);
