@@ -95,8 +95,8 @@ __device__ __forceinline__ void cols_reduce(const ChunkEnds<T>& e, ColShared<T, 
 }
 
 // cta_solve of L interleaved systems of n rows each
-template <class T, int NT, int L, class Row>
-__device__ __forceinline__ void cols_solve(T* oV, T* oC, T* X, int n, ColShared<T, NT, L>& sh, Row row) {
+template <class T, int NT, int L, class W, class Row>
+__device__ __forceinline__ void cols_solve(T* oV, T* oC, T* X, int n, ColShared<W, NT, L>& sh, Row row) {
   const int l = threadIdx.x % L, t = threadIdx.x / L;
   int S = (n + NT / L - 1) / (NT / L);
   S = (S < 3 ? 3 : S) | 1;
@@ -123,8 +123,9 @@ __device__ __forceinline__ void cols_solve(T* oV, T* oC, T* X, int n, ColShared<
   e.yL = yp;
   e.vL = vp;
   e.wL = -cp;
-  T x, xl;
-  cols_reduce<T, NT, L>(e, sh, x, xl);
+  W wx, wxl;
+  cols_reduce<W, NT, L>(ends_as<W>(e), sh, wx, wxl);
+  const T x = (T)wx, xl = (T)wxl;
   if (nu > 0) {
     X[(q0 + nu - 1) * L + l] = x;
     T xn = x;
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT < 1 ? 1 : (sizeof(typename Gen::
   using R = typename Gen::Real;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LineSeg seg[L];
-  __shared__ ColShared<R, NT, L> sh;
+  __shared__ ColShared<reduce_t<Gen>, NT, L> sh;
   auto solve = [&](const Gen& G) {
     const int tid = threadIdx.x, nc = G.cells_per_line(), l = tid % L, r0 = tid / L;
     const int line = blockIdx.x * L + l;

@@ -143,6 +143,12 @@ struct ChunkEnds {
   T yF = 0, vF = 0, wF = 1, yL = 0, vL = 0, wL = 0;
 };
 
+// the same in another type
+template <class W, class T>
+__device__ __forceinline__ ChunkEnds<W> ends_as(const ChunkEnds<T>& e) {
+  return ChunkEnds<W>{(W)e.as, (W)e.bs, (W)e.cs, (W)e.ds, (W)e.yF, (W)e.vF, (W)e.wF, (W)e.yL, (W)e.vL, (W)e.wL};
+}
+
 // Eliminates rows q0 .. q0 + nu - 1 (row(q, A, B, C, D) gives row q); where KEEP,
 // (v', c', y') go to oV, oC, oY, which may be the rows' own arrays.
 template <bool KEEP, class T, class Row>
@@ -299,15 +305,17 @@ __device__ __forceinline__ void tile_reduce(const ChunkEnds<T>& e, T (*blk)[8], 
 
 // The partition solve of n rows in shared memory by the NT threads of a CTA,
 // the solution in X: row(q, A, B, C, D) gives row q, (v', c') are kept in oV and
-// oC (all three may be the rows' own A, C, D arrays).
-template <class T, int NT, class Row>
-__device__ __forceinline__ void cta_solve(T* oV, T* oC, T* X, int n, T (*blk)[8], Row row) {
+// oC (all three may be the rows' own A, C, D arrays). The reduction is done in
+// blk's type W.
+template <class T, int NT, class W, class Row>
+__device__ __forceinline__ void cta_solve(T* oV, T* oC, T* X, int n, W (*blk)[8], Row row) {
   const int tid = threadIdx.x, S = bulk_chunk(n, NT), P = max(1, n / S);
   const int q0 = tid * S;
   const int nu = tid < P ? (tid == P - 1 ? n - q0 : S) : 0;
   const ChunkEnds<T> e = chunk_forward<true>(oV, oC, X, q0, nu, row);
-  T x, xl;
-  tile_reduce<T, NT, true>(e, blk, x, xl, nullptr);
+  W wx, wxl;
+  tile_reduce<W, NT, true>(ends_as<W>(e), blk, wx, wxl, nullptr);
+  const T x = (T)wx, xl = (T)wxl;
   if (nu > 0) {
     X[q0 + nu - 1] = x;
     T xn = x;

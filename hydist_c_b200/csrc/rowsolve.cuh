@@ -24,6 +24,7 @@
 #pragma once
 
 #include <climits>
+#include <type_traits>
 
 #include "common.cuh"
 #include "linesolve.cuh"
@@ -39,6 +40,15 @@ template <class Gen>
 constexpr bool row_normal() {
   return sizeof(typename Gen::Real) == 8;
 }
+
+// The separators' reduction of the plain FP32 form is done in FP64: its levels are
+// what the chunks in global memory did not have as many of, and in FP32 they
+// added to the result's error (the concentration against 64 bits after 20 steps of
+// 64x32 1.0e-7 -> 1.9e-7 of its norm, 256x128 1.3e-7 -> 1.6e-7; so 0.8e-7 and
+// 1.0e-7), for no time that shows: 64 against 62..64 us, 2048x1024. (The refined
+// form's correction takes the error out anyway.)
+template <class Gen>
+using reduce_t = std::conditional_t<Gen::REFINE, typename Gen::Real, double>;
 
 // arrays of a row's cells in shared memory: a, c, d or A, C, D, B; with
 // refinement also v', c' and the first solution
@@ -98,7 +108,7 @@ __global__ void __launch_bounds__(NT, row_min_blocks<typename Gen::Real, NT>())
   using R = typename Gen::Real;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LineSeg LS;
-  __shared__ R blk[NT / 32 + 1][8];
+  __shared__ reduce_t<Gen> blk[NT / 32 + 1][8];
   auto solve = [&](const Gen& G) {
     const int tid = threadIdx.x, nc = G.cells_per_line(), lp = G.line_pos(blockIdx.x);
     R* rA = reinterpret_cast<R*>(smem_raw);
