@@ -141,6 +141,7 @@ struct HydistHandle {
   cudaGraphExec_t graph[8] = {};
   long long graph_launches[8] = {};
   int eager_steps[8] = {};  // of hydist_step, before it captures the phase
+  bool no_capture = false;  // a capture of hydist_step's failed: it launches from then on
   Trace trace;                                    // kernel launch counter
   cudaEvent_t ev[PH_COUNT + 1] = {};
   cudaEvent_t kev[2 * KS_COUNT] = {};
@@ -1005,24 +1006,29 @@ Phase3 next_phase(const HydistHandle* h) {
   return Phase3{t1 >= h->o.sediment_start, t2 >= h->o.sediment_start, bed_on(h, t2), t2};
 }
 
-// One step by its phase's graph (the time advances on the device, so the
-// launches of a step are the same every step), captured on first use.
-int graph_step(HydistHandle* h, const Phase3& ph) {
+// The graph of a phase's step (the time advances on the device, so the launches
+// of a step are the same every step), captured on first use.
+int phase_graph(HydistHandle* h, const Phase3& ph) {
   const int gi = ph.index();
   cudaGraphExec_t& ex = h->graph[gi];
-  if (!ex) {
-    cudaGraph_t g = nullptr;
-    Trace tr;
-    CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    enqueue_step(h, ph.sx, ph.sy, ph.bd, &tr);
-    CK(cudaStreamEndCapture(h->stream, &g));
-    h->graph_launches[gi] = tr.launches;
-    const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
-    cudaGraphDestroy(g);
-    CK(e);
-  }
-  CK(cudaGraphLaunch(ex, h->stream));
-  h->trace.launches += h->graph_launches[gi];
+  if (ex) return HYDIST_OK;
+  cudaGraph_t g = nullptr;
+  Trace tr;
+  CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+  enqueue_step(h, ph.sx, ph.sy, ph.bd, &tr);
+  CK(cudaStreamEndCapture(h->stream, &g));
+  h->graph_launches[gi] = tr.launches;
+  const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) ex = nullptr;
+  CK(e);
+  return HYDIST_OK;
+}
+
+int graph_step(HydistHandle* h, const Phase3& ph) {
+  TRY(phase_graph(h, ph));
+  CK(cudaGraphLaunch(h->graph[ph.index()], h->stream));
+  h->trace.launches += h->graph_launches[ph.index()];
   h->t = ph.t2;
   return HYDIST_OK;
 }
@@ -1036,7 +1042,8 @@ extern "C" {
 // step, 132 us by graph): from the eighth step of a phase on, or at once where
 // the call still has eight of them to go (what the capture then costs is
 // less than they save), hydist_step replays the phase's graph too. A caller
-// that captures the handle's stream itself gets the launches.
+// that captures the handle's stream itself gets the launches, and so does one
+// whose step cannot be captured (no memory for the graph, say).
 int hydist_step(HydistHandle* h, int32_t nsteps) {
   if (!h) return fail(HYDIST_ERR_ARG, "null handle");
   if (h->next_half) return fail(HYDIST_ERR_STATE, "the second half-step is pending");
@@ -1049,10 +1056,14 @@ int hydist_step(HydistHandle* h, int32_t nsteps) {
   for (int k = 0; k < nsteps; ++k) {
     const Phase3 ph = next_phase(h);
     const int gi = ph.index();
-    if (cap == cudaStreamCaptureStatusNone &&
+    if (cap == cudaStreamCaptureStatusNone && !h->no_capture &&
         (h->graph[gi] || nsteps - k >= kCapture || h->eager_steps[gi] >= kCapture)) {
-      TRY(graph_step(h, ph));
-      continue;
+      if (phase_graph(h, ph) == HYDIST_OK) {
+        TRY(graph_step(h, ph));
+        continue;
+      }
+      h->no_capture = true;
+      cudaGetLastError();  // (of the capture; the launches below report their own)
     }
     ++h->eager_steps[gi];
     enqueue_step(h, ph.sx, ph.sy, ph.bd, &h->trace);

@@ -228,7 +228,8 @@ int hydist_create_external(const HydistExternal* ext, const HydistParams* p,
  * loop of Hydraulic_Calculation (engine.cpp:65-295). Stream-ordered on the
  * handle's stream; returns once the work is enqueued. Steps of a call of eight
  * or more, and those after eight single ones, replay a CUDA graph of the step
- * that the first of them captures (except inside a capture of the caller's). */
+ * that the first of them captures (except inside a capture of the caller's, and
+ * where the graph cannot be made: those are launched kernel by kernel). */
 int hydist_step(HydistHandle* h, int32_t nsteps);
 
 /* One half of a step: half 0 = t += dT/2, the x sweep (UZ), explicit v,

@@ -1,0 +1,64 @@
+"""Host calls of the CUDA runtime that fail (a preloaded fake returns the error
+code; no GPU work is involved): what the library makes of them."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    so = tmp_path_factory.mktemp("shim") / "fail_calls.so"
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", str(so),
+                    str(ROOT / "tests" / "native" / "fail_calls.c"), "-ldl"], check=True)
+    return so
+
+
+def _child(shim, call, code):
+    env = dict(os.environ, LD_PRELOAD=str(shim), FAIL_CALL=call, PYTHONPATH=str(ROOT))
+    head = f"import ctypes\nfail = ctypes.CDLL({str(shim)!r})\n"
+    r = subprocess.run([sys.executable, "-c", head + code], env=env, cwd=ROOT, capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "all well" in r.stdout
+
+
+@pytest.mark.gpu
+def test_step_launches_where_its_graph_cannot_be_made(shim):
+    """hydist_step of eight steps and more goes on launch by launch, with the
+    same result; hydist_step_graph, which promises the graph, reports it."""
+    _child(shim, "cudaGraphInstantiate", """
+import numpy as np
+import hydist_c_b200 as H
+from hydist_c_b200 import scenario as S
+b = S.make_channel(N=40, M=33, seed=11, dx=10.0, inflow=5.0 * 33)
+a, c = H.Simulation(b), H.Simulation(b)
+for _ in range(20):
+    a.half_step(0); a.half_step(1)
+a.sync()
+fail.fail_calls_left(1 << 20)
+c.step(12)
+for _ in range(7):
+    c.step(1)
+assert fail.fail_calls_failed() >= 1
+n = fail.fail_calls_failed()
+try:
+    c.step_graph(1)
+    raise SystemExit("no error")
+except H.HydistError:
+    pass
+assert fail.fail_calls_failed() == n + 1
+c.step(1)
+c.sync()
+assert c.t == a.t, (c.t, a.t)
+for f in ("u", "v", "z"):
+    assert np.array_equal(a.download(f), c.download(f)), f
+fail.fail_calls_left(0)
+c.step_graph(2)
+c.sync()
+print("all well")
+""")
