@@ -1015,14 +1015,28 @@ int ensure_scratch(DevScratch& s, size_t w_bytes, size_t nsys, size_t flag_bytes
     if (cudaMalloc(&s.lists, (size_t)hyd::GT_NC * nsys * sizeof(int)) != cudaSuccess) return HYDIST_ERR_OOM;
     s.lists_cap = nsys;
   }
+  // each on its own: what one call could not have, the next one asks for again
   if (!s.counts) {
     const size_t bytes = 2 * (hyd::GT_COUNTS + 1) * sizeof(int);
-    if (cudaMalloc(&s.counts, bytes) != cudaSuccess) return HYDIST_ERR_OOM;
-    if (cudaMemset(s.counts, 0, bytes) != cudaSuccess) return HYDIST_ERR_CUDA;
-    if (cudaHostAlloc((void**)&s.host, (hyd::GT_COUNTS + 1) * sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void**)&s.host_dev, s.host, 0) != cudaSuccess)
+    int* p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) return HYDIST_ERR_OOM;
+    if (cudaMemset(p, 0, bytes) != cudaSuccess) {
+      cudaFree(p);
       return HYDIST_ERR_CUDA;
-    s.host[hyd::GT_STALLED] = 0;
+    }
+    s.counts = p;
+  }
+  if (!s.host_dev) {
+    int *p = nullptr, *dp = nullptr;
+    if (cudaHostAlloc((void**)&p, (hyd::GT_COUNTS + 1) * sizeof(int), cudaHostAllocMapped) != cudaSuccess)
+      return HYDIST_ERR_OOM;
+    if (cudaHostGetDevicePointer((void**)&dp, p, 0) != cudaSuccess) {
+      cudaFreeHost(p);
+      return HYDIST_ERR_CUDA;
+    }
+    p[hyd::GT_STALLED] = 0;
+    s.host = p;
+    s.host_dev = dp;
   }
   return HYDIST_OK;
 }

@@ -62,3 +62,33 @@ c.step_graph(2)
 c.sync()
 print("all well")
 """)
+
+
+@pytest.mark.gpu
+def test_batched_solver_after_a_failed_allocation(shim):
+    """A first batch whose counts' host memory could not be had reports that;
+    the next batch asks again and is solved."""
+    _child(shim, "cudaHostAlloc", """
+import numpy as np, torch
+import hydist_c_b200 as H
+from hydist_c_b200 import scenario as S
+*rows, off, ln = S.tridiag_batch(lengths=np.array([5, 300, 900, 7000]), seed=3)
+t = [torch.from_numpy(v).cuda() for v in rows]
+off, ln = torch.from_numpy(off).cuda(), torch.from_numpy(ln).cuda()
+fail.fail_calls_left(1)
+try:
+    H.gtsv_batched(*t, off, ln)
+    raise SystemExit("no error")
+except H.HydistError:
+    pass
+assert fail.fail_calls_failed() == 1
+x = H.gtsv_batched(*t, off, ln)
+a, d, c, b = t
+r = d * x - b
+for s in range(4):
+    o, n = int(off[s]), int(ln[s])
+    r[o + 1:o + n] += a[o + 1:o + n] * x[o:o + n - 1]
+    r[o:o + n - 1] += c[o:o + n - 1] * x[o + 1:o + n]
+assert float(r.abs().max()) < 1e-13 * float(b.abs().max().clamp(min=1)), float(r.abs().max())
+print("all well")
+""")
