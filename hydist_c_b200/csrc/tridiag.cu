@@ -1070,18 +1070,12 @@ bool staged_algo(int a) {
          a == GTSV_TILES || a == GTSV_WARP_BULK;
 }
 
-// one batched solve with a given solver per band (table[b])
+// one batched solve with a given solver per band (table[b]), the scratch at hand
 template <class T>
-int solve_batch(const T* dl, const T* d, const T* du, const T* b, T* x, const int* off,
-                const int* len, int nsys, const int table[GT_NB], DevInfo& D, cudaStream_t st) {
+int solve_on(const T* dl, const T* d, const T* du, const T* b, T* x, const int* off,
+             const int* len, int nsys, const int table[GT_NB], DevInfo& D, cudaStream_t st) {
   using hyd::GT_NC;
-  int rc = ensure_scratch(D.scr, 0, (size_t)nsys);
-  if (rc != HYDIST_OK) return rc;
-  if (!D.done && cudaEventCreateWithFlags(&D.done, cudaEventDisableTiming) != cudaSuccess)
-    return HYDIST_ERR_CUDA;
-  // an earlier batch may still run on another stream
-  if (cudaStreamWaitEvent(st, D.done, 0) != cudaSuccess) return HYDIST_ERR_CUDA;
-  rc = classify(D.scr, off, len, nsys, st);
+  int rc = classify(D.scr, off, len, nsys, st);
   if (rc != HYDIST_OK) return rc;
   const int* counts = D.scr.host;
   // the CTA solvers stage rows with bulk copies, which need 16-byte aligned
@@ -1155,7 +1149,6 @@ int solve_batch(const T* dl, const T* d, const T* du, const T* b, T* x, const in
       return HYDIST_ERR_CUDA;
     if (rc != HYDIST_OK) return rc;
   }
-  if (cudaEventRecord(D.done, st) != cudaSuccess) return HYDIST_ERR_CUDA;
   if (staged) {
     // a CTA whose staging copy never completed left systems unsolved: read
     // its flag now, so that this batch, not a later one, reports it
@@ -1167,6 +1160,21 @@ int solve_batch(const T* dl, const T* d, const T* du, const T* b, T* x, const in
     }
   }
   return HYDIST_OK;
+}
+
+// A batch waits for the one before it, on whatever stream, and leaves the event
+// that the next one waits for: on every way out, an error's too, since some of its
+// classes may have been launched by then.
+template <class T>
+int solve_batch(const T* dl, const T* d, const T* du, const T* b, T* x, const int* off,
+                const int* len, int nsys, const int table[GT_NB], DevInfo& D, cudaStream_t st) {
+  if (!D.done && cudaEventCreateWithFlags(&D.done, cudaEventDisableTiming) != cudaSuccess)
+    return HYDIST_ERR_CUDA;
+  if (cudaStreamWaitEvent(st, D.done, 0) != cudaSuccess) return HYDIST_ERR_CUDA;
+  int rc = ensure_scratch(D.scr, 0, (size_t)nsys);
+  if (rc == HYDIST_OK) rc = solve_on<T>(dl, d, du, b, x, off, len, nsys, table, D, st);
+  if (cudaEventRecord(D.done, st) != cudaSuccess && rc == HYDIST_OK) rc = HYDIST_ERR_CUDA;
+  return rc;
 }
 
 template <class T>

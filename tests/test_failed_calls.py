@@ -92,3 +92,38 @@ for s in range(4):
 assert float(r.abs().max()) < 1e-13 * float(b.abs().max().clamp(min=1)), float(r.abs().max())
 print("all well")
 """)
+
+
+@pytest.mark.gpu
+def test_batch_after_one_that_failed_halfway(shim):
+    """A batch that fails with some of its classes launched: the next one, on
+    another stream, waits for those before it uses the scratch again."""
+    _child(shim, "cudaStreamWaitEvent", """
+import numpy as np, torch
+import hydist_c_b200 as H
+from hydist_c_b200 import scenario as S
+def batch(lens, seed):
+    *rows, off, ln = S.tridiag_batch(lengths=np.array(lens), seed=seed)
+    return [torch.from_numpy(v).cuda() for v in rows] + [torch.from_numpy(off).cuda(), torch.from_numpy(ln).cuda()]
+one, two = batch([7000] * 300 + [900] * 400 + [300] * 400, 3), batch([40] * 5000 + [700] * 900, 4)
+want = H.gtsv_batched(*two).clone()
+st = [torch.cuda.Stream(), torch.cuda.Stream()]
+torch.cuda.synchronize()
+for _ in range(4):
+    x = torch.full_like(want, float("nan"))
+    torch.cuda.synchronize()
+    # calls: the earlier batch, then the fork and the join of each class
+    fail.fail_calls_after(3)
+    n = fail.fail_calls_failed()
+    try:
+        with torch.cuda.stream(st[0]):
+            H.gtsv_batched(*one)
+        raise SystemExit("no error")
+    except H.HydistError:
+        assert fail.fail_calls_failed() == n + 1
+    with torch.cuda.stream(st[1]):
+        H.gtsv_batched(*two, x=x)
+    torch.cuda.synchronize()
+    assert torch.equal(x, want)
+print("all well")
+""")
