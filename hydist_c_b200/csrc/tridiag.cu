@@ -17,7 +17,7 @@
 //               in shared memory by TMA bulk copies (the next system's while
 //               one is solved, where two fit), partition method over chunks,
 //               warps and the CTA (systems up to the shared memory of one
-//               CTA, about 6000 FP64 / 12000 FP32 rows);
+//               CTA: 6144 rows of either type, the highest class);
 //   tiles       longer systems cut into tiles of one CTA each: a pass that
 //               reduces every tile to its last row, a small solve of those
 //               rows per system, a pass that solves the tiles.
@@ -1070,10 +1070,12 @@ bool staged_algo(int a) {
          a == GTSV_TILES || a == GTSV_WARP_BULK;
 }
 
-// one batched solve with a given solver per band (table[b]), the scratch at hand
+// one batched solve with a given solver per band (table[b]), the scratch at hand;
+// warp_asked: the caller named the warp solver (AUTO may stage for it instead)
 template <class T>
 int solve_on(const T* dl, const T* d, const T* du, const T* b, T* x, const int* off,
-             const int* len, int nsys, const int table[GT_NB], DevInfo& D, cudaStream_t st) {
+             const int* len, int nsys, const int table[GT_NB], bool warp_asked, DevInfo& D,
+             cudaStream_t st) {
   using hyd::GT_NC;
   int rc = classify(D.scr, off, len, nsys, st);
   if (rc != HYDIST_OK) return rc;
@@ -1115,13 +1117,12 @@ int solve_on(const T* dl, const T* d, const T* du, const T* b, T* x, const int* 
   // (k_gtsv_warp) keep the load units busy: 16384 systems on a B200, a call on
   // a cold cache, FP64 / FP32: 257..512 rows 164 -> 92 us / 106 -> 74, 129..256
   // 94 -> 76 / 71 -> 57, 33..128 58 -> 51 / 52 -> 51; up to 32 rows the copies
-  // are too short (46 / 43 against 50 / 49). Their stall flag costs a batch
-  // without longer systems 10 to 14 us more, so there only many systems of
-  // more than 256 rows pay (2048 in FP64: 66 -> 64 us, 51 -> 57 in FP32; 16384
-  // in FP32: 105 -> 86). Misaligned arrays keep the warps' own copies.
-  bool bulk = counts[3] >= (sizeof(T) == 8 ? 2048 : 8192);
+  // are too short (46 / 43 against 50 / 49). Only beside longer systems, whose
+  // solver waits for the stall flag anyway: a batch of systems of up to 512 rows
+  // alone returns once enqueued. Misaligned arrays keep the warps' own copies.
+  bool bulk = false;
   for (int k = 4; k < GT_NC; ++k) bulk |= counts[k] > 0 && staged_algo(tab[k]);
-  for (int k = 1; k <= top_warp && bulk && aligned && !merge; ++k)
+  for (int k = 1; k <= top_warp && bulk && aligned && !merge && !warp_asked; ++k)
     if (tab[k] == HYDIST_GTSV_WARP) tab[k] = GTSV_WARP_BULK;
   for (int k = 0; k < GT_NC; ++k) staged |= counts[k] > 0 && staged_algo(tab[k]);
   // the classes' solves are independent (disjoint systems, per-class lists,
@@ -1167,12 +1168,13 @@ int solve_on(const T* dl, const T* d, const T* du, const T* b, T* x, const int* 
 // classes may have been launched by then.
 template <class T>
 int solve_batch(const T* dl, const T* d, const T* du, const T* b, T* x, const int* off,
-                const int* len, int nsys, const int table[GT_NB], DevInfo& D, cudaStream_t st) {
+                const int* len, int nsys, const int table[GT_NB], bool warp_asked, DevInfo& D,
+                cudaStream_t st) {
   if (!D.done && cudaEventCreateWithFlags(&D.done, cudaEventDisableTiming) != cudaSuccess)
     return HYDIST_ERR_CUDA;
   if (cudaStreamWaitEvent(st, D.done, 0) != cudaSuccess) return HYDIST_ERR_CUDA;
   int rc = ensure_scratch(D.scr, 0, (size_t)nsys);
-  if (rc == HYDIST_OK) rc = solve_on<T>(dl, d, du, b, x, off, len, nsys, table, D, st);
+  if (rc == HYDIST_OK) rc = solve_on<T>(dl, d, du, b, x, off, len, nsys, table, warp_asked, D, st);
   if (cudaEventRecord(D.done, st) != cudaSuccess && rc == HYDIST_OK) rc = HYDIST_ERR_CUDA;
   return rc;
 }
@@ -1230,7 +1232,7 @@ int autotune(DevInfo& D, int dtype, cudaStream_t st) {
         float tmin = 1e30f;
         for (int rep = 0; rep < 4 && rc == HYDIST_OK; ++rep) {
           cudaEventRecord(e0, st);
-          rc = solve_batch<T>(dl, dd, du, bb, xx, doff, dlen, ns, table, D, st);
+          rc = solve_batch<T>(dl, dd, du, bb, xx, doff, dlen, ns, table, false, D, st);
           cudaEventRecord(e1, st);
           cudaEventSynchronize(e1);
           float ms = 0;
@@ -1320,12 +1322,13 @@ extern "C" int hydist_gtsv_batched(const void* dl, const void* d, const void* du
     table[bnd] = a;
   }
   int rc;
+  const bool warp = algo == HYDIST_GTSV_WARP;
   if (dtype == 0) {
-    rc = solve_batch<double>((const double*)dl, (const double*)d, (const double*)du,
-                             (const double*)b, (double*)x, offsets, lengths, nsys, table, *D, st);
+    rc = solve_batch<double>((const double*)dl, (const double*)d, (const double*)du, (const double*)b,
+                             (double*)x, offsets, lengths, nsys, table, warp, *D, st);
   } else {
     rc = solve_batch<float>((const float*)dl, (const float*)d, (const float*)du, (const float*)b,
-                            (float*)x, offsets, lengths, nsys, table, *D, st);
+                            (float*)x, offsets, lengths, nsys, table, warp, *D, st);
   }
   if (rc == HYDIST_ERR_ARG) hyd::set_last_error("hydist_gtsv_batched: a system has a negative offset");
   else if (rc == HYDIST_ERR_TIMEOUT)

@@ -401,10 +401,14 @@ int hydist_kernel_launches(HydistHandle* h, int64_t* count);
  * them. Scratch is allocated by the library on first use and grown as
  * needed. The call synchronises the
  * stream once to read the band sizes and the packed extent, and, when a
- * shared-memory CTA solver (PARTITION*) ran, once more at the end: every
- * wait of those solvers for a system's rows is bounded, and a CTA that gave
- * up leaves its remaining systems unsolved, which this call (not a later
- * one) reports as HYDIST_ERR_TIMEOUT. A batch with a negative offset is
+ * shared-memory CTA solver (PARTITION*) or the tiles ran, once more at the
+ * end: every wait of those solvers for a system's rows is bounded, and a CTA
+ * that gave up leaves its remaining systems unsolved, which this call (not a
+ * later one) reports as HYDIST_ERR_TIMEOUT. A batch of systems of up to 512
+ * rows (WARP; untuned, AUTO too) and one that asks for THOMAS or PIVOT return
+ * once enqueued. Beside longer systems AUTO stages the shorter ones like those
+ * (one or two warps a system, the partition method too); a named WARP runs as
+ * it is described. A batch with a negative offset is
  * refused with HYDIST_ERR_ARG. */
 enum HydistGtsvAlgo {
   HYDIST_GTSV_AUTO = 0,
