@@ -93,7 +93,9 @@ constexpr int line_min_blocks() {
   return (P == 128 && L == LPB) ? Gen::MIN_BLOCKS : (b > 32 ? 32 : b);
 }
 
-// The launch solves line groups 0 .. ngroups-1 of L lines from line0 on.
+// The launch solves line groups 0 .. ngroups-1 of L lines from line0 on (0 in every
+// launch; without it the compiler contracts the FP32 rows' sums and products
+// otherwise, and their bits are to stay, see pairgen.cuh).
 // BATCH: the groups of every member of a batch, gpm groups per member (the
 // member of group g is g / gpm, its state and coefficients bound into a
 // copy of G0 for that group); the persistent grid walks them all, each CTA

@@ -10,20 +10,18 @@
 //           unknown is its separator. The first interior row in terms of both
 //           neighbouring separators is accumulated on the way;
 //   reduce  the separators form a tridiagonal system of one unknown per
-//           chunk, solved by parallel cyclic reduction (shared memory for a
-//           CTA, shuffles for a warp);
+//           chunk, solved by cyclic reduction with shuffles: over a warp's
+//           chunks, and in a CTA then over its warps' last separators;
 //   pass C  back substitution, x written over D.
-// Shared-memory index of row q is q + q/S (one pad slot per chunk), so the
-// chunks a warp walks in step fall on different banks.
+// So that the chunks a warp walks in step fall on different banks, a CTA's are
+// of odd length (bulk_chunk); the warp solver pads instead, row q at q + q/S.
 #pragma once
 
 #include <cuda_runtime.h>
 
 namespace hyd {
 
-__host__ __device__ inline int part_idx(int q, int S) { return q + q / S; }
-
-// part_idx of q = t0, t0 + dt, t0 + 2 dt, ... without a division per step:
+// q + q / S of q = t0, t0 + dt, t0 + 2 dt, ... without a division per step:
 // carries the quotient and remainder of q / S.
 struct PartStrideIdx {
   int q, qd, qr, dd, dr, S;
@@ -329,7 +327,7 @@ __device__ __forceinline__ void cta_solve(T* oV, T* oC, T* X, int n, W (*blk)[8]
 }
 
 // Reduced-system work space of a CTA of NT threads: what each warp's first
-// and last chunks give the others (tridiag.cu, tile_reduce).
+// and last chunks give the others (tile_reduce).
 template <class T, int NT>
 struct PartCtaShared {
   T blk[NT / 32][8];

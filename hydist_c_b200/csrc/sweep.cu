@@ -31,7 +31,6 @@ struct HydroGen {
   static constexpr int UPC = 1;
   static constexpr int AUX = 3;  // c', y', v', then the emitter's value
   static constexpr int SCRATCH_ARRAYS = AUX + 1;
-  static constexpr bool HYDRO = true;
   static constexpr int DIRECTION = DIR;
   // resident CTAs per SM the chunked row solver is compiled for (two, with
   // their register cap, are slower)
@@ -396,36 +395,29 @@ static void launch_gen(const Gen& G, cudaStream_t st, int grid, int line0, int n
   }
 }
 
-// Threads per row of the staged row solver: 5 to 9 cells each (odd chunks),
-// a warp for the shortest rows.
+// Threads per row of the staged row solver: a warp for the shortest rows, else 5
+// to 9 cells each (odd chunks), more on rows of over 4608 cells (512 threads: 19
+// in FP64, 29 in FP32, 17 refined at the longest).
 static int row_threads(int ncells) {
   return ncells <= 160 ? 32 : ncells <= 352 ? 64 : ncells <= 1152 ? 128 : ncells <= 2304 ? 256 : 512;
 }
 
-// Device limits the launches need, queried once per device.
-struct DevLimits {
-  int nsm = 0, optin = 0;
-};
-static DevLimits dev_limits() {
-  static DevLimits lim[64] = {};
+// Shared memory a CTA may have, queried once per device.
+static int smem_optin() {
+  static int optin[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return {};
-  if (!lim[dev].optin) {
-    DevLimits l;
-    cudaDeviceGetAttribute(&l.nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&l.optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    lim[dev] = l;
-  }
-  return lim[dev];
+  if (dev < 0 || dev >= 64) return 0;
+  if (!optin[dev]) cudaDeviceGetAttribute(&optin[dev], cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return optin[dev];
 }
 
 // The staged row solver takes rows that one CTA's shared memory holds (beside
-// its tables): about 9300 cells in FP64, 18000 in FP32, 8000 refined. Longer
-// ones keep the chunked solver with its scratch in global memory.
+// its tables): 9344 cells in FP64, 14016 in FP32, 8009 refined. Longer ones keep
+// the chunked solver with its scratch in global memory.
 template <class Gen>
 static bool row_fits(int ncells) {
-  return row_smem<Gen>(ncells) + 8192 <= (size_t)dev_limits().optin;
+  return row_smem<Gen>(ncells) + 8192 <= (size_t)smem_optin();
 }
 
 template <class Gen, int NT, int BATCH>
@@ -433,11 +425,10 @@ static void launch_row_nt(const Gen& G, int ncells, int lines, cudaStream_t st,
                           const Batch<typename Gen::Real>& b) {
   int dev = 0;
   cudaGetDevice(&dev);
-  const DevLimits lim = dev_limits();
   static bool attr[64] = {};
   if (dev < 64 && !attr[dev]) {
     cudaFuncSetAttribute(k_row_solve<Gen, NT, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         lim.optin - 8192);
+                         smem_optin() - 8192);
     attr[dev] = true;
   }
   const dim3 grid(lines, std::max(b.n, 1));
@@ -469,8 +460,8 @@ static void launch_rows(const Gen& G, int ncells, int lines, cudaStream_t st,
 }
 
 // The staged column solver takes columns of up to COL_MAX cells, a 32-byte
-// sector of them per CTA (4 in FP64 and refined, 8 in FP32; up to 8800 cells
-// and 106 KB). Hydraulic x sweep, chunked -> staged: 64x32 50 -> 13 us,
+// sector of them per CTA (4 in FP64 and refined, 8 in FP32; 1100 cells take 106
+// KB in FP64, 141 in FP32, 123 refined). Hydraulic x sweep, chunked -> staged: 64x32 50 -> 13 us,
 // 256x128 31 -> 19, 512x256 32 -> 23, 1024x512 58 -> 42 (FP64); at 2048x1024 its
 // 196 KB of rows in one CTA per SM lose
 // (111 -> 220, two columns per CTA 168), so longer columns keep the chunks.
@@ -637,7 +628,6 @@ struct FSGen {
   static constexpr int AUX = 0;  // the emitter needs nothing but the solution
   static constexpr int SCRATCH_ARRAYS = REFINE ? 4 : 3;
   static constexpr int UPC = 1;
-  static constexpr bool HYDRO = false;
   static constexpr int DIRECTION = DIR;
   static constexpr int MIN_BLOCKS = 2;  // in both precisions
   StateT<R> S;
