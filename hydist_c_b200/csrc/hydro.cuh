@@ -55,7 +55,7 @@ int launch_fs_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t
                     const Batch<R>& b = {});
 // whether that sweep forms its rows itself, without k_fs_rows before it
 template <class R>
-bool fs_rows_in_sweep(const StateT<R>& S, int dir);
+bool fs_rows_in_sweep(const StateT<R>& S, int dir, const Batch<R>& b);
 // concentration step (after a half-step launched with sed): xdir = the
 // i-sweep after half-step A; bed: the bed change after the j-sweep
 template <class R>

@@ -1,7 +1,8 @@
 // linesolve.cuh -- chunked tridiagonal line solver: the hydraulic sweeps of the
 // FP32 forms (pairgen.cuh), and of the other sweeps the lines that the staged
 // solvers (rowsolve.cuh, colsolve.cuh) do not take: columns of more than 1100
-// cells, rows of more than one CTA's shared memory holds.
+// cells or in a part of a second round, rows of more than one CTA's shared memory
+// holds (sweep.cu).
 //
 // One CTA solves L adjacent lines at a time (LPB = 4 or XPB = 8; a persistent
 // loop walks the line groups). Each line is split into P chunks of consecutive

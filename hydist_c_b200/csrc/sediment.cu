@@ -253,7 +253,7 @@ void launch_sediment(const StateT<R>& S, const CoefT<R>& c, bool xdir, bool bed,
   // Find_VTH + hesoK ran in the half-step's commit (k_commit_a/k_commit_b)
   if (tr) tr->kbegin(st, xdir ? KS_FS_X : KS_FS_Y);
   const unsigned z = grid_z(b);
-  const bool rows = !fs_rows_in_sweep(S, xdir ? 0 : 1);
+  const bool rows = !fs_rows_in_sweep(S, xdir ? 0 : 1, b);
   if (rows) {
     const dim3 gr(cdiv(S.M - 1, 128), S.N - 1, z);
     if (b.n > 0) {

@@ -461,16 +461,39 @@ static void launch_rows(const Gen& G, int ncells, int lines, cudaStream_t st,
 
 // The staged column solver takes columns of up to COL_MAX cells, a 32-byte
 // sector of them per CTA (4 in FP64 and refined, 8 in FP32; 1100 cells take 106
-// KB in FP64, 141 in FP32, 123 refined). Hydraulic x sweep, chunked -> staged: 64x32 50 -> 13 us,
-// 256x128 31 -> 19, 512x256 32 -> 23, 1024x512 58 -> 42 (FP64); at 2048x1024 its
-// 196 KB of rows in one CTA per SM lose
-// (111 -> 220, two columns per CTA 168), so longer columns keep the chunks.
+// KB in FP64, 141 in FP32, 123 refined). Hydraulic x sweep, chunked -> staged: 64x32
+// 50 -> 13 us, 256x128 31 -> 19, 512x256 32 -> 23, 1024x512 58 -> 42 (FP64); at
+// 2048x1024 its 196 KB of rows in one CTA per SM lose (111 -> 220, two columns per
+// CTA 168), so longer columns keep the chunks. (Where one round of CTAs takes all
+// columns it wins further on, hydraulic and concentration 1300x300 70 -> 48 and 48 ->
+// 42, refined 50 -> 37; in FP32 the line lies at 1300, 1500x300 40 -> 58.)
+//
+// Groups of four that leave a second round of CTAs not nearly full go to the chunks
+// too, from 640 cells on, refined (two CTAs an SM up to about there) from 850 on. 590
+// and 600 columns (148 and 150 groups on 148 SMs), staged / chunked, us: 620 cells
+// hydraulic 29/46, 44/48, concentration 25/40, 40/40, refined 25/35, 27/35; 700
+// cells 33/50, 52/50, 29/42, 46/42, 29/38, 31/39; 800 cells refined 31/42, 37/42;
+// 900 cells 42/58, 66/58, 37/48, 62/48, 46/44, 64/44; 1100 cells with 900 columns
+// 80/72, 76/64, 68/52. A step of two members of 1024x512 (256 groups) 465 -> 457 us; with
+// more rounds the tail is a smaller part: six members of 900x200 (300 groups) 585
+// against 607, three of 1101x500 (375) 713 against 744, eight of 1024x512 1584
+// against 1596.
 constexpr int COL_MAX = 1100;
+template <class Gen>
+constexpr int col_tail() {
+  return Gen::REFINE ? 850 : 640;
+}
 template <class Gen>
 constexpr int col_group() {
   return sizeof(typename Gen::Real) == 8 || Gen::REFINE ? 4 : 8;
 }
-static bool cols_fit(int ncells) { return ncells <= COL_MAX; }
+template <class Gen>
+static bool cols_fit(const StateT<typename Gen::Real>& S, int ncells, int lines, int members) {
+  if (ncells > COL_MAX) return false;
+  const long long groups = (long long)cdiv(lines, col_group<Gen>()) * std::max(members, 1);
+  const int nsm = S.lslots / 2;
+  return col_group<Gen>() != 4 || ncells <= col_tail<Gen>() || groups <= nsm || groups > 2 * nsm;
+}
 
 template <class Gen, int NT, int L, int BATCH>
 static void launch_col_nt(const Gen& G, int ncells, int lines, cudaStream_t st,
@@ -531,7 +554,7 @@ static int launch_lines(const Gen& G, int ncells, int lines, cudaStream_t st,
                          b.n > 0 ? groups : 0);
     return 1;
   } else {
-    if (cols_fit(ncells)) {
+    if (cols_fit<Gen>(G.S, ncells, lines, b.n)) {
       launch_cols<Gen, col_group<Gen>()>(G, ncells, lines, st, b);
       return 1;
     }
@@ -842,11 +865,12 @@ struct FSGen {
 // whether the concentration sweep forms its rows itself (else k_fs_rows
 // writes them ahead of it)
 template <class R>
-bool fs_rows_in_sweep(const StateT<R>& S, int dir) {
-  if (dir == 0) return cols_fit(S.N - 1);
+bool fs_rows_in_sweep(const StateT<R>& S, int dir, const Batch<R>& b) {
   if constexpr (sizeof(R) == 4) {
+    if (S.refine && dir == 0) return cols_fit<FSGen<0, R, true>>(S, S.N - 1, S.M - 3, b.n);
     if (S.refine) return row_fits<FSGen<1, R, true>>(S.M - 1);
   }
+  if (dir == 0) return cols_fit<FSGen<0, R, false>>(S, S.N - 1, S.M - 3, b.n);
   return row_fits<FSGen<1, R, false>>(S.M - 1);
 }
 
@@ -879,8 +903,8 @@ int launch_sweep(const StateT<R>& S, const CoefT<R>& c, int dir, cudaStream_t st
   }
 }
 
-template bool fs_rows_in_sweep<double>(const StateT<double>&, int);
-template bool fs_rows_in_sweep<float>(const StateT<float>&, int);
+template bool fs_rows_in_sweep<double>(const StateT<double>&, int, const Batch<double>&);
+template bool fs_rows_in_sweep<float>(const StateT<float>&, int, const Batch<float>&);
 template int launch_sweep<double>(const StateT<double>&, const CoefT<double>&, int, cudaStream_t,
                                   const Batch<double>&);
 template int launch_sweep<float>(const StateT<float>&, const CoefT<float>&, int, cudaStream_t,
