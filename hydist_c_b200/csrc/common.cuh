@@ -204,12 +204,15 @@ struct Trace {
 // one start once every block of this one has come so far, so that a launch's
 // latency falls into the tail of the kernel before. A step on a B200, without
 // -> with: 64x32 49.2 -> 47.1 us, 256x128 63.7 -> 59.4, 464x324 with sediment
-// 129 -> 127, 24 members of 256x128 in FP32 306 -> 298; 2048x1024 706 -> 715
-// and 8 members of 1024x512 1583 -> 1625 (the waiting blocks take places in
-// which the kernel's own would have been spread), so only up to
-// DEPENDENT_CELLS cells in all, by kernels of their own: the two instructions,
+// 129 -> 127, 2000x500 434 -> 427, 16 members of 256x128 313 -> 306 (FP32 301 ->
+// 295), 30 of them 527 -> 524; 2048x1024 706 -> 715 and 8 members of 1024x512 1583
+// -> 1625 (the waiting blocks take places in which the kernel's own would have been
+// spread). Between the two the gain thins out: 3000x400 (1.2 M cells) 567 -> 560,
+// 3000x590 (1.8 M) 690 -> 687, 48 members of 256x128 (1.6 M) 774 -> 774. So only up
+// to DEPENDENT_CELLS cells in all, by kernels of their own: the two instructions,
 // or a branch around them, cost the large meshes 9 us too. (Letting the next
-// one start before the wait: 53.3, 63.5 and 138 us.)
+// one start before the wait: 53.3, 63.5 and 138 us.) The FP32 forms' hydraulic
+// sweeps wait for the whole kernel before, and the one after for them.
 constexpr size_t DEPENDENT_CELLS = (size_t)1 << 20;
 template <class R>
 inline bool dependent_launches(const StateT<R>& S, const Batch<R>& b) {
