@@ -1,11 +1,17 @@
 """Batches of short systems return once they are enqueued, however many they are;
 a named solver is the one that runs."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
 from hydist_c_b200 import capi
 
 pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parents[1]
 
 
 def _batch(lens, seed, dtype):
@@ -17,9 +23,7 @@ def _batch(lens, seed, dtype):
         torch.from_numpy(ln).cuda()
 
 
-@pytest.mark.parametrize("dtype", ["float64", "float32"])
-@pytest.mark.parametrize("algo", [capi.GTSV_AUTO, capi.GTSV_WARP])
-def test_short_batch_returns_before_it_is_solved(hyd, dtype, algo):
+def _returns_early(hyd, dtype, algo):
     """60000 systems of 500 rows (30 M rows, 1.2 GB in FP64): hundreds of
     microseconds of solving, enqueued in a few."""
     import torch
@@ -34,6 +38,22 @@ def test_short_batch_returns_before_it_is_solved(hyd, dtype, algo):
         running += not st.query()
         torch.cuda.synchronize()
     assert running >= 4
+
+
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_short_batch_returns_before_it_is_solved(hyd, dtype):
+    _returns_early(hyd, dtype, capi.GTSV_WARP)
+
+
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_short_untuned_batch_returns_before_it_is_solved(dtype):
+    """AUTO before any tuning, so in a process of its own (the autotuner's table
+    is the process's)."""
+    r = subprocess.run([sys.executable, "-c", "import hydist_c_b200 as H, test_gtsv_returns as T\n"
+                        f"T._returns_early(H, {dtype!r}, 0)\nprint('all well')"],
+                       cwd=ROOT, env=dict(os.environ, PYTHONPATH=f"{ROOT}:{ROOT / 'tests'}"),
+                       capture_output=True, text=True, timeout=300)
+    assert "all well" in r.stdout, r.stdout + r.stderr
 
 
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
