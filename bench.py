@@ -52,8 +52,10 @@ BYTES_PER_CELL_STEP = {  # algorithmic bytes per interior cell and full step
 #     Ky = 10 x 8 B; write tFS = 8 B                             -> 88 B
 #     (the concentration sweep of columns of more than 1100 cells is timed
 #     over its two launches: the per-cell row kernel k_fs_rows and the solve)
-# The chunked solver's scratch (3 doubles per unknown) and the concentration
-# rows passed between those two launches (4 doubles per cell) are not counted.
+# The chunked solver's scratch (4 values per cell in FP64 hydraulic sweeps, 3 in
+# concentration sweeps, 6 in the FP32 forms' hydraulic sweeps, 14 refined) and the
+# concentration rows passed between those two launches (4 values per cell) are not
+# counted.
 # In the FP32 form z is read (8 B) and t_z written (8 B) in FP64, the other
 # fields are 4 B: hydraulic 8 + 8 x 4 + 8 + 4 = 52 B, concentration 11 x 4 = 44 B.
 SWEEP_BYTES_PER_CELL = {
@@ -572,8 +574,8 @@ def run_tridiag(args):
     lib.hydist_gtsv_band_bounds(bands)
     nonempty = 0
     lo = 0
-    # one launch per non-empty length class (a batch of this many short systems
-    # is not merged into one)
+    # one launch per non-empty length class (gt_class_hi in csrc/tridiag.cu; a batch
+    # of this many short systems is not merged into one)
     for hi in (32, 128, 256, 512, 1024, 1536, 2048, 3072, 4096, 6144, 1 << 30):
         nonempty += int(((ln > lo) & (ln <= hi)).sum() > 0)
         lo = hi
